@@ -61,6 +61,7 @@ def build(verbose=False):
     if not os.path.exists(LIB) or any(os.path.getmtime(o) > os.path.getmtime(LIB) for o in objs):
         subprocess.check_call([_nvcc(), "-shared", "-o", LIB] + objs + ["-gencode", "arch=compute_100a,code=sm_100a"])
     build_host()
+    build_native()
     build_ceilings()
     return LIB
 
@@ -89,6 +90,30 @@ def build_host():
                           + ["-o", HOST_LIB, "-L", HERE, "-lnnf_b200", "-Wl,-rpath,$ORIGIN",
                              "-L", os.path.join(cuda_home, "lib64"), "-lcudart_static", "-ldl", "-lrt", "-lpthread", "-Wl,--exclude-libs,ALL"])
     return HOST_LIB
+
+
+NATIVE_LIB = os.path.join(HERE, "_native.so")
+NATIVE_SRC = os.path.join(CSRC, "python", "nnf_binding.cpp")
+
+
+def build_native():
+    """The module that capi.py and host.py call the two libraries through."""
+    deps = [NATIVE_SRC, os.path.join(os.path.dirname(HERE), "include", "nnf_b200.h")]
+    if os.path.exists(NATIVE_LIB) and os.path.getmtime(NATIVE_LIB) >= max(os.path.getmtime(d) for d in deps):
+        return NATIVE_LIB
+    import sysconfig
+
+    import torch
+    root = os.path.dirname(torch.__file__)
+    cuda_home = os.path.dirname(os.path.dirname(_nvcc())) if os.path.sep in _nvcc() else "/usr/local/cuda"
+    include = [os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"), os.path.join(cuda_home, "include"),
+               sysconfig.get_paths()["include"]]
+    # torch's libraries are in the process already when the module is imported (capi.py imports torch first): no run path to them
+    subprocess.check_call(["g++", "-std=c++17", "-O2", "-fPIC", "-shared", "-fvisibility=hidden",
+                           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)] + ["-isystem" + d for d in include]
+                          + [NATIVE_SRC, "-o", NATIVE_LIB, "-L", HERE, "-lnnf_b200", "-lnnf_b200_host", "-Wl,-rpath,$ORIGIN",
+                             "-L", os.path.join(root, "lib"), "-ltorch_python", "-ltorch_cpu", "-lc10", "-lc10_cuda"])
+    return NATIVE_LIB
 
 
 if __name__ == "__main__":

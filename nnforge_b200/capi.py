@@ -19,6 +19,12 @@ if not os.path.exists(LIB_PATH):
 
 lib = ct.CDLL(LIB_PATH)
 
+try:
+    from . import _native   # the calls a step makes; set-up calls and the multi-GPU exchange go through ctypes
+except ImportError as e:
+    raise ImportError("nnforge_b200/_native.so is missing or was built against another torch: build it with "
+                      "`python -m nnforge_b200.build`") from e
+
 ACT_NONE, ACT_RELU, ACT_PRELU, ACT_ELU, ACT_TANH, ACT_SIGMOID = range(6)
 MAX_ACTS = 2
 MAX_ADD_INPUTS = 8
@@ -28,6 +34,9 @@ class NnfError(RuntimeError):
     def __init__(self, status, text):
         super().__init__("nnf_b200 status %d: %s" % (status, text))
         self.status = status
+
+
+_native.set_error_type(NnfError)
 
 
 class Act(ct.Structure):
@@ -191,56 +200,43 @@ def _nchw(t):
 
 def bn_infer_act(y, x, bn=None, residual=None, add_alpha=1.0, acts=(), stream=None):
     """bn = (gamma, beta, mean, invsigma) device tensors or None."""
-    n, c, hw = _nchw(x)
-    g, b, m, i = bn if bn is not None else (None, None, None, None)
-    arr, k = _acts(acts)
-    _check(lib.nnf_bn_infer_act(_stream(stream), _ptr(y), _ptr(x), _ptr(g), _ptr(b), _ptr(m), _ptr(i), _ptr(residual), add_alpha, arr, k, n, c, hw))
+    _native.bn_infer_act(y, x, None, bn, residual, add_alpha, acts, stream)
 
 
 def bias_bn_infer_act(y, x, bias, bn=None, residual=None, add_alpha=1.0, acts=(), stream=None):
     """bn_infer_act with a per-channel bias added to x first."""
-    n, c, hw = _nchw(x)
-    g, b, m, i = bn if bn is not None else (None, None, None, None)
-    arr, k = _acts(acts)
-    _check(lib.nnf_bias_bn_infer_act(_stream(stream), _ptr(y), _ptr(x), _ptr(bias), _ptr(g), _ptr(b), _ptr(m), _ptr(i), _ptr(residual), add_alpha,
-                                     arr, k, n, c, hw))
+    _native.bn_infer_act(y, x, bias, bn, residual, add_alpha, acts, stream)
 
 
 def act_fwd(y, x, act, stream=None):
-    n, c, hw = _nchw(x)
-    _check(lib.nnf_act_fwd(_stream(stream), _ptr(y), _ptr(x), ct.byref(act), n, c, hw))
+    _native.act_fwd(y, x, act, stream)
 
 
 def act_bwd(dx, dy, neurons, act, add_to_destination=False, stream=None):
-    n, c, hw = _nchw(dy)
-    _check(lib.nnf_act_bwd(_stream(stream), _ptr(dx), _ptr(dy), _ptr(neurons), ct.byref(act), n, c, hw, int(add_to_destination)))
+    _native.act_bwd(dx, dy, neurons, act, add_to_destination, stream)
 
 
 def prelu_bwd_weights(dslope, dy, x, workspace=None, stream=None):
-    n, c, hw = _nchw(x)
-    need = lib.nnf_prelu_bwd_weights_workspace_bytes(n, c, hw)
     if workspace is None:
-        workspace = torch.empty(need, dtype=torch.uint8, device=x.device)
-    _check(lib.nnf_prelu_bwd_weights(_stream(stream), _ptr(dslope), _ptr(dy), _ptr(x), n, c, hw, _ptr(workspace), workspace.numel()))
+        n, c, hw = _nchw(x)
+        workspace = torch.empty(lib.nnf_prelu_bwd_weights_workspace_bytes(n, c, hw), dtype=torch.uint8, device=x.device)
+    _native.prelu_bwd_weights(dslope, dy, x, workspace, stream)
 
 
 def add_fwd(y, inputs, alpha=1.0, stream=None):
-    arr = (_P * len(inputs))(*[_ptr(t) for t in inputs])
-    _check(lib.nnf_add_fwd(_stream(stream), _ptr(y), arr, len(inputs), alpha, y.numel()))
+    _native.add_fwd(y, inputs, alpha, stream)
 
 
 def add_bwd(dx, dy, alpha=1.0, add_to_destination=False, stream=None):
-    _check(lib.nnf_add_bwd(_stream(stream), _ptr(dx), _ptr(dy), alpha, dy.numel(), int(add_to_destination)))
+    _native.add_bwd(dx, dy, alpha, add_to_destination, stream)
 
 
 def softmax_fwd(y, x, stream=None):
-    n, c, hw = _nchw(x)
-    _check(lib.nnf_softmax_fwd(_stream(stream), _ptr(y), _ptr(x), n, c, hw))
+    _native.softmax_fwd(y, x, stream)
 
 
 def softmax_bwd(dx, dy, y, add_to_destination=False, stream=None):
-    n, c, hw = _nchw(y)
-    _check(lib.nnf_softmax_bwd(_stream(stream), _ptr(dx), _ptr(dy), _ptr(y), n, c, hw, int(add_to_destination)))
+    _native.softmax_bwd(dx, dy, y, add_to_destination, stream)
 
 
 def pool(win, stride, round_up=(False, False), is_min=False):
@@ -253,26 +249,19 @@ def pool_out_shape(h, w, p):
 
 
 def maxpool_fwd(y, argmax, x, p, stream=None):
-    n, c, h, w = x.shape
-    _check(lib.nnf_maxpool_fwd(_stream(stream), _ptr(y), _ptr(argmax), _ptr(x), n, c, h, w, ct.byref(p)))
+    _native.maxpool_fwd(y, argmax, x, p, stream)
 
 
 def maxpool_bwd(dx, dy, argmax, p, add_to_destination=False, stream=None):
-    n, c, h, w = dx.shape
-    _check(lib.nnf_maxpool_bwd(_stream(stream), _ptr(dx), _ptr(dy), _ptr(argmax), n, c, h, w, ct.byref(p), int(add_to_destination)))
+    _native.maxpool_bwd(dx, dy, argmax, p, add_to_destination, stream)
 
 
 def bn_add_relu_maxpool_fwd(z, pooled, argmax, x, residual, bn, relu_slope, p, stream=None):
-    n, c, h, w = x.shape
-    g, b, m, i = bn if bn is not None else (None, None, None, None)
-    _check(lib.nnf_bn_add_relu_maxpool_fwd(_stream(stream), _ptr(z), _ptr(pooled), _ptr(argmax), _ptr(x), _ptr(residual), _ptr(g), _ptr(b),
-                                           _ptr(m), _ptr(i), relu_slope, n, c, h, w, ct.byref(p)))
+    _native.bn_add_relu_maxpool_fwd(z, pooled, argmax, x, residual, bn, relu_slope, p, stream)
 
 
 def bn_add_relu_maxpool_bwd(dx, dresidual, dpooled, argmax, z, gamma, invsigma, relu_slope, p, stream=None):
-    n, c, h, w = z.shape
-    _check(lib.nnf_bn_add_relu_maxpool_bwd(_stream(stream), _ptr(dx), _ptr(dresidual), _ptr(dpooled), _ptr(argmax), _ptr(z), _ptr(gamma),
-                                           _ptr(invsigma), relu_slope, n, c, h, w, ct.byref(p)))
+    _native.bn_add_relu_maxpool_bwd(dx, dresidual, dpooled, argmax, z, gamma, invsigma, relu_slope, p, stream)
 
 
 def bn_train_workspace_bytes(n, c, hw):
@@ -280,39 +269,26 @@ def bn_train_workspace_bytes(n, c, hw):
 
 
 def bn_train_stats(sums, x, workspace, stream=None):
-    n, c, hw = _nchw(x)
-    _check(lib.nnf_bn_train_stats(_stream(stream), _ptr(sums), _ptr(x), n, c, hw, _ptr(workspace), workspace.numel() * workspace.element_size()))
+    _native.bn_train_stats(sums, x, workspace, stream)
 
 
 def bn_train_stats_static(sums, x, stream=None):
     """nnf_bn_train_stats without a workspace argument (library-resident scratch, c <= 1024)."""
-    n, c, hw = _nchw(x)
-    _check(lib.nnf_bn_train_stats_static(_stream(stream), _ptr(sums), _ptr(x), n, c, hw))
+    _native.bn_train_stats_static(sums, x, stream)
 
 
 def bn_train_apply_act(y, saved, x, gamma, beta, sums, count_total, eps, acts=(), stream=None):
-    n, c, hw = _nchw(x)
-    arr, k = _acts(acts)
-    _check(lib.nnf_bn_train_apply_act(_stream(stream), _ptr(y), _ptr(saved), _ptr(x), _ptr(gamma), _ptr(beta), _ptr(sums), float(count_total), eps,
-                                      arr, k, n, c, hw))
+    _native.bn_train_apply_act(y, saved, x, gamma, beta, sums, count_total, eps, acts, stream)
 
 
 def bn_train_fwd(y, saved, sums, x, gamma, beta, eps, acts=(), workspace=None, stream=None):
-    n, c, hw = _nchw(x)
-    arr, k = _acts(acts)
-    nbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
-    _check(lib.nnf_bn_train_fwd(_stream(stream), _ptr(y), _ptr(saved), _ptr(sums), _ptr(x), _ptr(gamma), _ptr(beta), eps, arr, k, n, c, hw,
-                                _ptr(workspace), nbytes))
+    _native.bn_train_fwd(y, saved, sums, x, gamma, beta, eps, acts, workspace, stream)
 
 
 def bn_train_bwd(dx, bsums, dy, x, gamma, beta, saved, acts=(), grad_gamma=None, grad_beta=None, grad_mean=None, grad_invsigma=None,
                  grad_slope=None, mean=None, invsigma=None, entry_count=0.0, add_to_destination=False, workspace=None, stream=None):
-    n, c, hw = _nchw(x)
-    arr, k = _acts(acts)
-    nbytes = workspace.numel() * workspace.element_size() if workspace is not None else 0
-    _check(lib.nnf_bn_train_bwd(_stream(stream), _ptr(dx), _ptr(bsums), _ptr(dy), _ptr(x), _ptr(gamma), _ptr(beta), _ptr(saved), arr, k,
-                                _ptr(grad_gamma), _ptr(grad_beta), _ptr(grad_mean), _ptr(grad_invsigma), _ptr(grad_slope), _ptr(mean), _ptr(invsigma),
-                                float(entry_count), n, c, hw, int(add_to_destination), _ptr(workspace), nbytes))
+    _native.bn_train_bwd(dx, bsums, dy, x, gamma, beta, saved, acts, grad_gamma, grad_beta, grad_mean, grad_invsigma, grad_slope, mean, invsigma,
+                         entry_count, add_to_destination, workspace, stream)
 
 
 def peer_exchange_bytes(kmax):
@@ -378,78 +354,58 @@ def parse_report(host_words):
 
 
 def bn_train_bwd_stats(bsums, dy, x, gamma, beta, saved, acts, workspace, gsums=None, stream=None):
-    n, c, hw = _nchw(x)
-    arr, k = _acts(acts)
-    _check(lib.nnf_bn_train_bwd_stats(_stream(stream), _ptr(bsums), _ptr(gsums), _ptr(dy), _ptr(x), _ptr(gamma), _ptr(beta), _ptr(saved), arr, k, n, c, hw,
-                                      _ptr(workspace), workspace.numel() * workspace.element_size()))
+    _native.bn_train_bwd_stats(bsums, gsums, dy, x, gamma, beta, saved, acts, workspace, stream)
 
 
 def bn_train_bwd_apply(dx, dy, x, gamma, beta, saved, gsums, bsums, count_total, acts=(), grad_gamma=None, grad_beta=None, grad_mean=None,
                        grad_invsigma=None, grad_slope=None, mean=None, invsigma=None, entry_count=0.0, add_to_destination=False, stream=None):
-    n, c, hw = _nchw(x)
-    arr, k = _acts(acts)
-    _check(lib.nnf_bn_train_bwd_apply(_stream(stream), _ptr(dx), _ptr(dy), _ptr(x), _ptr(gamma), _ptr(beta), _ptr(saved), _ptr(gsums), _ptr(bsums),
-                                      float(count_total), arr, k, _ptr(grad_gamma), _ptr(grad_beta), _ptr(grad_mean), _ptr(grad_invsigma),
-                                      _ptr(grad_slope), _ptr(mean), _ptr(invsigma), float(entry_count), n, c, hw, int(add_to_destination)))
+    _native.bn_train_bwd_apply(dx, dy, x, gamma, beta, saved, gsums, bsums, count_total, acts, grad_gamma, grad_beta, grad_mean, grad_invsigma,
+                               grad_slope, mean, invsigma, entry_count, add_to_destination, stream)
 
 
 def avgpool_fwd(y, x, win, mult, stream=None):
     """x [N,C,H,W]; win = (w, h)."""
-    n, c, h, w = x.shape
-    _check(lib.nnf_avgpool_fwd(_stream(stream), _ptr(y), _ptr(x), n, c, h, w, win[0], win[1], mult))
+    _native.avgpool_fwd(y, x, win[0], win[1], mult, stream)
 
 
 def avgpool_bwd(dx, dy, win, mult, add_to_destination=False, stream=None):
-    n, c, h, w = dx.shape
-    _check(lib.nnf_avgpool_bwd(_stream(stream), _ptr(dx), _ptr(dy), n, c, h, w, win[0], win[1], mult, int(add_to_destination)))
+    _native.avgpool_bwd(dx, dy, win[0], win[1], mult, add_to_destination, stream)
 
 
 def bn_add_relu_avgpool_fwd(z, pooled, x, residual, bn, relu_slope, win, mult, stream=None):
-    n, c, h, w = x.shape
-    g, b, m, i = bn if bn is not None else (None, None, None, None)
-    _check(lib.nnf_bn_add_relu_avgpool_fwd(_stream(stream), _ptr(z), _ptr(pooled), _ptr(x), _ptr(residual), _ptr(g), _ptr(b), _ptr(m), _ptr(i),
-                                           relu_slope, n, c, h, w, win[0], win[1], mult))
+    _native.bn_add_relu_avgpool_fwd(z, pooled, x, residual, bn, relu_slope, win[0], win[1], mult, stream)
 
 
 def bn_add_relu_avgpool_bwd(dx, dresidual, dpooled, z, gamma, invsigma, relu_slope, win, mult, stream=None):
-    n, c, h, w = z.shape
-    _check(lib.nnf_bn_add_relu_avgpool_bwd(_stream(stream), _ptr(dx), _ptr(dresidual), _ptr(dpooled), _ptr(z), _ptr(gamma), _ptr(invsigma), relu_slope,
-                                           n, c, h, w, win[0], win[1], mult))
+    _native.bn_add_relu_avgpool_bwd(dx, dresidual, dpooled, z, gamma, invsigma, relu_slope, win[0], win[1], mult, stream)
 
 
 def accuracy_fwd(out, predicted, targets, mask=None, top_n=1, stream=None):
-    n, c, hw = _nchw(predicted)
-    _check(lib.nnf_accuracy_fwd(_stream(stream), _ptr(out), _ptr(predicted), _ptr(targets), _ptr(mask), top_n, n, c, hw))
+    _native.accuracy_fwd(out, predicted, targets, mask, top_n, stream)
 
 
 def nll_fwd(err, predicted, targets, mask=None, scale=1.0, stream=None):
-    n, c, hw = _nchw(predicted)
-    _check(lib.nnf_nll_fwd(_stream(stream), _ptr(err), _ptr(predicted), _ptr(targets), _ptr(mask), scale, n, c, hw))
+    _native.nll_fwd(err, predicted, targets, mask, scale, stream)
 
 
 def nll_bwd(dpredicted, predicted, targets, mask=None, scale=1.0, add_to_destination=False, stream=None):
-    n, c, hw = _nchw(predicted)
-    _check(lib.nnf_nll_bwd(_stream(stream), _ptr(dpredicted), _ptr(predicted), _ptr(targets), _ptr(mask), scale, n, c, hw, int(add_to_destination)))
+    _native.nll_bwd(dpredicted, predicted, targets, mask, scale, add_to_destination, stream)
 
 
 def cross_entropy_fwd(err, predicted, targets, mask=None, scale=1.0, stream=None):
-    n, c, hw = _nchw(predicted)
-    _check(lib.nnf_cross_entropy_fwd(_stream(stream), _ptr(err), _ptr(predicted), _ptr(targets), _ptr(mask), scale, n, c, hw))
+    _native.cross_entropy_fwd(err, predicted, targets, mask, scale, stream)
 
 
 def cross_entropy_bwd(dpredicted, predicted, targets, mask=None, scale=1.0, add_to_destination=False, stream=None):
-    n, c, hw = _nchw(predicted)
-    _check(lib.nnf_cross_entropy_bwd(_stream(stream), _ptr(dpredicted), _ptr(predicted), _ptr(targets), _ptr(mask), scale, n, c, hw, int(add_to_destination)))
+    _native.cross_entropy_bwd(dpredicted, predicted, targets, mask, scale, add_to_destination, stream)
 
 
 def softmax_nll_fwd(probs, err, logits, targets, mask=None, scale=1.0, stream=None):
-    n, c, hw = _nchw(logits)
-    _check(lib.nnf_softmax_nll_fwd(_stream(stream), _ptr(probs), _ptr(err), _ptr(logits), _ptr(targets), _ptr(mask), scale, n, c, hw))
+    _native.softmax_nll_fwd(probs, err, logits, targets, mask, scale, stream)
 
 
 def softmax_nll_bwd(dlogits, probs, targets, mask=None, scale=1.0, add_to_destination=False, stream=None):
-    n, c, hw = _nchw(probs)
-    _check(lib.nnf_softmax_nll_bwd(_stream(stream), _ptr(dlogits), _ptr(probs), _ptr(targets), _ptr(mask), scale, n, c, hw, int(add_to_destination)))
+    _native.softmax_nll_bwd(dlogits, probs, targets, mask, scale, add_to_destination, stream)
 
 
 def bn_train_sharded_supported(n, c, hw):
@@ -512,11 +468,7 @@ def bn_train_bwd_apply_peer(dx, dy, x, gamma, beta, saved, my_buf, world, kmax, 
 def apply_gradient(parts, momentum_type=MOMENTUM_NONE, momentum=0.9, momentum2=0.999, normalizer=1.0, iteration_id=1, stream=None):
     """parts: list of dicts {data, gradient, [prev_upd], [prev_upd2], [update_accum (float64 tensor of 1)], learning_rate,
     [weight_decay]}; every chunk of the list is updated by one launch (48 chunks per launch)."""
-    arr = (OptPart * max(len(parts), 1))()
-    for k, part in enumerate(parts):
-        arr[k] = OptPart(_ptr(part["data"]), _ptr(part["gradient"]), _ptr(part.get("prev_upd")), _ptr(part.get("prev_upd2")),
-                         _ptr(part.get("update_accum")), part["learning_rate"], part.get("weight_decay", 0.0), part["data"].numel())
-    _check(lib.nnf_apply_gradient(_stream(stream), arr, len(parts), momentum_type, momentum, momentum2, normalizer, iteration_id))
+    _native.apply_gradient(parts, momentum_type, momentum, momentum2, normalizer, iteration_id, stream)
 
 
 def bn_calibrate_accumulator(c, device="cuda"):

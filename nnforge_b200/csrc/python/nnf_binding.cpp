@@ -1,0 +1,846 @@
+// The call path between Python and the C ABI: one native function per entry point that a training or serving loop calls
+// every step. capi.py and host.py keep the signatures, the documentation and the checks of set-up calls; what a step pays
+// for is here. For a small tensor the host, not the GPU, is what bounds a call: the same call through ctypes spent 8 us on
+// attribute look-ups of its tensors, argument conversions and torch.cuda.current_stream(), against 2.4 us of GPU time for
+// batch norm + ReLU of one 64x32x32 image. Reading the tensors' addresses and extents from the objects themselves and the
+// stream from c10 costs a few tens of nanoseconds.
+//
+// The interpreter's lock is released around every call into the library, as ctypes does: a launch can block while the
+// stream's queue is full, and other threads keep enqueueing on theirs.
+#include <torch/csrc/autograd/python_variable.h>
+#include <c10/cuda/CUDAStream.h>
+
+#include "../../../include/nnf_b200.h"
+
+#include <vector>
+
+extern "C"
+{
+	// the flat interface of the layer objects (host/nnf_layers.cpp)
+	const char * nnfh_last_error(void);
+	int nnfh_tester_forward(void *, void *, void *, const void * const *, int, const void * const *, int, unsigned int);
+	int nnfh_updater_forward(void *, void *, void *, const void * const *, int, const void * const *, int, void *, size_t, void *, void *, unsigned int);
+	int nnfh_forward(void *, void *, void * const *, int, const void * const *, int, const void * const *, int, void *, size_t, void *, void *, unsigned int);
+	int nnfh_backward_data(void *, void *, unsigned int, void *, const void *, const void * const *, int, const void * const *, int, const void *, const void *,
+		const void *, int, unsigned int);
+	int nnfh_backward_weights(void *, void *, void * const *, int, const void * const *, int, const void *, void *, size_t, unsigned int);
+	int nnfh_backward_data_and_weights(void *, void *, void * const *, int, const void *, void * const *, int, const void * const *, int,
+		const void * const *, int, const void *, void *, size_t, void *, int, unsigned int);
+}
+
+namespace
+{
+	PyObject * g_error_type = nullptr;   // capi.NnfError
+
+	struct extents
+	{
+		int64_t n = 0, c = 0, h = 1, w = 1, hw = 1;
+	};
+
+	// Reads the positional arguments of one call in order. The first conversion that fails leaves its exception set, and
+	// the rest of the reads return zeros.
+	class arguments
+	{
+	public:
+		arguments(PyObject * const * a, Py_ssize_t n) : a(a), n(n) {}
+
+		bool ok() const { return good; }
+
+		PyObject * next()
+		{
+			if (i >= n)
+			{
+				if (good)
+					PyErr_SetString(PyExc_TypeError, "missing argument");
+				good = false;
+				return Py_None;
+			}
+			return a[i++];
+		}
+
+		// a tensor's address (None: null; an int: itself)
+		template <bool CHECKED = true>
+		void * address_of(PyObject * o)
+		{
+			if (o == Py_None)
+				return nullptr;
+			if (THPVariable_Check(o))
+			{
+				const at::Tensor& t = THPVariable_Unpack(o);
+				if (CHECKED && !(t.is_cuda() && t.is_contiguous()))
+					fail(PyExc_AssertionError, "tensors must be contiguous CUDA tensors");
+				return good ? t.data_ptr() : nullptr;
+			}
+			if (CHECKED && PyLong_Check(o))
+			{
+				void * p = PyLong_AsVoidPtr(o);
+				if (p == nullptr && PyErr_Occurred())
+					good = false;
+				return p;
+			}
+			fail(PyExc_TypeError, "a tensor, an address or None is expected");
+			return nullptr;
+		}
+		float * ptr() { return static_cast<float *>(address_of(next())); }
+		void * raw() { return address_of(next()); }
+		void * loose() { return address_of<false>(next()); }
+
+		const at::Tensor * tensor()
+		{
+			PyObject * o = next();
+			if (!THPVariable_Check(o))
+			{
+				fail(PyExc_TypeError, "a tensor is expected");
+				return nullptr;
+			}
+			return &THPVariable_Unpack(o);
+		}
+
+		// a tensor's address and its extents [n][c][h...][w]
+		float * ptr(extents& e, bool planes = false)
+		{
+			PyObject * o = next();
+			float * p = static_cast<float *>(address_of(o));
+			if (!good || !THPVariable_Check(o))
+			{
+				fail(PyExc_TypeError, "a tensor is expected");
+				return nullptr;
+			}
+			const auto s = THPVariable_Unpack(o).sizes();
+			if (s.size() < 2 || (planes && s.size() != 4))
+			{
+				fail(PyExc_ValueError, planes ? "a tensor [n][c][h][w] is expected" : "a tensor [n][c][...] is expected");
+				return nullptr;
+			}
+			e.n = s[0];
+			e.c = s[1];
+			for (size_t d = 2; d < s.size(); ++d)
+				e.hw *= s[d];
+			if (planes)
+			{
+				e.h = s[2];
+				e.w = s[3];
+			}
+			return p;
+		}
+
+		// a working buffer and its size in bytes (None: none of 0 bytes)
+		template <bool CHECKED = true>
+		void * buffer(size_t& bytes)
+		{
+			PyObject * o = next();
+			bytes = 0;
+			void * p = address_of<CHECKED>(o);
+			if (good && THPVariable_Check(o))
+				bytes = THPVariable_Unpack(o).nbytes();
+			return p;
+		}
+
+		double number()
+		{
+			PyObject * o = next();
+			const double v = PyFloat_CheckExact(o) ? PyFloat_AS_DOUBLE(o) : PyFloat_AsDouble(o);
+			if (v == -1.0 && PyErr_Occurred())
+				good = false;
+			return v;
+		}
+
+		long long integer()
+		{
+			const long long v = PyLong_AsLongLong(next());
+			if (v == -1 && PyErr_Occurred())
+				good = false;
+			return v;
+		}
+
+		int flag()
+		{
+			const int v = PyObject_IsTrue(next());
+			if (v < 0)
+				good = false;
+			return v;
+		}
+
+		void * handle()
+		{
+			PyObject * o = next();
+			if (o == Py_None)
+				return nullptr;
+			void * p = PyLong_AsVoidPtr(o);
+			if (p == nullptr && PyErr_Occurred())
+				good = false;
+			return p;
+		}
+
+		// torch's current stream unless one is given (an object with a cuda_stream, or the stream's address)
+		nnf_stream_t stream()
+		{
+			PyObject * o = next();
+			if (o == Py_None)
+				return (nnf_stream_t)c10::cuda::getCurrentCUDAStream().stream();
+			PyObject * v = PyObject_GetAttrString(o, "cuda_stream");
+			if (!v)
+			{
+				PyErr_Clear();
+				v = PyNumber_Long(o);
+			}
+			void * s = v ? PyLong_AsVoidPtr(v) : nullptr;
+			Py_XDECREF(v);
+			if (PyErr_Occurred())
+				good = false;
+			return (nnf_stream_t)s;
+		}
+
+		// the fields of one ctypes structure
+		template <class T>
+		void structure(PyObject * o, T& out)
+		{
+			Py_buffer b;
+			if (!good || PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) != 0)
+			{
+				good = false;
+				return;
+			}
+			if (b.len == (Py_ssize_t)sizeof(T))
+				memcpy(&out, b.buf, sizeof(T));
+			else
+				fail(PyExc_TypeError, "a structure of another size");
+			PyBuffer_Release(&b);
+		}
+
+		// an activation chain of any length (the library refuses those that are too long)
+		std::vector<nnf_act>& acts()
+		{
+			PyObject * o = next();
+			chain.clear();
+			if (o == Py_None)
+				return chain;
+			sequence(o, [&](PyObject * item) { nnf_act a = {}; structure(item, a); chain.push_back(a); });
+			return chain;
+		}
+
+		template <bool CHECKED>
+		void addresses(std::vector<void *>& out)
+		{
+			PyObject * o = next();
+			out.clear();
+			if (o != Py_None)
+				sequence(o, [&](PyObject * item) { out.push_back(address_of<CHECKED>(item)); });
+		}
+
+		template <class F>
+		void sequence(PyObject * o, F f)
+		{
+			PyObject * s = good ? PySequence_Fast(o, "a sequence is expected") : nullptr;
+			if (!s)
+			{
+				good = false;
+				return;
+			}
+			const Py_ssize_t count = PySequence_Fast_GET_SIZE(s);
+			for (Py_ssize_t k = 0; k < count && good; ++k)
+				f(PySequence_Fast_GET_ITEM(s, k));
+			Py_DECREF(s);
+		}
+
+		void fail(PyObject * type, const char * text)
+		{
+			if (good)
+				PyErr_SetString(type, text);
+			good = false;
+		}
+
+	private:
+		PyObject * const * a;
+		Py_ssize_t n, i = 0;
+		bool good = true;
+		std::vector<nnf_act> chain;
+	};
+
+	// calls the library without the interpreter's lock; a status raises NnfError with the library's text
+	template <class F>
+	PyObject * call(const arguments& a, F f)
+	{
+		if (!a.ok())
+			return nullptr;
+		int status;
+		Py_BEGIN_ALLOW_THREADS
+		status = f();
+		Py_END_ALLOW_THREADS
+		if (status == 0)
+			Py_RETURN_NONE;
+		PyObject * e = PyObject_CallFunction(g_error_type ? g_error_type : PyExc_RuntimeError, "is", status, nnf_last_error_string());
+		if (e)
+		{
+			PyErr_SetObject((PyObject *)Py_TYPE(e), e);
+			Py_DECREF(e);
+		}
+		return nullptr;
+	}
+
+	// the same for the layer objects, whose errors host.py raises
+	template <class F>
+	PyObject * call_object(const arguments& a, F f)
+	{
+		if (!a.ok())
+			return nullptr;
+		int status;
+		Py_BEGIN_ALLOW_THREADS
+		status = f();
+		Py_END_ALLOW_THREADS
+		return PyLong_FromLong(status);
+	}
+
+	#define NNF_NATIVE(name) PyObject * name(PyObject *, PyObject * const * args, Py_ssize_t nargs)
+	#define NNF_READ arguments a(args, nargs)
+
+	// (gamma, beta, mean, invsigma) or None
+	struct bn_arrays
+	{
+		const float * gamma = nullptr, * beta = nullptr, * mean = nullptr, * invsigma = nullptr;
+
+		explicit bn_arrays(arguments& a)
+		{
+			PyObject * o = a.next();
+			if (o == Py_None)
+				return;
+			const float * p[4] = {};
+			int k = 0;
+			a.sequence(o, [&](PyObject * item) { const float * v = static_cast<const float *>(a.address_of(item)); if (k < 4) p[k] = v; ++k; });
+			if (k != 4)
+				a.fail(PyExc_ValueError, "batch norm takes (gamma, beta, mean, invsigma)");
+			gamma = p[0]; beta = p[1]; mean = p[2]; invsigma = p[3];
+		}
+	};
+
+	NNF_NATIVE(bn_infer_act)   // y, x, bias, bn, residual, add_alpha, acts, stream
+	{
+		NNF_READ;
+		extents e;
+		float * y = a.ptr();
+		const float * x = a.ptr(e), * bias = a.ptr();
+		const bn_arrays bn(a);
+		const float * residual = a.ptr();
+		const float alpha = (float)a.number();
+		const auto& acts = a.acts();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return !bias ? nnf_bn_infer_act(s, y, x, bn.gamma, bn.beta, bn.mean, bn.invsigma, residual, alpha, acts.data(), (int)acts.size(), e.n, e.c, e.hw)
+			: nnf_bias_bn_infer_act(s, y, x, bias, bn.gamma, bn.beta, bn.mean, bn.invsigma, residual, alpha, acts.data(), (int)acts.size(), e.n, e.c, e.hw); });
+	}
+
+	NNF_NATIVE(act_fwd)   // y, x, act, stream
+	{
+		NNF_READ;
+		extents e;
+		nnf_act act = {};
+		float * y = a.ptr();
+		const float * x = a.ptr(e);
+		a.structure(a.next(), act);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_act_fwd(s, y, x, &act, e.n, e.c, e.hw); });
+	}
+
+	NNF_NATIVE(act_bwd)   // dx, dy, neurons, act, add_to_destination, stream
+	{
+		NNF_READ;
+		extents e;
+		nnf_act act = {};
+		float * dx = a.ptr();
+		const float * dy = a.ptr(e), * neurons = a.ptr();
+		a.structure(a.next(), act);
+		const int add = a.flag();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_act_bwd(s, dx, dy, neurons, &act, e.n, e.c, e.hw, add); });
+	}
+
+	NNF_NATIVE(prelu_bwd_weights)   // dslope, dy, x, workspace, stream
+	{
+		NNF_READ;
+		extents e;
+		float * dslope = a.ptr();
+		const float * dy = a.ptr(), * x = a.ptr(e);
+		size_t bytes;
+		void * ws = a.buffer(bytes);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_prelu_bwd_weights(s, dslope, dy, x, e.n, e.c, e.hw, ws, bytes); });
+	}
+
+	NNF_NATIVE(add_fwd)   // y, inputs, alpha, stream
+	{
+		NNF_READ;
+		const at::Tensor * t = a.tensor();
+		float * y = a.ok() ? static_cast<float *>(a.address_of(args[0])) : nullptr;
+		std::vector<void *> in;
+		a.addresses<true>(in);
+		const float alpha = (float)a.number();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_add_fwd(s, y, (const float * const *)in.data(), (int)in.size(), alpha, t->numel()); });
+	}
+
+	NNF_NATIVE(add_bwd)   // dx, dy, alpha, add_to_destination, stream
+	{
+		NNF_READ;
+		float * dx = a.ptr();
+		const at::Tensor * t = a.tensor();
+		const float * dy = a.ok() ? static_cast<const float *>(a.address_of(args[1])) : nullptr;
+		const float alpha = (float)a.number();
+		const int add = a.flag();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_add_bwd(s, dx, dy, alpha, t->numel(), add); });
+	}
+
+	NNF_NATIVE(softmax_fwd)   // y, x, stream
+	{
+		NNF_READ;
+		extents e;
+		float * y = a.ptr();
+		const float * x = a.ptr(e);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_softmax_fwd(s, y, x, e.n, e.c, e.hw); });
+	}
+
+	NNF_NATIVE(softmax_bwd)   // dx, dy, y, add_to_destination, stream
+	{
+		NNF_READ;
+		extents e;
+		float * dx = a.ptr();
+		const float * dy = a.ptr(), * y = a.ptr(e);
+		const int add = a.flag();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_softmax_bwd(s, dx, dy, y, e.n, e.c, e.hw, add); });
+	}
+
+	NNF_NATIVE(maxpool_fwd)   // y, argmax, x, pool, stream
+	{
+		NNF_READ;
+		extents e;
+		nnf_pool pool = {};
+		float * y = a.ptr();
+		uint32_t * argmax = static_cast<uint32_t *>(a.raw());
+		const float * x = a.ptr(e, true);
+		a.structure(a.next(), pool);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_maxpool_fwd(s, y, argmax, x, e.n, e.c, e.h, e.w, &pool); });
+	}
+
+	NNF_NATIVE(maxpool_bwd)   // dx, dy, argmax, pool, add_to_destination, stream
+	{
+		NNF_READ;
+		extents e;
+		nnf_pool pool = {};
+		float * dx = a.ptr(e, true);
+		const float * dy = a.ptr();
+		const uint32_t * argmax = static_cast<const uint32_t *>(a.raw());
+		a.structure(a.next(), pool);
+		const int add = a.flag();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_maxpool_bwd(s, dx, dy, argmax, e.n, e.c, e.h, e.w, &pool, add); });
+	}
+
+	NNF_NATIVE(bn_add_relu_maxpool_fwd)   // z, pooled, argmax, x, residual, bn, relu_slope, pool, stream
+	{
+		NNF_READ;
+		extents e;
+		nnf_pool pool = {};
+		float * z = a.ptr(), * pooled = a.ptr();
+		uint32_t * argmax = static_cast<uint32_t *>(a.raw());
+		const float * x = a.ptr(e, true), * residual = a.ptr();
+		const bn_arrays bn(a);
+		const float slope = (float)a.number();
+		a.structure(a.next(), pool);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_add_relu_maxpool_fwd(s, z, pooled, argmax, x, residual, bn.gamma, bn.beta, bn.mean, bn.invsigma, slope, e.n, e.c, e.h, e.w, &pool); });
+	}
+
+	NNF_NATIVE(bn_add_relu_maxpool_bwd)   // dx, dresidual, dpooled, argmax, z, gamma, invsigma, relu_slope, pool, stream
+	{
+		NNF_READ;
+		extents e;
+		nnf_pool pool = {};
+		float * dx = a.ptr(), * dresidual = a.ptr();
+		const float * dpooled = a.ptr();
+		const uint32_t * argmax = static_cast<const uint32_t *>(a.raw());
+		const float * z = a.ptr(e, true), * gamma = a.ptr(), * invsigma = a.ptr();
+		const float slope = (float)a.number();
+		a.structure(a.next(), pool);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_add_relu_maxpool_bwd(s, dx, dresidual, dpooled, argmax, z, gamma, invsigma, slope, e.n, e.c, e.h, e.w, &pool); });
+	}
+
+	NNF_NATIVE(bn_train_stats)   // sums, x, workspace, stream
+	{
+		NNF_READ;
+		extents e;
+		float * sums = a.ptr();
+		const float * x = a.ptr(e);
+		size_t bytes;
+		void * ws = a.buffer(bytes);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_train_stats(s, sums, x, e.n, e.c, e.hw, ws, bytes); });
+	}
+
+	NNF_NATIVE(bn_train_stats_static)   // sums, x, stream
+	{
+		NNF_READ;
+		extents e;
+		float * sums = a.ptr();
+		const float * x = a.ptr(e);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_train_stats_static(s, sums, x, e.n, e.c, e.hw); });
+	}
+
+	NNF_NATIVE(bn_train_apply_act)   // y, saved, x, gamma, beta, sums, count_total, eps, acts, stream
+	{
+		NNF_READ;
+		extents e;
+		float * y = a.ptr(), * saved = a.ptr();
+		const float * x = a.ptr(e), * gamma = a.ptr(), * beta = a.ptr(), * sums = a.ptr();
+		const double count = a.number();
+		const float eps = (float)a.number();
+		const auto& acts = a.acts();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_train_apply_act(s, y, saved, x, gamma, beta, sums, count, eps, acts.data(), (int)acts.size(), e.n, e.c, e.hw); });
+	}
+
+	NNF_NATIVE(bn_train_fwd)   // y, saved, sums, x, gamma, beta, eps, acts, workspace, stream
+	{
+		NNF_READ;
+		extents e;
+		float * y = a.ptr(), * saved = a.ptr(), * sums = a.ptr();
+		const float * x = a.ptr(e), * gamma = a.ptr(), * beta = a.ptr();
+		const float eps = (float)a.number();
+		const auto& acts = a.acts();
+		size_t bytes;
+		void * ws = a.buffer(bytes);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_train_fwd(s, y, saved, sums, x, gamma, beta, eps, acts.data(), (int)acts.size(), e.n, e.c, e.hw, ws, bytes); });
+	}
+
+	NNF_NATIVE(bn_train_bwd)   // dx, bsums, dy, x, gamma, beta, saved, acts, 5 gradients, mean, invsigma, entry_count, add_to_destination, workspace, stream
+	{
+		NNF_READ;
+		extents e;
+		float * dx = a.ptr(), * bsums = a.ptr();
+		const float * dy = a.ptr(), * x = a.ptr(e), * gamma = a.ptr(), * beta = a.ptr(), * saved = a.ptr();
+		const auto& acts = a.acts();
+		float * gg = a.ptr(), * gb = a.ptr(), * gm = a.ptr(), * gi = a.ptr(), * gs = a.ptr();
+		const float * mean = a.ptr(), * invsigma = a.ptr();
+		const float entries = (float)a.number();
+		const int add = a.flag();
+		size_t bytes;
+		void * ws = a.buffer(bytes);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_train_bwd(s, dx, bsums, dy, x, gamma, beta, saved, acts.data(), (int)acts.size(), gg, gb, gm, gi, gs, mean, invsigma, entries, e.n, e.c, e.hw, add, ws, bytes); });
+	}
+
+	NNF_NATIVE(bn_train_bwd_stats)   // bsums, gsums, dy, x, gamma, beta, saved, acts, workspace, stream
+	{
+		NNF_READ;
+		extents e;
+		float * bsums = a.ptr(), * gsums = a.ptr();
+		const float * dy = a.ptr(), * x = a.ptr(e), * gamma = a.ptr(), * beta = a.ptr(), * saved = a.ptr();
+		const auto& acts = a.acts();
+		size_t bytes;
+		void * ws = a.buffer(bytes);
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_train_bwd_stats(s, bsums, gsums, dy, x, gamma, beta, saved, acts.data(), (int)acts.size(), e.n, e.c, e.hw, ws, bytes); });
+	}
+
+	NNF_NATIVE(bn_train_bwd_apply)   // dx, dy, x, gamma, beta, saved, gsums, bsums, count_total, acts, 5 gradients, mean, invsigma, entry_count, add, stream
+	{
+		NNF_READ;
+		extents e;
+		float * dx = a.ptr();
+		const float * dy = a.ptr(), * x = a.ptr(e), * gamma = a.ptr(), * beta = a.ptr(), * saved = a.ptr(), * gsums = a.ptr(), * bsums = a.ptr();
+		const double count = a.number();
+		const auto& acts = a.acts();
+		float * gg = a.ptr(), * gb = a.ptr(), * gm = a.ptr(), * gi = a.ptr(), * gs = a.ptr();
+		const float * mean = a.ptr(), * invsigma = a.ptr();
+		const float entries = (float)a.number();
+		const int add = a.flag();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_train_bwd_apply(s, dx, dy, x, gamma, beta, saved, gsums, bsums, count, acts.data(), (int)acts.size(), gg, gb, gm, gi, gs, mean, invsigma, entries, e.n, e.c, e.hw, add); });
+	}
+
+	NNF_NATIVE(avgpool_fwd)   // y, x, win_w, win_h, mult, stream
+	{
+		NNF_READ;
+		extents e;
+		float * y = a.ptr();
+		const float * x = a.ptr(e, true);
+		const int ww = (int)a.integer(), wh = (int)a.integer();
+		const float mult = (float)a.number();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_avgpool_fwd(s, y, x, e.n, e.c, e.h, e.w, ww, wh, mult); });
+	}
+
+	NNF_NATIVE(avgpool_bwd)   // dx, dy, win_w, win_h, mult, add_to_destination, stream
+	{
+		NNF_READ;
+		extents e;
+		float * dx = a.ptr(e, true);
+		const float * dy = a.ptr();
+		const int ww = (int)a.integer(), wh = (int)a.integer();
+		const float mult = (float)a.number();
+		const int add = a.flag();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_avgpool_bwd(s, dx, dy, e.n, e.c, e.h, e.w, ww, wh, mult, add); });
+	}
+
+	NNF_NATIVE(bn_add_relu_avgpool_fwd)   // z, pooled, x, residual, bn, relu_slope, win_w, win_h, mult, stream
+	{
+		NNF_READ;
+		extents e;
+		float * z = a.ptr(), * pooled = a.ptr();
+		const float * x = a.ptr(e, true), * residual = a.ptr();
+		const bn_arrays bn(a);
+		const float slope = (float)a.number();
+		const int ww = (int)a.integer(), wh = (int)a.integer();
+		const float mult = (float)a.number();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_add_relu_avgpool_fwd(s, z, pooled, x, residual, bn.gamma, bn.beta, bn.mean, bn.invsigma, slope, e.n, e.c, e.h, e.w, ww, wh, mult); });
+	}
+
+	NNF_NATIVE(bn_add_relu_avgpool_bwd)   // dx, dresidual, dpooled, z, gamma, invsigma, relu_slope, win_w, win_h, mult, stream
+	{
+		NNF_READ;
+		extents e;
+		float * dx = a.ptr(), * dresidual = a.ptr();
+		const float * dpooled = a.ptr(), * z = a.ptr(e, true), * gamma = a.ptr(), * invsigma = a.ptr();
+		const float slope = (float)a.number();
+		const int ww = (int)a.integer(), wh = (int)a.integer();
+		const float mult = (float)a.number();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_bn_add_relu_avgpool_bwd(s, dx, dresidual, dpooled, z, gamma, invsigma, slope, e.n, e.c, e.h, e.w, ww, wh, mult); });
+	}
+
+	NNF_NATIVE(accuracy_fwd)   // out, predicted, targets, mask, top_n, stream
+	{
+		NNF_READ;
+		extents e;
+		float * out = a.ptr();
+		const float * predicted = a.ptr(e), * targets = a.ptr(), * mask = a.ptr();
+		const int top_n = (int)a.integer();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_accuracy_fwd(s, out, predicted, targets, mask, top_n, e.n, e.c, e.hw); });
+	}
+
+	// err, predicted, targets, mask, scale, stream
+	template <int (*F)(nnf_stream_t, float *, const float *, const float *, const float *, float, int64_t, int64_t, int64_t)>
+	NNF_NATIVE(loss_fwd)
+	{
+		NNF_READ;
+		extents e;
+		float * err = a.ptr();
+		const float * predicted = a.ptr(e), * targets = a.ptr(), * mask = a.ptr();
+		const float scale = (float)a.number();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return F(s, err, predicted, targets, mask, scale, e.n, e.c, e.hw); });
+	}
+
+	// dpredicted, predicted, targets, mask, scale, add_to_destination, stream
+	template <int (*F)(nnf_stream_t, float *, const float *, const float *, const float *, float, int64_t, int64_t, int64_t, int)>
+	NNF_NATIVE(loss_bwd)
+	{
+		NNF_READ;
+		extents e;
+		float * d = a.ptr();
+		const float * predicted = a.ptr(e), * targets = a.ptr(), * mask = a.ptr();
+		const float scale = (float)a.number();
+		const int add = a.flag();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return F(s, d, predicted, targets, mask, scale, e.n, e.c, e.hw, add); });
+	}
+
+	NNF_NATIVE(softmax_nll_fwd)   // probs, err, logits, targets, mask, scale, stream
+	{
+		NNF_READ;
+		extents e;
+		float * probs = a.ptr(), * err = a.ptr();
+		const float * logits = a.ptr(e), * targets = a.ptr(), * mask = a.ptr();
+		const float scale = (float)a.number();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_softmax_nll_fwd(s, probs, err, logits, targets, mask, scale, e.n, e.c, e.hw); });
+	}
+
+	// the keys of one chunk's dict, interned once
+	struct part_keys
+	{
+		PyObject * data = PyUnicode_InternFromString("data"), * gradient = PyUnicode_InternFromString("gradient"),
+			* prev_upd = PyUnicode_InternFromString("prev_upd"), * prev_upd2 = PyUnicode_InternFromString("prev_upd2"),
+			* update_accum = PyUnicode_InternFromString("update_accum"), * learning_rate = PyUnicode_InternFromString("learning_rate"),
+			* weight_decay = PyUnicode_InternFromString("weight_decay");
+	};
+
+	NNF_NATIVE(apply_gradient)   // parts, momentum_type, momentum, momentum2, normalizer, iteration_id, stream
+	{
+		static const part_keys keys;
+		NNF_READ;
+		std::vector<nnf_opt_part> parts;
+		a.sequence(a.next(), [&](PyObject * d)
+		{
+			// borrowed references; a key that has to be there raises KeyError as d[key] does
+			auto get = [&](PyObject * key, bool needed) -> PyObject *
+			{
+				if (!PyDict_Check(d))
+				{
+					a.fail(PyExc_TypeError, "a chunk is a dict");
+					return Py_None;
+				}
+				PyObject * v = PyDict_GetItemWithError(d, key);
+				if (v)
+					return v;
+				if (needed && !PyErr_Occurred())
+					PyErr_SetObject(PyExc_KeyError, key);
+				if (PyErr_Occurred())
+					a.fail(PyExc_KeyError, "");
+				return Py_None;
+			};
+			auto number = [&](PyObject * o) { const double v = PyFloat_AsDouble(o); if (v == -1.0 && PyErr_Occurred()) a.fail(PyExc_TypeError, "a number is expected"); return (float)v; };
+			nnf_opt_part p = {};
+			PyObject * data = get(keys.data, true);
+			p.data = static_cast<float *>(a.address_of(data));
+			p.gradient = static_cast<float *>(a.address_of(get(keys.gradient, true)));
+			p.prev_upd = static_cast<float *>(a.address_of(get(keys.prev_upd, false)));
+			p.prev_upd2 = static_cast<float *>(a.address_of(get(keys.prev_upd2, false)));
+			p.update_accum = static_cast<double *>(a.address_of(get(keys.update_accum, false)));
+			PyObject * rate = get(keys.learning_rate, true);
+			if (!a.ok())
+				return;
+			p.learning_rate = number(rate);
+			PyObject * decay = get(keys.weight_decay, false);
+			p.weight_decay = decay == Py_None ? 0.0F : number(decay);
+			if (!THPVariable_Check(data))
+			{
+				a.fail(PyExc_TypeError, "a chunk's data is a tensor");
+				return;
+			}
+			p.elem_count = THPVariable_Unpack(data).numel();
+			parts.push_back(p);
+		});
+		const int type = (int)a.integer();
+		const float m1 = (float)a.number(), m2 = (float)a.number(), normalizer = (float)a.number();
+		const unsigned int iteration = (unsigned int)a.integer();
+		const nnf_stream_t s = a.stream();
+		return call(a, [&] { return nnf_apply_gradient(s, parts.data(), (int)parts.size(), type, m1, m2, normalizer, iteration); });
+	}
+
+	// ---- layer objects (host.py) ---------------------------------------------------------------------
+	nnf_stream_t current_stream() { return (nnf_stream_t)c10::cuda::getCurrentCUDAStream().stream(); }
+
+	NNF_NATIVE(tester_forward)   // handle, output, data, inputs, entry_count
+	{
+		NNF_READ;
+		std::vector<void *> data, in;
+		void * h = a.handle(), * out = a.loose();
+		a.addresses<false>(data);
+		a.addresses<false>(in);
+		const unsigned int n = (unsigned int)a.integer();
+		return call_object(a, [&] { return nnfh_tester_forward(h, current_stream(), out, data.data(), (int)data.size(), in.data(), (int)in.size(), n); });
+	}
+
+	NNF_NATIVE(updater_forward)   // handle, output, data, inputs, working, fixed, per_entry, entry_count
+	{
+		NNF_READ;
+		std::vector<void *> data, in;
+		void * h = a.handle(), * out = a.loose();
+		a.addresses<false>(data);
+		a.addresses<false>(in);
+		size_t bytes;
+		void * ws = a.buffer<false>(bytes), * fixed = a.loose(), * per_entry = a.loose();
+		const unsigned int n = (unsigned int)a.integer();
+		return call_object(a, [&] { return nnfh_updater_forward(h, current_stream(), out, data.data(), (int)data.size(), in.data(), (int)in.size(), ws, bytes, fixed, per_entry, n); });
+	}
+
+	NNF_NATIVE(object_forward)   // handle, outputs, data, inputs, working, fixed, per_entry, entry_count
+	{
+		NNF_READ;
+		std::vector<void *> out, data, in;
+		void * h = a.handle();
+		a.addresses<false>(out);
+		a.addresses<false>(data);
+		a.addresses<false>(in);
+		size_t bytes;
+		void * ws = a.buffer<false>(bytes), * fixed = a.loose(), * per_entry = a.loose();
+		const unsigned int n = (unsigned int)a.integer();
+		return call_object(a, [&] { return nnfh_forward(h, current_stream(), out.data(), (int)out.size(), data.data(), (int)data.size(), in.data(), (int)in.size(), ws, bytes, fixed, per_entry, n); });
+	}
+
+	NNF_NATIVE(object_backward_data)   // handle, input_index, input_errors, output_errors, data, input_neurons, output_neurons, fixed, per_entry, add, entry_count
+	{
+		NNF_READ;
+		std::vector<void *> data, in;
+		void * h = a.handle();
+		const unsigned int index = (unsigned int)a.integer();
+		void * ie = a.loose(), * oe = a.loose();
+		a.addresses<false>(data);
+		a.addresses<false>(in);
+		void * on = a.loose(), * fixed = a.loose(), * per_entry = a.loose();
+		const int add = a.flag();
+		const unsigned int n = (unsigned int)a.integer();
+		return call_object(a, [&] { return nnfh_backward_data(h, current_stream(), index, ie, oe, data.data(), (int)data.size(), in.data(), (int)in.size(), on, fixed, per_entry, add, n); });
+	}
+
+	NNF_NATIVE(object_backward_weights)   // handle, gradient, input_neurons, output_errors, working, entry_count
+	{
+		NNF_READ;
+		std::vector<void *> gradient, in;
+		void * h = a.handle();
+		a.addresses<false>(gradient);
+		a.addresses<false>(in);
+		void * oe = a.loose();
+		size_t bytes;
+		void * ws = a.buffer<false>(bytes);
+		const unsigned int n = (unsigned int)a.integer();
+		return call_object(a, [&] { return nnfh_backward_weights(h, current_stream(), gradient.data(), (int)gradient.size(), in.data(), (int)in.size(), oe, ws, bytes, n); });
+	}
+
+	NNF_NATIVE(object_backward_data_and_weights)   // handle, input_errors, output_errors, gradient, data, input_neurons, output_neurons, working, fixed, add, entry_count
+	{
+		NNF_READ;
+		std::vector<void *> ie, gradient, data, in;
+		void * h = a.handle();
+		a.addresses<false>(ie);
+		void * oe = a.loose();
+		a.addresses<false>(gradient);
+		a.addresses<false>(data);
+		a.addresses<false>(in);
+		void * on = a.loose();
+		size_t bytes;
+		void * ws = a.buffer<false>(bytes), * fixed = a.loose();
+		const int add = a.flag();
+		const unsigned int n = (unsigned int)a.integer();
+		return call_object(a, [&] { return nnfh_backward_data_and_weights(h, current_stream(), ie.data(), (int)ie.size(), oe, gradient.data(), (int)gradient.size(),
+			data.data(), (int)data.size(), in.data(), (int)in.size(), on, ws, bytes, fixed, add, n); });
+	}
+
+	PyObject * set_error_type(PyObject *, PyObject * type)
+	{
+		Py_INCREF(type);
+		Py_XSETREF(g_error_type, type);
+		Py_RETURN_NONE;
+	}
+
+	#define NNF_ENTRY(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
+	#define NNF_ENTRY_AS(name, ...) {name, (PyCFunction)(void (*)(void))__VA_ARGS__, METH_FASTCALL, nullptr}
+	PyMethodDef g_methods[] = {
+		NNF_ENTRY(bn_infer_act), NNF_ENTRY(act_fwd), NNF_ENTRY(act_bwd), NNF_ENTRY(prelu_bwd_weights), NNF_ENTRY(add_fwd), NNF_ENTRY(add_bwd),
+		NNF_ENTRY(softmax_fwd), NNF_ENTRY(softmax_bwd), NNF_ENTRY(maxpool_fwd), NNF_ENTRY(maxpool_bwd), NNF_ENTRY(bn_add_relu_maxpool_fwd),
+		NNF_ENTRY(bn_add_relu_maxpool_bwd), NNF_ENTRY(bn_train_stats), NNF_ENTRY(bn_train_stats_static), NNF_ENTRY(bn_train_apply_act),
+		NNF_ENTRY(bn_train_fwd), NNF_ENTRY(bn_train_bwd), NNF_ENTRY(bn_train_bwd_stats), NNF_ENTRY(bn_train_bwd_apply), NNF_ENTRY(avgpool_fwd),
+		NNF_ENTRY(avgpool_bwd), NNF_ENTRY(bn_add_relu_avgpool_fwd), NNF_ENTRY(bn_add_relu_avgpool_bwd), NNF_ENTRY(accuracy_fwd),
+		NNF_ENTRY_AS("nll_fwd", loss_fwd<nnf_nll_fwd>), NNF_ENTRY_AS("nll_bwd", loss_bwd<nnf_nll_bwd>),
+		NNF_ENTRY_AS("cross_entropy_fwd", loss_fwd<nnf_cross_entropy_fwd>), NNF_ENTRY_AS("cross_entropy_bwd", loss_bwd<nnf_cross_entropy_bwd>),
+		NNF_ENTRY(softmax_nll_fwd), NNF_ENTRY_AS("softmax_nll_bwd", loss_bwd<nnf_softmax_nll_bwd>), NNF_ENTRY(apply_gradient),
+		NNF_ENTRY(tester_forward), NNF_ENTRY(updater_forward), NNF_ENTRY(object_forward), NNF_ENTRY(object_backward_data),
+		NNF_ENTRY(object_backward_weights), NNF_ENTRY(object_backward_data_and_weights),
+		{"set_error_type", set_error_type, METH_O, nullptr},
+		{nullptr, nullptr, 0, nullptr}};
+
+	PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "Call path between Python and the C ABI.", -1, g_methods, nullptr, nullptr, nullptr, nullptr};
+}
+
+PyMODINIT_FUNC PyInit__native(void)
+{
+	return PyModule_Create(&g_module);
+}

@@ -9,6 +9,8 @@ import os
 
 import torch
 
+from . import _native
+
 HERE = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(HERE, "libnnf_b200_host.so")
 if not os.path.exists(LIB_PATH):
@@ -101,9 +103,7 @@ class Tester(_Layer):
         super().__init__(type_name, False, feature_maps, w, h, **kw)
 
     def enqueue_forward_propagation(self, output_buffer, data, input_buffers, entry_count):
-        d, nd = _arr(data)
-        i, ni = _arr(input_buffers)
-        _check(lib.nnfh_tester_forward(self.h, _stream(), _ptr(output_buffer), d, nd, i, ni, entry_count))
+        _check(_native.tester_forward(self.h, output_buffer, data, input_buffers, entry_count))
 
     def get_input_index_layer_can_write(self):
         return lib.nnfh_tester_can_write(self.h)
@@ -133,11 +133,8 @@ class Updater(_Layer):
 
     def enqueue_forward_propagation(self, output_buffer, data, input_buffers, entry_count, temporary_working_fixed_buffer=None,
                                     temporary_fixed_buffer=None, temporary_per_entry_buffer=None):
-        d, nd = _arr(data)
-        i, ni = _arr(input_buffers)
-        wf = temporary_working_fixed_buffer
-        _check(lib.nnfh_updater_forward(self.h, _stream(), _ptr(output_buffer), d, nd, i, ni, _ptr(wf), wf.numel() * wf.element_size() if wf is not None else 0,
-                                        _ptr(temporary_fixed_buffer), _ptr(temporary_per_entry_buffer), entry_count))
+        _check(_native.updater_forward(self.h, output_buffer, data, input_buffers, temporary_working_fixed_buffer, temporary_fixed_buffer,
+                                       temporary_per_entry_buffer, entry_count))
 
     def enqueue_backward_data_propagation(self, input_errors_buffer, output_errors_buffer, data, input_neurons_buffer, output_neurons_buffer, entry_count,
                                           temporary_fixed_buffer=None, temporary_per_entry_buffer=None, add_update_to_destination=False):
@@ -246,37 +243,23 @@ class LayerObject:
 
     def enqueue_forward_propagation(self, output_buffers, data, input_buffers, entry_count, temporary_working_fixed_buffer=None,
                                     temporary_fixed_buffer=None, temporary_per_entry_buffer=None):
-        o, no = _arr(output_buffers)
-        d, nd = _arr(data)
-        i, ni = _arr(input_buffers)
-        wf = temporary_working_fixed_buffer
-        _check(lib.nnfh_forward(self.h, _stream(), o, no, d, nd, i, ni, _ptr(wf), _bytes(wf), _ptr(temporary_fixed_buffer), _ptr(temporary_per_entry_buffer),
-                                entry_count))
+        _check(_native.object_forward(self.h, output_buffers, data, input_buffers, temporary_working_fixed_buffer, temporary_fixed_buffer,
+                                      temporary_per_entry_buffer, entry_count))
 
     def enqueue_backward_data_propagation(self, input_index, input_errors_buffer, output_errors_buffer, data, input_neurons_buffers, output_neurons_buffer,
                                           entry_count, temporary_fixed_buffer=None, temporary_per_entry_buffer=None, add_update_to_destination=False):
-        d, nd = _arr(data)
-        i, ni = _arr(input_neurons_buffers)
-        _check(lib.nnfh_backward_data(self.h, _stream(), input_index, _ptr(input_errors_buffer), _ptr(output_errors_buffer), d, nd, i, ni,
-                                      _ptr(output_neurons_buffer), _ptr(temporary_fixed_buffer), _ptr(temporary_per_entry_buffer),
-                                      int(add_update_to_destination), entry_count))
+        _check(_native.object_backward_data(self.h, input_index, input_errors_buffer, output_errors_buffer, data, input_neurons_buffers,
+                                            output_neurons_buffer, temporary_fixed_buffer, temporary_per_entry_buffer, add_update_to_destination, entry_count))
 
     def enqueue_backward_weights_propagation(self, gradient, input_neurons_buffers, output_errors_buffer, entry_count, temporary_working_fixed_buffer=None):
-        g, ng = _arr(gradient)
-        i, ni = _arr(input_neurons_buffers)
-        wf = temporary_working_fixed_buffer
-        _check(lib.nnfh_backward_weights(self.h, _stream(), g, ng, i, ni, _ptr(output_errors_buffer), _ptr(wf), _bytes(wf), entry_count))
+        _check(_native.object_backward_weights(self.h, gradient, input_neurons_buffers, output_errors_buffer, temporary_working_fixed_buffer, entry_count))
 
     def enqueue_backward_data_and_weights_propagation(self, input_errors_buffers, output_errors_buffer, gradient, data, input_neurons_buffers,
                                                       output_neurons_buffer, entry_count, temporary_working_fixed_buffer=None, temporary_fixed_buffer=None,
                                                       add_update_to_destination=False):
-        e, ne = _arr(input_errors_buffers)
-        g, ng = _arr(gradient)
-        d, nd = _arr(data)
-        i, ni = _arr(input_neurons_buffers)
-        wf = temporary_working_fixed_buffer
-        _check(lib.nnfh_backward_data_and_weights(self.h, _stream(), e, ne, _ptr(output_errors_buffer), g, ng, d, nd, i, ni, _ptr(output_neurons_buffer),
-                                                  _ptr(wf), _bytes(wf), _ptr(temporary_fixed_buffer), int(add_update_to_destination), entry_count))
+        _check(_native.object_backward_data_and_weights(self.h, input_errors_buffers, output_errors_buffer, gradient, data, input_neurons_buffers,
+                                                        output_neurons_buffer, temporary_working_fixed_buffer, temporary_fixed_buffer,
+                                                        add_update_to_destination, entry_count))
 
     def get_data(self, host_parts):
         """Uploads the weight chunks (lists / numpy arrays of float32) through the object's get_data; returns CUDA tensors viewing
