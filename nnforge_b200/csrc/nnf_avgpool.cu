@@ -42,6 +42,7 @@ namespace nnf
 		template <bool FUSED>
 		__global__ void __launch_bounds__(kAvgThreads) avgpool_fwd_kernel(const avg_params p)
 		{
+			pdl_begin();
 			extern __shared__ float s_z[];
 			__shared__ float s_mult[FUSED ? kAvgMaxGroup : 1];
 			__shared__ float s_add[FUSED ? kAvgMaxGroup : 1];
@@ -172,6 +173,7 @@ namespace nnf
 		// (((0 + x00) + x01) + x10) + x11. No shared memory, every access 8 or 16 bytes wide.
 		__global__ void __launch_bounds__(kAvgThreads) avgpool_fwd_2x2_kernel(float * pooled, const float * x, int64_t out_rows, uint32_t w4, fastdiv d_w4, float mult)
 		{
+			pdl_begin();
 			const int64_t total = out_rows * w4;
 			const int64_t stride = int64_t(gridDim.x) * kAvgThreads * 2;
 			for (int64_t i0 = int64_t(blockIdx.x) * kAvgThreads * 2 + threadIdx.x; i0 < total; i0 += stride)
@@ -210,6 +212,7 @@ namespace nnf
 		// the same for rows of whole float2s only (14x14): one output per thread
 		__global__ void __launch_bounds__(kAvgThreads) avgpool_fwd_2x2_pair_kernel(float * pooled, const float * x, int64_t out_rows, uint32_t w2, fastdiv d_w2, float mult)
 		{
+			pdl_begin();
 			const int64_t total = out_rows * w2;
 			const int64_t stride = int64_t(gridDim.x) * kAvgThreads * 4;
 			for (int64_t i0 = int64_t(blockIdx.x) * kAvgThreads * 4 + threadIdx.x; i0 < total; i0 += stride)
@@ -242,6 +245,7 @@ namespace nnf
 		// into, the two float2s of its window
 		__global__ void __launch_bounds__(kAvgThreads) avgpool_bwd_2x2_pair_kernel(float * dx, const float * dy, int64_t out_rows, uint32_t w2, fastdiv d_w2, float mult, int add)
 		{
+			pdl_begin();
 			const int64_t total = out_rows * w2;
 			const int64_t stride = int64_t(gridDim.x) * kAvgThreads * 4;
 			for (int64_t i0 = int64_t(blockIdx.x) * kAvgThreads * 4 + threadIdx.x; i0 < total; i0 += stride)
@@ -280,6 +284,7 @@ namespace nnf
 		// planes too large for shared memory: one thread per output reads its window from global memory
 		__global__ void __launch_bounds__(kAvgThreads) avgpool_fwd_direct_kernel(const avg_params p)
 		{
+			pdl_begin();
 			const int64_t total = p.planes * p.ohw;
 			const int64_t stride = int64_t(gridDim.x) * kAvgThreads;
 			for (int64_t o = int64_t(blockIdx.x) * kAvgThreads + threadIdx.x; o < total; o += stride)
@@ -300,6 +305,7 @@ namespace nnf
 		template <bool FUSED>
 		__global__ void __launch_bounds__(kAvgThreads) avgpool_bwd_kernel(const avg_params p, int64_t base, uint32_t count)
 		{
+			pdl_begin();
 			// elements [base, base + count) of the input-sized tensors; base is a multiple of hw
 			const int64_t plane_base = base / p.hw;
 			// position of an element inside the launch: plane (relative), row, column; advanced element by element
@@ -419,7 +425,7 @@ namespace nnf
 				const uint32_t w4 = p.w / 4;
 				const int64_t blocks = div_up(out_rows * w4, kAvgThreads * 2);
 				const int grid = (int)(blocks < int64_t(sm_count()) * 64 ? blocks : int64_t(sm_count()) * 64);
-				avgpool_fwd_2x2_kernel<<<grid, kAvgThreads, 0, s>>>(p.pooled, p.x, out_rows, w4, fastdiv(w4), p.mult);
+				launch(avgpool_fwd_2x2_kernel, grid, kAvgThreads, 0, s, p.pooled, p.x, out_rows, w4, fastdiv(w4), p.mult);
 				return check_launch("avgpool_fwd_2x2_kernel");
 			}
 			if (!fused && p.win_w == 2 && p.win_h == 2 && p.w % 2 == 0 && p.h % 2 == 0 && (reinterpret_cast<uintptr_t>(p.x) & 7) == 0
@@ -429,7 +435,7 @@ namespace nnf
 				const uint32_t w2 = p.w / 2;
 				const int64_t blocks = div_up(out_rows * w2, kAvgThreads * 4);
 				const int grid = (int)(blocks < int64_t(sm_count()) * 64 ? blocks : int64_t(sm_count()) * 64);
-				avgpool_fwd_2x2_pair_kernel<<<grid, kAvgThreads, 0, s>>>(p.pooled, p.x, out_rows, w2, fastdiv(w2), p.mult);
+				launch(avgpool_fwd_2x2_pair_kernel, grid, kAvgThreads, 0, s, p.pooled, p.x, out_rows, w2, fastdiv(w2), p.mult);
 				return check_launch("avgpool_fwd_2x2_pair_kernel");
 			}
 			const size_t plane_bytes = size_t(p.hw) * sizeof(float);
@@ -448,7 +454,7 @@ namespace nnf
 				if (fused)
 					return set_error(NNF_ERR_UNSUPPORTED, "fused average pooling needs planes of at most %zu bytes", staging_smem_limit());
 				const int64_t blocks = div_up(p.planes * p.ohw, kAvgThreads);
-				avgpool_fwd_direct_kernel<<<(int)(blocks < int64_t(sm_count()) * 8 ? blocks : int64_t(sm_count()) * 8), kAvgThreads, 0, s>>>(p);
+				launch(avgpool_fwd_direct_kernel, (int)(blocks < int64_t(sm_count()) * 8 ? blocks : int64_t(sm_count()) * 8), kAvgThreads, 0, s, p);
 				return check_launch("avgpool_fwd_direct_kernel");
 			}
 			p.group = (uint32_t)group;
@@ -463,13 +469,13 @@ namespace nnf
 			{
 				e = cudaFuncSetAttribute(avgpool_fwd_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit());
 				if (e == cudaSuccess)
-					avgpool_fwd_kernel<true><<<grid, kAvgThreads, smem, s>>>(p);
+					launch(avgpool_fwd_kernel<true>, grid, kAvgThreads, smem, s, p);
 			}
 			else
 			{
 				e = cudaFuncSetAttribute(avgpool_fwd_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit());
 				if (e == cudaSuccess)
-					avgpool_fwd_kernel<false><<<grid, kAvgThreads, smem, s>>>(p);
+					launch(avgpool_fwd_kernel<false>, grid, kAvgThreads, smem, s, p);
 			}
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
@@ -488,7 +494,7 @@ namespace nnf
 				const uint32_t w2 = p.w / 2;
 				const int64_t blocks = div_up(out_rows * w2, kAvgThreads * 4);
 				const int grid = (int)(blocks < int64_t(sm_count()) * 64 ? blocks : int64_t(sm_count()) * 64);
-				avgpool_bwd_2x2_pair_kernel<<<grid, kAvgThreads, 0, s>>>(p.dx, p.dpooled, out_rows, w2, fastdiv(w2), p.mult, p.add);
+				launch(avgpool_bwd_2x2_pair_kernel, grid, kAvgThreads, 0, s, p.dx, p.dpooled, out_rows, w2, fastdiv(w2), p.mult, p.add);
 				return check_launch("avgpool_bwd_2x2_pair_kernel");
 			}
 			p.vec_ok = ((!p.dx || aligned16(p.dx)) && (!fused || (aligned16(p.zin) && (!p.dres || aligned16(p.dres))))) ? 1 : 0;
@@ -509,9 +515,9 @@ namespace nnf
 				const int64_t blocks = div_up(int64_t(count) / 4 + 1, kAvgThreads);
 				const int grid = (int)(blocks < int64_t(sm_count()) * 64 ? blocks : int64_t(sm_count()) * 64);
 				if (fused)
-					avgpool_bwd_kernel<true><<<grid, kAvgThreads, 0, s>>>(q, base, count);
+					launch(avgpool_bwd_kernel<true>, grid, kAvgThreads, 0, s, q, base, count);
 				else
-					avgpool_bwd_kernel<false><<<grid, kAvgThreads, 0, s>>>(q, base, count);
+					launch(avgpool_bwd_kernel<false>, grid, kAvgThreads, 0, s, q, base, count);
 				const int st = check_launch("avgpool_bwd_kernel");
 				if (st != NNF_OK)
 					return st;

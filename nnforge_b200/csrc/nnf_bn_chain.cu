@@ -324,6 +324,7 @@ namespace nnf
 		template <int A0, int A1, bool BWD, bool PEER>
 		__global__ void __launch_bounds__(kChainThreads, BWD ? kCtasBwd : kCtasFwd) bn_train_chain_kernel(const stream_params p)
 		{
+			pdl_begin();
 			constexpr int K = BWD ? 3 : 2;
 			constexpr int T = BWD ? 2 : 1;
 			constexpr int L = BWD ? kStreamSlotsBwd : kStreamSlots;
@@ -815,6 +816,7 @@ namespace nnf
 		template <int A0, int A1, bool BWD, bool PEER>
 		__global__ void __launch_bounds__(kChainThreads, 4) bn_train_chain_grouped_kernel(const chain_params p)
 		{
+			pdl_begin();
 			constexpr int K = BWD ? 3 : 2;
 			constexpr int U = BWD ? 2 : 4;              // entries in flight per thread and tensor
 			constexpr int NC = BWD ? 6 : 2;             // per-channel constants an A item derives
@@ -1485,7 +1487,7 @@ namespace nnf
 			cudaError_t e = cudaMemsetAsync(workspace, 0, sizeof(launch_report) + size_t(p.c) * sizeof(uint32_t), s);
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "%s: cudaMemsetAsync: %s", what, cudaGetErrorString(e));
-			kernel<<<p.total_items, kChainThreads, 0, s>>>(p);
+			launch(kernel, p.total_items, kChainThreads, 0, s, p);
 			return check_launch(what);
 		}
 
@@ -1513,7 +1515,7 @@ namespace nnf
 			e = cudaMemsetAsync(workspace, 0, sizeof(launch_report) + size_t(p.c) * sizeof(uint32_t), s);
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "%s: cudaMemsetAsync: %s", what, cudaGetErrorString(e));
-			kernel<<<p.total, kChainThreads, smem, s>>>(p);
+			launch(kernel, p.total, kChainThreads, smem, s, p);
 			return check_launch(what);
 		}
 	}

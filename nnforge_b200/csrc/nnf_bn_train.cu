@@ -75,6 +75,7 @@ namespace nnf
 		// workspace layout: double partial[c][split][kSums]
 		__global__ void __launch_bounds__(kThreads) bn_stats_kernel(double * partial, const float * x, chan_geom g)
 		{
+			pdl_begin();
 			__shared__ double s_red[(kThreads / 32) * 2];
 			const uint32_t ch = blockIdx.x / g.split;
 			const uint32_t sp = blockIdx.x - ch * g.split;
@@ -148,8 +149,9 @@ namespace nnf
 		// sums[k*c + ch] (+)= float(sum over splits of partial[ch][split][k]), k < count
 		// copy (may be null) receives the first copy_count sums too: the buffer a caller all-reduces
 		__global__ void bn_reduce_partials_kernel(float * sums, const double * partial, uint32_t c, uint32_t split, int count, int accumulate,
-			float * copy = nullptr, int copy_count = 0)
+			float * copy, int copy_count)
 		{
+			pdl_begin();
 			const uint32_t ch = blockIdx.x * blockDim.x + threadIdx.x;
 			if (ch >= c)
 				return;
@@ -170,6 +172,7 @@ namespace nnf
 		__global__ void __launch_bounds__(1024) bn_reduce_publish_kernel(float * sums, const double * partial, uint32_t c, uint32_t split, int count,
 			float * copy, int copy_count, peer_dst dst, int publish_count)
 		{
+			pdl_begin();
 			for (uint32_t ch = threadIdx.x; ch < c; ch += blockDim.x)
 				for (int k = 0; k < count; ++k)
 				{
@@ -189,6 +192,7 @@ namespace nnf
 		// PReLU slope gradient partials: sum dy * (x >= 0 ? 0 : x) per (channel, slice of entries)
 		__global__ void __launch_bounds__(kThreads) prelu_dslope_kernel(double * partial, const float * dy, const float * x, chan_geom g)
 		{
+			pdl_begin();
 			__shared__ double s_red[kThreads / 32];
 			const uint32_t ch = blockIdx.x / g.split;
 			const uint32_t sp = blockIdx.x - ch * g.split;
@@ -251,6 +255,7 @@ namespace nnf
 		template <int A0, int A1>
 		__global__ void __launch_bounds__(kThreads) bn_bwd_stats_kernel(double * partial, const bwd_params p, chan_geom g)
 		{
+			pdl_begin();
 			__shared__ double s_red[(kThreads / 32) * 3];
 			// channels in descending order: whatever ran before (the forward kernels walk the channels upwards)
 			// left the highest channels of x in L2; bn_bwd_apply_kernel then walks upwards again
@@ -334,6 +339,7 @@ namespace nnf
 		template <int A0, int A1>
 		__global__ void __launch_bounds__(kThreads) bn_bwd_apply_kernel(const bwd_params p, chan_geom g)
 		{
+			pdl_begin();
 			// channels in ascending order: bn_bwd_stats_kernel, which ran just before, walked them downwards with
 			// default-policy loads, so the channels it read last (the lowest, ~100 MB still in L2) come first
 			const uint32_t ch = blockIdx.x / g.split;
@@ -455,6 +461,7 @@ namespace nnf
 		template <int A0, int A1>
 		__global__ void __launch_bounds__(kThreads) bn_apply_channel_kernel(const apply_params p, chan_geom g)
 		{
+			pdl_begin();
 			const uint32_t ch = g.c - 1 - blockIdx.x / g.split;
 			const uint32_t sp = blockIdx.x % g.split;
 			const uint32_t e0 = sp * g.entries_per_cta;
@@ -689,6 +696,7 @@ namespace nnf
 		template <int R>
 		__global__ void __launch_bounds__(kThreads) bn_stats_grouped_kernel(double * partial, const float * x, const group_geom g)
 		{
+			pdl_begin();
 			__shared__ float s_pos[2][kGroupMaxRun];
 			constexpr int U = 4;   // entries in flight
 			const group_cta t = group_locate(g);
@@ -742,6 +750,7 @@ namespace nnf
 		template <int R>
 		__global__ void __launch_bounds__(kThreads) prelu_dslope_grouped_kernel(double * partial, const float * dy, const float * x, const group_geom g)
 		{
+			pdl_begin();
 			__shared__ float s_pos[1][kGroupMaxRun];
 			constexpr int U = 2;
 			const group_cta t = group_locate(g);
@@ -832,6 +841,7 @@ namespace nnf
 		template <int A0, int A1, int R>
 		__global__ void __launch_bounds__(kThreads) bn_bwd_stats_grouped_kernel(double * partial, const bwd_params p, const group_geom g)
 		{
+			pdl_begin();
 			__shared__ float s_pos[3][kGroupMaxRun];
 			constexpr int U = 2;
 			const group_cta t = group_locate(g, true);
@@ -906,6 +916,7 @@ namespace nnf
 		template <int A0, int A1, int R>
 		__global__ void __launch_bounds__(kThreads) bn_bwd_apply_grouped_kernel(const bwd_params p, const group_geom g)
 		{
+			pdl_begin();
 			constexpr int U = 2;
 			const group_cta t = group_locate(g);
 			if (t.sp == 0)
@@ -980,6 +991,7 @@ namespace nnf
 		template <int A0, int A1, int R>
 		__global__ void __launch_bounds__(kThreads) bn_apply_grouped_kernel(const apply_params p, const group_geom g)
 		{
+			pdl_begin();
 			__shared__ float s_mult[kGroupMaxChannels], s_add[kGroupMaxChannels];
 			constexpr int U = 4;
 			const group_cta t = group_locate(g, true);
@@ -1108,9 +1120,9 @@ int stats_impl(nnf_stream_t stream, float * sums, const float * x, int64_t n, in
 	if (make_group_geom(gg, n, c, hw, aligned16(x)))
 	{
 		if (gg.vectors_per_thread == 1)
-			bn_stats_grouped_kernel<1><<<gg.groups * gg.split, kThreads, 0, s>>>(static_cast<double *>(workspace), x, gg);
+			launch(bn_stats_grouped_kernel<1>, gg.groups * gg.split, kThreads, 0, s, static_cast<double *>(workspace), x, gg);
 		else
-			bn_stats_grouped_kernel<2><<<gg.groups * gg.split, kThreads, 0, s>>>(static_cast<double *>(workspace), x, gg);
+			launch(bn_stats_grouped_kernel<2>, gg.groups * gg.split, kThreads, 0, s, static_cast<double *>(workspace), x, gg);
 		st = check_launch("bn_stats_grouped_kernel");
 		g.c = gg.c;
 		g.split = gg.split;
@@ -1120,17 +1132,17 @@ int stats_impl(nnf_stream_t stream, float * sums, const float * x, int64_t n, in
 		st = make_chan_geom(g, "nnf_bn_train_stats", n, c, hw, aligned16(x), resident_ctas_per_sm(bn_stats_kernel), 1);
 		if (st != NNF_OK)
 			return st;
-		bn_stats_kernel<<<g.c * g.split, kThreads, 0, s>>>(static_cast<double *>(workspace), x, g);
+		launch(bn_stats_kernel, g.c * g.split, kThreads, 0, s, static_cast<double *>(workspace), x, g);
 		st = check_launch("bn_stats_kernel");
 	}
 	if (st != NNF_OK)
 		return st;
 	if (publish)
 	{
-		bn_reduce_publish_kernel<<<1, 1024, 0, s>>>(sums, static_cast<const double *>(workspace), g.c, g.split, 2, nullptr, 0, *publish, 2);
+		launch(bn_reduce_publish_kernel, 1, 1024, 0, s, sums, static_cast<const double *>(workspace), g.c, g.split, 2, nullptr, 0, *publish, 2);
 		return check_launch("bn_reduce_publish_kernel");
 	}
-	bn_reduce_partials_kernel<<<(unsigned)div_up(c, 128), 128, 0, s>>>(sums, static_cast<const double *>(workspace), g.c, g.split, 2, 0);
+	launch(bn_reduce_partials_kernel, (unsigned)div_up(c, 128), 128, 0, s, sums, static_cast<const double *>(workspace), g.c, g.split, 2, 0, nullptr, 0);
 	return check_launch("bn_reduce_partials_kernel");
 }
 }
@@ -1195,8 +1207,8 @@ int apply_impl(nnf_stream_t stream, float * y, float * saved, const float * x, c
 		const unsigned grid = gg.groups * gg.split;
 		cudaStream_t s = (cudaStream_t)stream;
 		#define NNF_GROUPED_APPLY(A0, A1) \
-			do { if (gg.vectors_per_thread == 1) bn_apply_grouped_kernel<A0, A1, 1><<<grid, kThreads, 0, s>>>(p, gg); \
-			     else bn_apply_grouped_kernel<A0, A1, 2><<<grid, kThreads, 0, s>>>(p, gg); } while (0)
+			do { if (gg.vectors_per_thread == 1) launch(bn_apply_grouped_kernel<A0, A1, 1>, grid, kThreads, 0, s, p, gg); \
+			     else launch(bn_apply_grouped_kernel<A0, A1, 2>, grid, kThreads, 0, s, p, gg); } while (0)
 		switch (chain_id(chain))
 		{
 		case 0: NNF_GROUPED_APPLY(NNF_ACT_NONE, 0); break;
@@ -1223,10 +1235,10 @@ int apply_impl(nnf_stream_t stream, float * y, float * saved, const float * x, c
 		cudaStream_t s = (cudaStream_t)stream;
 		switch (chain_id(chain))
 		{
-		case 0: bn_apply_channel_kernel<NNF_ACT_NONE, 0><<<g.c * g.split, kThreads, 0, s>>>(p, g); break;
-		case 1: bn_apply_channel_kernel<NNF_ACT_PRELU, NNF_ACT_ELU><<<g.c * g.split, kThreads, 0, s>>>(p, g); break;
-		case 2: bn_apply_channel_kernel<NNF_ACT_RELU, 0><<<g.c * g.split, kThreads, 0, s>>>(p, g); break;
-		default: bn_apply_channel_kernel<-1, 0><<<g.c * g.split, kThreads, 0, s>>>(p, g); break;
+		case 0: launch(bn_apply_channel_kernel<NNF_ACT_NONE, 0>, g.c * g.split, kThreads, 0, s, p, g); break;
+		case 1: launch(bn_apply_channel_kernel<NNF_ACT_PRELU, NNF_ACT_ELU>, g.c * g.split, kThreads, 0, s, p, g); break;
+		case 2: launch(bn_apply_channel_kernel<NNF_ACT_RELU, 0>, g.c * g.split, kThreads, 0, s, p, g); break;
+		default: launch(bn_apply_channel_kernel<-1, 0>, g.c * g.split, kThreads, 0, s, p, g); break;
 		}
 		return check_launch("bn_apply_channel_kernel");
 	}
@@ -1311,8 +1323,8 @@ int bwd_stats_impl(nnf_stream_t stream, float * bsums, float * gsums, const floa
 		double * ws = static_cast<double *>(workspace);
 		const unsigned grid = gg.groups * gg.split;
 		#define NNF_GROUPED_BWD_STATS(A0, A1) \
-			do { if (gg.vectors_per_thread == 1) bn_bwd_stats_grouped_kernel<A0, A1, 1><<<grid, kThreads, 0, s>>>(ws, p, gg); \
-			     else bn_bwd_stats_grouped_kernel<A0, A1, 2><<<grid, kThreads, 0, s>>>(ws, p, gg); } while (0)
+			do { if (gg.vectors_per_thread == 1) launch(bn_bwd_stats_grouped_kernel<A0, A1, 1>, grid, kThreads, 0, s, ws, p, gg); \
+			     else launch(bn_bwd_stats_grouped_kernel<A0, A1, 2>, grid, kThreads, 0, s, ws, p, gg); } while (0)
 		switch (chain_id(p.chain))
 		{
 		case 0: NNF_GROUPED_BWD_STATS(NNF_ACT_NONE, 0); break;
@@ -1332,10 +1344,10 @@ int bwd_stats_impl(nnf_stream_t stream, float * bsums, float * gsums, const floa
 			return st;
 		switch (chain_id(p.chain))
 		{
-		case 0: bn_bwd_stats_kernel<NNF_ACT_NONE, 0><<<g.c * g.split, kThreads, 0, s>>>(static_cast<double *>(workspace), p, g); break;
-		case 1: bn_bwd_stats_kernel<NNF_ACT_PRELU, NNF_ACT_ELU><<<g.c * g.split, kThreads, 0, s>>>(static_cast<double *>(workspace), p, g); break;
-		case 2: bn_bwd_stats_kernel<NNF_ACT_RELU, 0><<<g.c * g.split, kThreads, 0, s>>>(static_cast<double *>(workspace), p, g); break;
-		default: bn_bwd_stats_kernel<-1, 0><<<g.c * g.split, kThreads, 0, s>>>(static_cast<double *>(workspace), p, g); break;
+		case 0: launch(bn_bwd_stats_kernel<NNF_ACT_NONE, 0>, g.c * g.split, kThreads, 0, s, static_cast<double *>(workspace), p, g); break;
+		case 1: launch(bn_bwd_stats_kernel<NNF_ACT_PRELU, NNF_ACT_ELU>, g.c * g.split, kThreads, 0, s, static_cast<double *>(workspace), p, g); break;
+		case 2: launch(bn_bwd_stats_kernel<NNF_ACT_RELU, 0>, g.c * g.split, kThreads, 0, s, static_cast<double *>(workspace), p, g); break;
+		default: launch(bn_bwd_stats_kernel<-1, 0>, g.c * g.split, kThreads, 0, s, static_cast<double *>(workspace), p, g); break;
 		}
 		st = check_launch("bn_bwd_stats_kernel");
 	}
@@ -1343,10 +1355,10 @@ int bwd_stats_impl(nnf_stream_t stream, float * bsums, float * gsums, const floa
 		return st;
 	if (publish)
 	{
-		bn_reduce_publish_kernel<<<1, 1024, 0, s>>>(bsums, static_cast<const double *>(workspace), g.c, g.split, 3, gsums, 2, *publish, 2);
+		launch(bn_reduce_publish_kernel, 1, 1024, 0, s, bsums, static_cast<const double *>(workspace), g.c, g.split, 3, gsums, 2, *publish, 2);
 		return check_launch("bn_reduce_publish_kernel");
 	}
-	bn_reduce_partials_kernel<<<(unsigned)div_up(c, 128), 128, 0, s>>>(bsums, static_cast<const double *>(workspace), g.c, g.split, 3, 0, gsums, 2);
+	launch(bn_reduce_partials_kernel, (unsigned)div_up(c, 128), 128, 0, s, bsums, static_cast<const double *>(workspace), g.c, g.split, 3, 0, gsums, 2);
 	return check_launch("bn_reduce_partials_kernel");
 }
 }
@@ -1427,8 +1439,8 @@ int bwd_apply_impl(nnf_stream_t stream, float * dx, const float * dy, const floa
 		const unsigned grid = gg.groups * gg.split;
 		cudaStream_t s = (cudaStream_t)stream;
 		#define NNF_GROUPED_BWD_APPLY(A0, A1) \
-			do { if (gg.vectors_per_thread == 1) bn_bwd_apply_grouped_kernel<A0, A1, 1><<<grid, kThreads, 0, s>>>(p, gg); \
-			     else bn_bwd_apply_grouped_kernel<A0, A1, 2><<<grid, kThreads, 0, s>>>(p, gg); } while (0)
+			do { if (gg.vectors_per_thread == 1) launch(bn_bwd_apply_grouped_kernel<A0, A1, 1>, grid, kThreads, 0, s, p, gg); \
+			     else launch(bn_bwd_apply_grouped_kernel<A0, A1, 2>, grid, kThreads, 0, s, p, gg); } while (0)
 		switch (chain_id(p.chain))
 		{
 		case 0: NNF_GROUPED_BWD_APPLY(NNF_ACT_NONE, 0); break;
@@ -1445,10 +1457,10 @@ int bwd_apply_impl(nnf_stream_t stream, float * dx, const float * dy, const floa
 		return st;
 	switch (chain_id(p.chain))
 	{
-	case 0: bn_bwd_apply_kernel<NNF_ACT_NONE, 0><<<g.c * g.split, kThreads, 0, (cudaStream_t)stream>>>(p, g); break;
-	case 1: bn_bwd_apply_kernel<NNF_ACT_PRELU, NNF_ACT_ELU><<<g.c * g.split, kThreads, 0, (cudaStream_t)stream>>>(p, g); break;
-	case 2: bn_bwd_apply_kernel<NNF_ACT_RELU, 0><<<g.c * g.split, kThreads, 0, (cudaStream_t)stream>>>(p, g); break;
-	default: bn_bwd_apply_kernel<-1, 0><<<g.c * g.split, kThreads, 0, (cudaStream_t)stream>>>(p, g); break;
+	case 0: launch(bn_bwd_apply_kernel<NNF_ACT_NONE, 0>, g.c * g.split, kThreads, 0, (cudaStream_t)stream, p, g); break;
+	case 1: launch(bn_bwd_apply_kernel<NNF_ACT_PRELU, NNF_ACT_ELU>, g.c * g.split, kThreads, 0, (cudaStream_t)stream, p, g); break;
+	case 2: launch(bn_bwd_apply_kernel<NNF_ACT_RELU, 0>, g.c * g.split, kThreads, 0, (cudaStream_t)stream, p, g); break;
+	default: launch(bn_bwd_apply_kernel<-1, 0>, g.c * g.split, kThreads, 0, (cudaStream_t)stream, p, g); break;
 	}
 	return check_launch("bn_bwd_apply_kernel");
 }
@@ -1477,9 +1489,9 @@ extern "C" int nnf_prelu_bwd_weights(nnf_stream_t stream, float * dslope, const 
 	if (make_group_geom(gg, n, c, hw, aligned16(x) && aligned16(dy)))
 	{
 		if (gg.vectors_per_thread == 1)
-			prelu_dslope_grouped_kernel<1><<<gg.groups * gg.split, kThreads, 0, s>>>(static_cast<double *>(workspace), dy, x, gg);
+			launch(prelu_dslope_grouped_kernel<1>, gg.groups * gg.split, kThreads, 0, s, static_cast<double *>(workspace), dy, x, gg);
 		else
-			prelu_dslope_grouped_kernel<2><<<gg.groups * gg.split, kThreads, 0, s>>>(static_cast<double *>(workspace), dy, x, gg);
+			launch(prelu_dslope_grouped_kernel<2>, gg.groups * gg.split, kThreads, 0, s, static_cast<double *>(workspace), dy, x, gg);
 		st = check_launch("prelu_dslope_grouped_kernel");
 		g.c = gg.c;
 		g.split = gg.split;
@@ -1489,12 +1501,12 @@ extern "C" int nnf_prelu_bwd_weights(nnf_stream_t stream, float * dslope, const 
 		st = make_chan_geom(g, "nnf_prelu_bwd_weights", n, c, hw, aligned16(x) && aligned16(dy), resident_ctas_per_sm(prelu_dslope_kernel), 1);
 		if (st != NNF_OK)
 			return st;
-		prelu_dslope_kernel<<<g.c * g.split, kThreads, 0, s>>>(static_cast<double *>(workspace), dy, x, g);
+		launch(prelu_dslope_kernel, g.c * g.split, kThreads, 0, s, static_cast<double *>(workspace), dy, x, g);
 		st = check_launch("prelu_dslope_kernel");
 	}
 	if (st != NNF_OK)
 		return st;
-	bn_reduce_partials_kernel<<<(unsigned)div_up(c, 128), 128, 0, s>>>(dslope, static_cast<const double *>(workspace), g.c, g.split, 1, 1);
+	launch(bn_reduce_partials_kernel, (unsigned)div_up(c, 128), 128, 0, s, dslope, static_cast<const double *>(workspace), g.c, g.split, 1, 1, nullptr, 0);
 	return check_launch("bn_reduce_partials_kernel");
 }
 
@@ -1566,10 +1578,10 @@ extern "C" int nnf_bn_train_stats_static(nnf_stream_t stream, float * sums, cons
 	if (st != NNF_OK)
 		return st;
 	cudaStream_t s = (cudaStream_t)stream;
-	bn_stats_kernel<<<g.c * g.split, kThreads, 0, s>>>(scratch, x, g);
+	launch(bn_stats_kernel, g.c * g.split, kThreads, 0, s, scratch, x, g);
 	st = check_launch("bn_stats_kernel");
 	if (st != NNF_OK)
 		return st;
-	bn_reduce_partials_kernel<<<(unsigned)div_up(c, 128), 128, 0, s>>>(sums, scratch, g.c, g.split, 2, 0);
+	launch(bn_reduce_partials_kernel, (unsigned)div_up(c, 128), 128, 0, s, sums, scratch, g.c, g.split, 2, 0, nullptr, 0);
 	return check_launch("bn_reduce_partials_kernel");
 }

@@ -131,6 +131,7 @@ namespace nnf
 		template <int MODE, int A0, int A1>
 		__global__ void __launch_bounds__(kThreads) bn_act_kernel(const ew_params p)
 		{
+			pdl_begin();
 			extern __shared__ float s_params[];
 			float * s_mult = s_params;
 			float * s_add = s_params + p.c;
@@ -323,6 +324,7 @@ namespace nnf
 		template <int A0, int A1>
 		__global__ void __launch_bounds__(kThreads) bn_act_grouped_kernel(const ew_params p, const ewg_geom g)
 		{
+			pdl_begin();
 			extern __shared__ float s_params[];
 			float * s_mult = s_params;
 			float * s_add = s_params + g.group;
@@ -450,7 +452,7 @@ namespace nnf
 			const int k1 = p.chain.n > 1 ? p.chain.a[1].kind : NNF_ACT_NONE;
 			const unsigned grid = g.groups * g.split;
 			const size_t smem = size_t(2) * g.group * sizeof(float);
-#define NNF_EWG_CASE(A0, A1) bn_act_grouped_kernel<A0, A1><<<grid, g.threads, smem, s>>>(p, g)
+#define NNF_EWG_CASE(A0, A1) launch(bn_act_grouped_kernel<A0, A1>, grid, g.threads, smem, s, p, g)
 			if (p.chain.n == 0)
 				NNF_EWG_CASE(NNF_ACT_NONE, 0);
 			else if (k0 == NNF_ACT_RELU && k1 == NNF_ACT_NONE)
@@ -499,7 +501,7 @@ namespace nnf
 		{
 			const int k0 = p.chain.n > 0 ? p.chain.a[0].kind : NNF_ACT_NONE;
 			const int k1 = p.chain.n > 1 ? p.chain.a[1].kind : NNF_ACT_NONE;
-#define NNF_EW_CASE(A0, A1) bn_act_kernel<MODE, A0, A1><<<resident_grid<MODE, A0, A1>(smem, work), kThreads, smem, s>>>(p)
+#define NNF_EW_CASE(A0, A1) launch(bn_act_kernel<MODE, A0, A1>, resident_grid<MODE, A0, A1>(smem, work), kThreads, smem, s, p)
 			if (k1 == NNF_ACT_NONE)
 			{
 				switch (k0)
@@ -619,6 +621,7 @@ namespace nnf
 		template <int KIND, int MODE>
 		__global__ void __launch_bounds__(kThreads) act_bwd_kernel(const bw_params p)
 		{
+			pdl_begin();
 			auto channel_of = [&](uint32_t e) -> uint32_t {
 				const uint32_t plane = p.hw.div(e);
 				return plane - p.cdiv.div(plane) * p.c;
@@ -710,11 +713,11 @@ namespace nnf
 		cudaError_t launch_bwd(const bw_params& p, int mode, int grid, cudaStream_t s)
 		{
 			if (mode == 0)
-				act_bwd_kernel<KIND, 0><<<grid, kThreads, 0, s>>>(p);
+				launch(act_bwd_kernel<KIND, 0>, grid, kThreads, 0, s, p);
 			else if (mode == 1)
-				act_bwd_kernel<KIND, 1><<<grid, kThreads, 0, s>>>(p);
+				launch(act_bwd_kernel<KIND, 1>, grid, kThreads, 0, s, p);
 			else
-				act_bwd_kernel<KIND, 2><<<grid, kThreads, 0, s>>>(p);
+				launch(act_bwd_kernel<KIND, 2>, grid, kThreads, 0, s, p);
 			return cudaGetLastError();
 		}
 
@@ -731,6 +734,7 @@ namespace nnf
 		template <int MODE>
 		__global__ void __launch_bounds__(kThreads) add_kernel(const add_params p)
 		{
+			pdl_begin();
 			if (MODE == 2)
 			{
 				const uint32_t stride = gridDim.x * kThreads;
@@ -776,6 +780,7 @@ namespace nnf
 		template <int MODE>
 		__global__ void __launch_bounds__(kThreads) scale_kernel(float * dx, const float * dy, float alpha, uint32_t count, int add)
 		{
+			pdl_begin();
 			if (MODE == 2)
 			{
 				const uint32_t stride = gridDim.x * kThreads;
@@ -1011,9 +1016,9 @@ extern "C" int nnf_add_fwd(nnf_stream_t stream, float * y, const float * const *
 		p.alpha = alpha;
 		p.count = (uint32_t)cnt;
 		if (vec_ok)
-			add_kernel<0><<<grid_for(cnt, 1), kThreads, 0, (cudaStream_t)stream>>>(p);
+			launch(add_kernel<0>, grid_for(cnt, 1), kThreads, 0, (cudaStream_t)stream, p);
 		else
-			add_kernel<2><<<grid_for(cnt * 4, 1), kThreads, 0, (cudaStream_t)stream>>>(p);
+			launch(add_kernel<2>, grid_for(cnt * 4, 1), kThreads, 0, (cudaStream_t)stream, p);
 		cudaError_t e = cudaGetLastError();
 		if (e != cudaSuccess)
 			return set_error(NNF_ERR_CUDA, "add_kernel launch failed: %s", cudaGetErrorString(e));
@@ -1036,9 +1041,9 @@ extern "C" int nnf_add_bwd(nnf_stream_t stream, float * dx, const float * dy, fl
 	{
 		const int64_t cnt = (count - off < step) ? (count - off) : step;
 		if (aligned16(dx + off) && aligned16(dy + off))
-			scale_kernel<0><<<grid_for(cnt, 1), kThreads, 0, (cudaStream_t)stream>>>(dx + off, dy + off, alpha, (uint32_t)cnt, add_to_destination ? 1 : 0);
+			launch(scale_kernel<0>, grid_for(cnt, 1), kThreads, 0, (cudaStream_t)stream, dx + off, dy + off, alpha, (uint32_t)cnt, add_to_destination ? 1 : 0);
 		else
-			scale_kernel<2><<<grid_for(cnt * 4, 1), kThreads, 0, (cudaStream_t)stream>>>(dx + off, dy + off, alpha, (uint32_t)cnt, add_to_destination ? 1 : 0);
+			launch(scale_kernel<2>, grid_for(cnt * 4, 1), kThreads, 0, (cudaStream_t)stream, dx + off, dy + off, alpha, (uint32_t)cnt, add_to_destination ? 1 : 0);
 		cudaError_t e = cudaGetLastError();
 		if (e != cudaSuccess)
 			return set_error(NNF_ERR_CUDA, "scale_kernel launch failed: %s", cudaGetErrorString(e));

@@ -128,6 +128,7 @@ namespace nnf
 		template <int VPL, int MODE>
 		__global__ void __launch_bounds__(256) loss_rows_kernel(const loss_params p)
 		{
+			pdl_begin();
 			const int lane = threadIdx.x & 31;
 			const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
 			const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
@@ -294,6 +295,7 @@ namespace nnf
 		template <int CMAX, int MODE, bool EXACT = false>
 		__global__ void __launch_bounds__(256) loss_pixels_kernel(const loss_params p)
 		{
+			pdl_begin();
 			const int64_t stride = int64_t(gridDim.x) * blockDim.x;
 			const int c = EXACT ? CMAX : p.c;
 			const uint32_t hw = p.hw;
@@ -446,11 +448,11 @@ namespace nnf
 				const int64_t blocks_needed = div_up(n, 8); // 8 warps per CTA
 				const int grid = (int)(blocks_needed < int64_t(sm_count()) * 64 ? blocks_needed : int64_t(sm_count()) * 64);
 				const bool vec = (c & 3) == 0 && c <= 1024 && aligned16(in) && aligned16(targets) && (!out || aligned16(out));
-				if (vec && c <= 128) loss_rows_kernel<1, MODE><<<grid, 256, 0, s>>>(p);
-				else if (vec && c <= 256) loss_rows_kernel<2, MODE><<<grid, 256, 0, s>>>(p);
-				else if (vec && c <= 512) loss_rows_kernel<4, MODE><<<grid, 256, 0, s>>>(p);
-				else if (vec) loss_rows_kernel<8, MODE><<<grid, 256, 0, s>>>(p);
-				else loss_rows_kernel<0, MODE><<<grid, 256, 0, s>>>(p);
+				if (vec && c <= 128) launch(loss_rows_kernel<1, MODE>, grid, 256, 0, s, p);
+				else if (vec && c <= 256) launch(loss_rows_kernel<2, MODE>, grid, 256, 0, s, p);
+				else if (vec && c <= 512) launch(loss_rows_kernel<4, MODE>, grid, 256, 0, s, p);
+				else if (vec) launch(loss_rows_kernel<8, MODE>, grid, 256, 0, s, p);
+				else launch(loss_rows_kernel<0, MODE>, grid, 256, 0, s, p);
 				return check_launch("loss_rows_kernel");
 			}
 			const int64_t entries_per_launch = kMaxElemsPerLaunch / hw;
@@ -475,7 +477,7 @@ namespace nnf
 					// one instantiation per column length, as in the per-pixel softmax kernel: no dead slots in the unrolled loops
 					// and no more registers than the column needs (softmax + loss fused at logits[512,21,128,128]: forward 446 us
 					// with 24 slots for 21 elements, 329 us with 21; backward 401 -> 320 us)
-#define NNF_EXACT(C) case C: loss_pixels_kernel<C, MODE, true><<<grid, 256, 0, s>>>(p); launched = true; break;
+#define NNF_EXACT(C) case C: launch(loss_pixels_kernel<C, MODE, true>, grid, 256, 0, s, p); launched = true; break;
 					switch ((int)c)
 					{
 					NNF_EXACT(2) NNF_EXACT(3) NNF_EXACT(4) NNF_EXACT(5) NNF_EXACT(6) NNF_EXACT(7) NNF_EXACT(8)
@@ -487,11 +489,11 @@ namespace nnf
 #undef NNF_EXACT
 				}
 				if (launched) {}
-				else if (c <= 8) loss_pixels_kernel<8, MODE><<<grid, 256, 0, s>>>(p);
-				else if (c <= 16) loss_pixels_kernel<16, MODE><<<grid, 256, 0, s>>>(p);
-				else if (c <= 24) loss_pixels_kernel<24, MODE><<<grid, 256, 0, s>>>(p);
-				else if (c <= 32) loss_pixels_kernel<32, MODE><<<grid, 256, 0, s>>>(p);
-				else loss_pixels_kernel<0, MODE><<<grid, 256, 0, s>>>(p);
+				else if (c <= 8) launch(loss_pixels_kernel<8, MODE>, grid, 256, 0, s, p);
+				else if (c <= 16) launch(loss_pixels_kernel<16, MODE>, grid, 256, 0, s, p);
+				else if (c <= 24) launch(loss_pixels_kernel<24, MODE>, grid, 256, 0, s, p);
+				else if (c <= 32) launch(loss_pixels_kernel<32, MODE>, grid, 256, 0, s, p);
+				else launch(loss_pixels_kernel<0, MODE>, grid, 256, 0, s, p);
 				const int st = check_launch("loss_pixels_kernel");
 				if (st != NNF_OK)
 					return st;
@@ -530,6 +532,7 @@ namespace nnf
 		// H*W == 1: warp per row
 		__global__ void __launch_bounds__(256) accuracy_rows_kernel(const accuracy_params p)
 		{
+			pdl_begin();
 			const int lane = threadIdx.x & 31;
 			const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
 			const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
@@ -587,6 +590,7 @@ namespace nnf
 		// H*W > 1: thread per pixel, channels strided by H*W
 		__global__ void __launch_bounds__(256) accuracy_pixels_kernel(const accuracy_params p)
 		{
+			pdl_begin();
 			const int64_t stride = int64_t(gridDim.x) * blockDim.x;
 			for (int64_t q = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; q < p.rows; q += stride)
 			{
@@ -648,7 +652,7 @@ extern "C" int nnf_accuracy_fwd(nnf_stream_t stream, float * out, const float * 
 		p.hw = 1;
 		const int64_t blocks_needed = div_up(n, 8);
 		const int grid = (int)(blocks_needed < int64_t(sm_count()) * 64 ? blocks_needed : int64_t(sm_count()) * 64);
-		accuracy_rows_kernel<<<grid, 256, 0, s>>>(p);
+		launch(accuracy_rows_kernel, grid, 256, 0, s, p);
 		return check_launch("accuracy_rows_kernel");
 	}
 	const int64_t entries_per_launch = kMaxElemsPerLaunch / hw;
@@ -666,7 +670,7 @@ extern "C" int nnf_accuracy_fwd(nnf_stream_t stream, float * out, const float * 
 		p.hwdiv = fastdiv((uint32_t)hw);
 		const int64_t blocks_needed = div_up(p.rows, 256);
 		const int grid = (int)(blocks_needed < int64_t(sm_count()) * 128 ? blocks_needed : int64_t(sm_count()) * 128);
-		accuracy_pixels_kernel<<<grid, 256, 0, s>>>(p);
+		launch(accuracy_pixels_kernel, grid, 256, 0, s, p);
 		const int st = check_launch("accuracy_pixels_kernel");
 		if (st != NNF_OK)
 			return st;

@@ -57,6 +57,7 @@ namespace nnf
 		template <int TYPE>
 		__global__ void __launch_bounds__(kOptThreads) apply_gradient_kernel(const __grid_constant__ opt_params p)
 		{
+			pdl_begin();
 			__shared__ double s_red[kOptThreads / 32];
 			int k = 0;
 			while (k + 1 < p.n_parts && blockIdx.x >= p.part[k + 1].first_cta)
@@ -157,6 +158,7 @@ namespace nnf
 
 		__global__ void __launch_bounds__(kCalThreads) bn_calibrate_stats_kernel(const cal_params p)
 		{
+			pdl_begin();
 			__shared__ double s_red[kCalThreads / 32][kCalPartials];
 			const uint32_t ch = blockIdx.x / p.split;
 			const uint32_t sp = blockIdx.x - ch * p.split;
@@ -253,6 +255,7 @@ namespace nnf
 		// set was cut into batches beyond double rounding.
 		__global__ void bn_calibrate_merge_kernel(const cal_params p)
 		{
+			pdl_begin();
 			const uint32_t ch = blockIdx.x * blockDim.x + threadIdx.x;
 			if (ch >= p.c)
 				return;
@@ -294,6 +297,7 @@ namespace nnf
 		// statistics (nnforge/toolset.cpp:1613-1620)
 		__global__ void bn_calibrate_finish_kernel(float * mean, float * invsigma, float * stats, const double * acc, uint32_t c)
 		{
+			pdl_begin();
 			const uint32_t ch = blockIdx.x * blockDim.x + threadIdx.x;
 			if (ch >= c)
 				return;
@@ -359,10 +363,10 @@ extern "C" int nnf_apply_gradient(nnf_stream_t stream, const nnf_opt_part * part
 			return NNF_OK;
 		switch (momentum_type)
 		{
-		case NNF_MOMENTUM_NONE: apply_gradient_kernel<NNF_MOMENTUM_NONE><<<ctas, kOptThreads, 0, cs>>>(p); break;
-		case NNF_MOMENTUM_VANILLA: apply_gradient_kernel<NNF_MOMENTUM_VANILLA><<<ctas, kOptThreads, 0, cs>>>(p); break;
-		case NNF_MOMENTUM_NESTEROV: apply_gradient_kernel<NNF_MOMENTUM_NESTEROV><<<ctas, kOptThreads, 0, cs>>>(p); break;
-		default: apply_gradient_kernel<NNF_MOMENTUM_ADAM><<<ctas, kOptThreads, 0, cs>>>(p); break;
+		case NNF_MOMENTUM_NONE: launch(apply_gradient_kernel<NNF_MOMENTUM_NONE>, ctas, kOptThreads, 0, cs, p); break;
+		case NNF_MOMENTUM_VANILLA: launch(apply_gradient_kernel<NNF_MOMENTUM_VANILLA>, ctas, kOptThreads, 0, cs, p); break;
+		case NNF_MOMENTUM_NESTEROV: launch(apply_gradient_kernel<NNF_MOMENTUM_NESTEROV>, ctas, kOptThreads, 0, cs, p); break;
+		default: launch(apply_gradient_kernel<NNF_MOMENTUM_ADAM>, ctas, kOptThreads, 0, cs, p); break;
 		}
 		p.n_parts = 0;
 		return check_launch("apply_gradient_kernel");
@@ -448,11 +452,11 @@ extern "C" int nnf_bn_calibrate_accumulate(nnf_stream_t stream, void * accumulat
 	p.entries_per_cta = uint32_t(per);
 	p.d_per_plane = fastdiv(p.vec ? p.hw >> 2 : p.hw);
 	cudaStream_t cs = (cudaStream_t)stream;
-	bn_calibrate_stats_kernel<<<uint32_t(c * split), kCalThreads, 0, cs>>>(p);
+	launch(bn_calibrate_stats_kernel, uint32_t(c * split), kCalThreads, 0, cs, p);
 	int rc = check_launch("bn_calibrate_stats_kernel");
 	if (rc != NNF_OK)
 		return rc;
-	bn_calibrate_merge_kernel<<<uint32_t((c + 127) / 128), 128, 0, cs>>>(p);
+	launch(bn_calibrate_merge_kernel, uint32_t((c + 127) / 128), 128, 0, cs, p);
 	return check_launch("bn_calibrate_merge_kernel");
 }
 
@@ -460,7 +464,7 @@ extern "C" int nnf_bn_calibrate_finish(nnf_stream_t stream, float * mean, float 
 {
 	if (!accumulator || c <= 0 || (!mean != !invsigma) || (!mean && !stats))
 		return set_error(NNF_ERR_INVALID_ARGUMENT, "nnf_bn_calibrate_finish: null pointer or empty shape");
-	bn_calibrate_finish_kernel<<<uint32_t((c + 127) / 128), 128, 0, (cudaStream_t)stream>>>(mean, invsigma, stats,
+	launch(bn_calibrate_finish_kernel, uint32_t((c + 127) / 128), 128, 0, (cudaStream_t)stream, mean, invsigma, stats,
 		static_cast<const double *>(accumulator), uint32_t(c));
 	return check_launch("bn_calibrate_finish_kernel");
 }

@@ -43,6 +43,7 @@ namespace nnf
 		template <int PER_LANE, bool BACKWARD>
 		__global__ void __launch_bounds__(256) softmax_rows_warp_kernel(float * out, const float * in0, const float * in1, int64_t rows, int c, int add)
 		{
+			pdl_begin();
 			const int lane = threadIdx.x & 31;
 			const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
 			const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
@@ -117,6 +118,7 @@ namespace nnf
 		template <int VPL, bool BACKWARD>
 		__global__ void __launch_bounds__(256) softmax_rows_warp4_kernel(float * out, const float * in0, const float * in1, int64_t rows, int c, int add)
 		{
+			pdl_begin();
 			const int lane = threadIdx.x & 31;
 			const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
 			const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
@@ -217,6 +219,7 @@ namespace nnf
 		template <bool BACKWARD, bool IN_SMEM, int THREADS, bool VEC>
 		__global__ void __launch_bounds__(THREADS) softmax_rows_block_kernel(float * out, const float * in0, const float * in1, int64_t rows, int c, int add)
 		{
+			pdl_begin();
 			extern __shared__ float s_row[];
 			__shared__ float s_red[THREADS / 32];
 			for (int64_t row = blockIdx.x; row < rows; row += gridDim.x)
@@ -353,6 +356,7 @@ namespace nnf
 		template <int CMAX, bool BACKWARD>
 		__global__ void __launch_bounds__(256, BACKWARD ? 2 : 4) softmax_pixels_reg_kernel(float * out, const float * in0, const float * in1, int64_t pixels, uint32_t hw, fastdiv hwdiv, int add)
 		{
+			pdl_begin();
 			constexpr int c = CMAX;
 			const int64_t stride = int64_t(gridDim.x) * blockDim.x;
 			for (int64_t p = int64_t(blockIdx.x) * blockDim.x + threadIdx.x; p < pixels; p += stride)
@@ -424,6 +428,7 @@ namespace nnf
 		template <int CPW, int WARPS, bool BACKWARD>
 		__global__ void __launch_bounds__(WARPS * 32, 2) softmax_pixels_wide_kernel(float * out, const float * in0, const float * in1, int64_t quads, uint32_t hw4, fastdiv hw4div, int c, int add)
 		{
+			pdl_begin();
 			__shared__ float4 s_red[WARPS][32];
 			const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 			const int64_t ntiles = (quads + 31) / 32;
@@ -547,6 +552,7 @@ namespace nnf
 		template <bool BACKWARD, bool IN_SMEM>
 		__global__ void __launch_bounds__(256) softmax_pixels_tile_kernel(float * out, const float * in0, const float * in1, int64_t pixels, uint32_t hw, fastdiv hwdiv, int c, int add)
 		{
+			pdl_begin();
 			extern __shared__ float s_tile[]; // [c][32] when IN_SMEM (second [c][32] for backward)
 			__shared__ float s_red[8][32];
 			const int lane = threadIdx.x & 31, grp = threadIdx.x >> 5;
@@ -682,7 +688,7 @@ namespace nnf
 						const int threads4 = rows <= int64_t(sm_count()) * 2 ? 32 : (rows <= int64_t(sm_count()) * 8 ? 64 : 256);
 						const int64_t blocks4 = div_up(rows, threads4 / 32);
 						const int grid4 = (int)(blocks4 < int64_t(sm_count()) * 64 ? blocks4 : int64_t(sm_count()) * 64);
-#define NNF_ROWS4(VPL) softmax_rows_warp4_kernel<VPL, BACKWARD><<<grid4, threads4, 0, s>>>(out, in0, in1, rows, (int)c, add)
+#define NNF_ROWS4(VPL) launch(softmax_rows_warp4_kernel<VPL, BACKWARD>, grid4, threads4, 0, s, out, in0, in1, rows, (int)c, add)
 						if (c <= 128) NNF_ROWS4(1);
 						else if (c <= 256) NNF_ROWS4(2);
 						else if (c <= 512) NNF_ROWS4(4);
@@ -690,7 +696,7 @@ namespace nnf
 #undef NNF_ROWS4
 						return check_launch("softmax_rows_warp4_kernel");
 					}
-#define NNF_ROWS(PL) case PL: softmax_rows_warp_kernel<PL, BACKWARD><<<grid, 256, 0, s>>>(out, in0, in1, rows, (int)c, add); break;
+#define NNF_ROWS(PL) case PL: launch(softmax_rows_warp_kernel<PL, BACKWARD>, grid, 256, 0, s, out, in0, in1, rows, (int)c, add); break;
 					switch ((int)div_up(c, 32))
 					{
 					NNF_ROWS(1) NNF_ROWS(2) NNF_ROWS(3) NNF_ROWS(4) NNF_ROWS(5) NNF_ROWS(6) NNF_ROWS(7) NNF_ROWS(8)
@@ -720,7 +726,7 @@ namespace nnf
 						if (e != cudaSuccess) \
 							return set_error(NNF_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e)); \
 					} \
-					softmax_rows_block_kernel<BACKWARD, IN, TH, VE><<<grid, TH, IN ? smem : 0, s>>>(out, in0, in1, rows, (int)c, add); \
+					launch(softmax_rows_block_kernel<BACKWARD, IN, TH, VE>, grid, TH, IN ? smem : 0, s, out, in0, in1, rows, (int)c, add); \
 				} while (0)
 				if (in_smem)
 				{
@@ -756,7 +762,7 @@ namespace nnf
 					const int grid = (int)(blocks_needed < int64_t(sm_count()) * 128 ? blocks_needed : int64_t(sm_count()) * 128);
 					// one instantiation per column length: no dead slots in the unrolled loops and no more registers than the
 					// column needs (x[32,21,128,128] forward: 20.7 us with 32 slots for 21 elements, 16.4 us with 21)
-#define NNF_EXACT(C) case C: softmax_pixels_reg_kernel<C, BACKWARD><<<grid, 256, 0, s>>>(o, a, b, pixels, (uint32_t)hw, fastdiv((uint32_t)hw), add); break;
+#define NNF_EXACT(C) case C: launch(softmax_pixels_reg_kernel<C, BACKWARD>, grid, 256, 0, s, o, a, b, pixels, (uint32_t)hw, fastdiv((uint32_t)hw), add); break;
 					switch ((int)c)
 					{
 					NNF_EXACT(1) NNF_EXACT(2) NNF_EXACT(3) NNF_EXACT(4) NNF_EXACT(5) NNF_EXACT(6) NNF_EXACT(7) NNF_EXACT(8)
@@ -779,7 +785,7 @@ namespace nnf
 					const int64_t ntiles = div_up(quads, 32);
 					const int64_t cap = int64_t(sm_count()) * 4;
 					const int grid = (int)(ntiles < cap ? ntiles : cap);
-#define NNF_WIDE(CPW) case CPW: softmax_pixels_wide_kernel<CPW, kWarps, BACKWARD><<<grid, kWarps * 32, 0, s>>>(o, a, b, quads, (uint32_t)(hw / 4), fastdiv((uint32_t)(hw / 4)), (int)c, add); break;
+#define NNF_WIDE(CPW) case CPW: launch(softmax_pixels_wide_kernel<CPW, kWarps, BACKWARD>, grid, kWarps * 32, 0, s, o, a, b, quads, (uint32_t)(hw / 4), fastdiv((uint32_t)(hw / 4)), (int)c, add); break;
 					switch (cpw)   // more than 32 channels: at least three per warp
 					{
 					NNF_WIDE(3) NNF_WIDE(4) NNF_WIDE(5) NNF_WIDE(6) NNF_WIDE(7) NNF_WIDE(8) NNF_WIDE(9) NNF_WIDE(10)
@@ -803,10 +809,10 @@ namespace nnf
 						cudaError_t e = cudaFuncSetAttribute(softmax_pixels_tile_kernel<BACKWARD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit());
 						if (e != cudaSuccess)
 							return set_error(NNF_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
-						softmax_pixels_tile_kernel<BACKWARD, true><<<grid, 256, smem, s>>>(o, a, b, pixels, (uint32_t)hw, fastdiv((uint32_t)hw), (int)c, add);
+						launch(softmax_pixels_tile_kernel<BACKWARD, true>, grid, 256, smem, s, o, a, b, pixels, (uint32_t)hw, fastdiv((uint32_t)hw), (int)c, add);
 					}
 					else
-						softmax_pixels_tile_kernel<BACKWARD, false><<<grid, 256, 0, s>>>(o, a, b, pixels, (uint32_t)hw, fastdiv((uint32_t)hw), (int)c, add);
+						launch(softmax_pixels_tile_kernel<BACKWARD, false>, grid, 256, 0, s, o, a, b, pixels, (uint32_t)hw, fastdiv((uint32_t)hw), (int)c, add);
 					int st = check_launch("softmax_pixels_tile_kernel");
 					if (st != NNF_OK)
 						return st;
