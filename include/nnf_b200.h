@@ -93,7 +93,7 @@ typedef struct nnf_running_configuration
 NNF_API int nnf_get_running_configuration(nnf_running_configuration * out);
 
 /* Knobs of the launch plans (process-wide; nothing in the library reads the environment). No counterpart in
- * the reference. name: "elementwise_waves", "elementwise_group_waves", "pool_waves", "pool_group_floats",
+ * the reference. name: "elementwise_waves", "elementwise_group_waves", "pool_waves", "pool_group_floats", "pool_staged",
  * "channel_waves", "group_waves", "chain_s_kb", "chain_a_kb", "chain_dist" (-1: built-in), "chain_chunk_mb",
  * "chain_lag" (lag + 1), "no_grouped", "apply_flat", "peer_wait_ns" (how long a batch-sharded launch waits for
  * another rank's statistics before it gives up; default 10 s), or "reset" (all back to the built-in choices).

@@ -81,6 +81,7 @@ namespace nnf
 		int elementwise_group_waves;  // the same for the channel-group inference kernel
 		int pool_waves;               // max / average subsampling grids
 		int pool_group_floats;        // floats of one staged plane group
+		int pool_staged;              // 1: max subsampling stages plane groups whatever its window
 		int channel_waves;            // training kernels with one CTA per (channel, slice)
 		int group_waves;              // the same for the channel-group training kernels
 		int chain_s_kb, chain_a_kb;   // single-launch training kernel: KB of one tensor per statistics / apply item

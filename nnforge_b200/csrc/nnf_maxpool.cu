@@ -1,6 +1,9 @@
 // 2-D max subsampling forward/backward, stand-alone and fused behind batch norm -> residual add ->
 // ReLU (the tail of a ResNet block). HBM-bound.
 //
+// Windows of 3x3 or 2x2 at stride 2 go through the row kernels of nnf_maxpool_rows.cuh, the rest (and large fused tensors with odd rows)
+// through the plane-group kernels of this file.
+//
 // Data movement: a CTA owns a group of whole consecutive (n, c) planes, which are contiguous in the
 // planar layout. Forward: the group is read once with coalesced 128-bit loads, the fused
 // per-element result z is written straight back (it is needed by later layers and by backward) and
@@ -21,6 +24,8 @@
 
 #include <stdlib.h>
 
+#include <initializer_list>
+
 namespace nnf
 {
 	namespace
@@ -36,6 +41,15 @@ namespace nnf
 			fastdiv d_w, d_hw, d_ow, d_ohw, d_sw, d_sh, d_c;
 		};
 
+	}
+}
+
+#include "nnf_maxpool_rows.cuh"
+
+namespace nnf
+{
+	namespace
+	{
 		struct pool_fwd_params
 		{
 			pool_geom g;
@@ -96,6 +110,7 @@ namespace nnf
 		template <bool FUSED, int WW, int WH, bool CLIP>
 		__global__ void __launch_bounds__(kThreads) pool_fwd_staged_kernel(const pool_fwd_params p)
 		{
+			pdl_begin();
 			extern __shared__ float s_z[];
 			__shared__ float s_mult[FUSED ? kMaxGroup : 1];
 			__shared__ float s_add[FUSED ? kMaxGroup : 1];
@@ -249,6 +264,7 @@ namespace nnf
 		// Fallback for planes that do not fit shared memory: one thread per output element, from global.
 		__global__ void __launch_bounds__(kThreads) pool_fwd_direct_kernel(float * pooled, uint32_t * argmax, const float * x, pool_geom g, int64_t planes)
 		{
+			pdl_begin();
 			const int64_t total = planes * g.ohw;
 			const int64_t stride = int64_t(gridDim.x) * kThreads;
 			for (int64_t o = int64_t(blockIdx.x) * kThreads + threadIdx.x; o < total; o += stride)
@@ -281,8 +297,7 @@ namespace nnf
 			int group;
 			int vec_ok;
 			int add;               // stand-alone only
-			int row4_vec;          // 3x3/2 fast path: rows are whole float4s (W % 4 == 0, aligned buffers)
-			fastdiv d_cpr, d_hcpr; // 3x3/2 fast path with ragged rows: chunks per row, chunks per plane
+			fastdiv d_cpr, d_hcpr; // 3x3/2 in row chunks: chunks per row, chunks per plane
 		};
 
 		// Gradient reaching input element (iy, ix) of a plane whose pooled gradients / argmax start at
@@ -377,45 +392,10 @@ namespace nnf
 			}
 		}
 
-		// 2x2 windows, stride 2, four consecutive elements of one input row: windows do not overlap, the four elements
-		// belong to the two windows {k, k + 1} of output row iy / 2, k = ix0 / 2 - two (argmax, gradient) pairs per vector
-		__device__ __forceinline__ void gather_row4_2x2s2(const pool_geom& g, const float * dyp, const uint32_t * idp, uint32_t iy, uint32_t ix0,
-			uint32_t abs0, float (&acc)[4])
-		{
-			const uint32_t oy = iy >> 1;
-			if (oy > g.oh - 1)
-				return;
-			const uint32_t k = ix0 >> 1;
-			const uint32_t row = oy * g.ow + k;
-			if (k <= g.ow - 1)
-			{
-				const uint32_t i = idp[row];
-				const float d = dyp[row];
-				if (i == abs0) acc[0] = __fadd_rn(acc[0], d);
-				if (i == abs0 + 1) acc[1] = __fadd_rn(acc[1], d);
-			}
-			if (k + 1 <= g.ow - 1)
-			{
-				const uint32_t i = idp[row + 1];
-				const float d = dyp[row + 1];
-				if (i == abs0 + 2) acc[2] = __fadd_rn(acc[2], d);
-				if (i == abs0 + 3) acc[3] = __fadd_rn(acc[3], d);
-			}
-		}
-
-		template <int WW>
-		__device__ __forceinline__ void gather_row4(const pool_geom& g, const float * dyp, const uint32_t * idp, uint32_t iy, uint32_t ix0,
-			uint32_t abs0, float (&acc)[4])
-		{
-			if (WW == 2)
-				gather_row4_2x2s2(g, dyp, idp, iy, ix0, abs0, acc);
-			else
-				gather_row4_3x3s2(g, dyp, idp, iy, ix0, abs0, acc);
-		}
-
 		template <bool FUSED, int WW, int WH, int SW, int SH, bool ROW4 = false>
 		__global__ void __launch_bounds__(kThreads) pool_bwd_staged_kernel(const pool_bwd_params p)
 		{
+			pdl_begin();
 			extern __shared__ float s_raw[];
 			const pool_geom& g = p.g;
 			const int64_t ngroups = (p.planes + p.group - 1) / p.group;
@@ -435,7 +415,7 @@ namespace nnf
 					s_idx[o] = __ldcs(p.argmax + obase + o);
 				}
 				const uint32_t ch0 = (uint32_t)(plane0 - int64_t(g.d_c.div((uint32_t)plane0)) * g.c);
-				if (FUSED && ROW4 && !p.row4_vec)
+				if (ROW4)
 					for (uint32_t lp = threadIdx.x; lp < np; lp += kThreads)
 					{
 						uint32_t channel = ch0 + lp;
@@ -473,7 +453,7 @@ namespace nnf
 						out_dx = dz;
 				};
 
-				if (ROW4 && !p.row4_vec)
+				if (ROW4)
 				{
 					// rows that are not a multiple of four elements (14x14, 7x7): the same four-element row
 					// chunks, with scalar accesses and the last chunk of a row cut short
@@ -488,65 +468,48 @@ namespace nnf
 						const uint32_t e0 = lp * g.hw + iy * g.w + ix0;
 						const uint32_t nvalid = min(4u, g.w - ix0);
 						float acc[4] = {0.0F, 0.0F, 0.0F, 0.0F};
-						if (!FUSED && p.add)
-						{
-							#pragma unroll
-							for (int k = 0; k < 4; ++k)
-								if ((uint32_t)k < nvalid)
-									acc[k] = p.dx[base + e0 + k];
-						}
-						gather_row4<WW>(g, s_dy + lp * g.ohw, s_idx + lp * g.ohw, iy, ix0, (uint32_t)(base + e0), acc);
+						gather_row4_3x3s2(g, s_dy + lp * g.ohw, s_idx + lp * g.ohw, iy, ix0, (uint32_t)(base + e0), acc);
 						#pragma unroll
 						for (int k = 0; k < 4; ++k)
 							if ((uint32_t)k < nvalid)
-							{
-								// (staging the stand-alone result too and storing it with 128-bit stores was measured slower:
-								// 14x14 81 -> 100 us)
-								if (FUSED)
-									s_dz[e0 + k] = acc[k]; // gathered gradient of the group, consumed with coalesced accesses below
-								else
-									p.dx[base + e0 + k] = acc[k];
-							}
+								s_dz[e0 + k] = acc[k]; // gathered gradient of the group, consumed with coalesced accesses below
 					}
-					if (FUSED)
+					__syncthreads();
+					// the batch-norm factor of a plane comes from shared memory; a vector of four elements lies in
+					// one plane unless it straddles a plane boundary (H*W not a multiple of 4)
+					auto finish = [&](float mult, float zval, float dz, float& odx, float& ores)
 					{
-						__syncthreads();
-						// the batch-norm factor of a plane comes from shared memory; a vector of four elements lies in
-						// one plane unless it straddles a plane boundary (H*W not a multiple of 4)
-						auto finish = [&](float mult, float zval, float dz, float& odx, float& ores)
-						{
-							const float ds = (__float_as_uint(zval) >> 31) ? __fmul_rn(dz, p.slope) : dz;
-							ores = ds;
-							odx = p.gamma ? __fmul_rn(ds, mult) : ds;
-						};
-						const uint32_t nvec = p.vec_ok ? (count >> 2) : 0;
-						for (uint32_t v = threadIdx.x; v < nvec; v += kThreads)
-						{
-							const float4 z4 = ld_stream(reinterpret_cast<const float4 *>(p.z + base) + v);
-							const float4 d4 = reinterpret_cast<const float4 *>(s_dz)[v];
-							const uint32_t lp0 = g.d_hw.div(v << 2);
-							const uint32_t left = (lp0 + 1) * g.hw - (v << 2); // elements of this vector in plane lp0 (>= 1)
-							const float m0 = s_mult[lp0];
-							const float m1 = left >= 4 ? m0 : s_mult[lp0 + 1];
-							float4 ox, orr;
-							finish(m0, z4.x, d4.x, ox.x, orr.x);
-							finish(left > 1 ? m0 : m1, z4.y, d4.y, ox.y, orr.y);
-							finish(left > 2 ? m0 : m1, z4.z, d4.z, ox.z, orr.z);
-							finish(left > 3 ? m0 : m1, z4.w, d4.w, ox.w, orr.w);
-							if (p.dx)
-								st_stream(reinterpret_cast<float4 *>(p.dx + base) + v, ox);
-							if (p.dres)
-								st_stream(reinterpret_cast<float4 *>(p.dres + base) + v, orr);
-						}
-						for (uint32_t e = (nvec << 2) + threadIdx.x; e < count; e += kThreads)
-						{
-							float odx, ores;
-							finish(s_mult[g.d_hw.div(e)], p.z[base + e], s_dz[e], odx, ores);
-							if (p.dx)
-								p.dx[base + e] = odx;
-							if (p.dres)
-								p.dres[base + e] = ores;
-						}
+						const float ds = (__float_as_uint(zval) >> 31) ? __fmul_rn(dz, p.slope) : dz;
+						ores = ds;
+						odx = p.gamma ? __fmul_rn(ds, mult) : ds;
+					};
+					const uint32_t nvec = p.vec_ok ? (count >> 2) : 0;
+					for (uint32_t v = threadIdx.x; v < nvec; v += kThreads)
+					{
+						const float4 z4 = ld_stream(reinterpret_cast<const float4 *>(p.z + base) + v);
+						const float4 d4 = reinterpret_cast<const float4 *>(s_dz)[v];
+						const uint32_t lp0 = g.d_hw.div(v << 2);
+						const uint32_t left = (lp0 + 1) * g.hw - (v << 2); // elements of this vector in plane lp0 (>= 1)
+						const float m0 = s_mult[lp0];
+						const float m1 = left >= 4 ? m0 : s_mult[lp0 + 1];
+						float4 ox, orr;
+						finish(m0, z4.x, d4.x, ox.x, orr.x);
+						finish(left > 1 ? m0 : m1, z4.y, d4.y, ox.y, orr.y);
+						finish(left > 2 ? m0 : m1, z4.z, d4.z, ox.z, orr.z);
+						finish(left > 3 ? m0 : m1, z4.w, d4.w, ox.w, orr.w);
+						if (p.dx)
+							st_stream(reinterpret_cast<float4 *>(p.dx + base) + v, ox);
+						if (p.dres)
+							st_stream(reinterpret_cast<float4 *>(p.dres + base) + v, orr);
+					}
+					for (uint32_t e = (nvec << 2) + threadIdx.x; e < count; e += kThreads)
+					{
+						float odx, ores;
+						finish(s_mult[g.d_hw.div(e)], p.z[base + e], s_dz[e], odx, ores);
+						if (p.dx)
+							p.dx[base + e] = odx;
+						if (p.dres)
+							p.dres[base + e] = ores;
 					}
 				}
 				else if (p.vec_ok)
@@ -567,39 +530,9 @@ namespace nnf
 							seed[0] = d4.x; seed[1] = d4.y; seed[2] = d4.z; seed[3] = d4.w;
 						}
 						float odx[4], ores[4];
-						if (ROW4)
-						{
-							const uint32_t e0 = v << 2;
-							const uint32_t lp = g.d_hw.div(e0);
-							const uint32_t rem = e0 - lp * g.hw;
-							const uint32_t iy = g.d_w.div(rem);
-							gather_row4<WW>(g, s_dy + lp * g.ohw, s_idx + lp * g.ohw, iy, rem - iy * g.w, (uint32_t)(base + e0), seed);
-							float mult = 1.0F;
-							if (FUSED && p.gamma)
-							{
-								uint32_t channel = ch0 + lp;
-								channel -= g.d_c.div(channel) * g.c;
-								mult = __fmul_rn(__ldg(p.gamma + channel), __ldg(p.invsigma + channel));
-							}
-							#pragma unroll
-							for (int k = 0; k < 4; ++k)
-							{
-								if (FUSED)
-								{
-									const float ds = (__float_as_uint(zv[k]) >> 31) ? __fmul_rn(seed[k], p.slope) : seed[k];
-									ores[k] = ds;
-									odx[k] = p.gamma ? __fmul_rn(ds, mult) : ds;
-								}
-								else
-									odx[k] = seed[k];
-							}
-						}
-						else
-						{
-							#pragma unroll
-							for (int k = 0; k < 4; ++k)
-								element((v << 2) + k, zv[k], seed[k], odx[k], ores[k]);
-						}
+						#pragma unroll
+						for (int k = 0; k < 4; ++k)
+							element((v << 2) + k, zv[k], seed[k], odx[k], ores[k]);
 						if (p.dx)
 							st_stream(reinterpret_cast<float4 *>(p.dx + base) + v, make_float4(odx[0], odx[1], odx[2], odx[3]));
 						if (FUSED && p.dres)
@@ -635,6 +568,7 @@ namespace nnf
 		template <bool FUSED>
 		__global__ void __launch_bounds__(kThreads) pool_bwd_direct_kernel(const pool_bwd_params p)
 		{
+			pdl_begin();
 			const pool_geom& g = p.g;
 			const int64_t total = p.planes * g.hw;
 			const int64_t stride = int64_t(gridDim.x) * kThreads;
@@ -716,6 +650,15 @@ namespace nnf
 			return (int)grp;
 		}
 
+		// the largest power of two, up to 16, that divides the addresses (null pointers aside)
+		size_t common_alignment(std::initializer_list<const void *> pointers)
+		{
+			uintptr_t bits = 16;
+			for (const void * p : pointers)
+				bits |= reinterpret_cast<uintptr_t>(p);
+			return size_t(bits & (~bits + 1));
+		}
+
 		int run_pool_fwd(cudaStream_t s, bool fused, pool_fwd_params& p, int64_t n)
 		{
 			// only round-up makes the last window stick out of the input
@@ -727,6 +670,26 @@ namespace nnf
 				return set_error(NNF_ERR_UNSUPPORTED, "max subsampling: more than 2^31 planes");
 			if (p.argmax && p.planes * p.g.hw > int64_t(0xffffffffll))
 				return set_error(NNF_ERR_UNSUPPORTED, "max subsampling: argmax offsets need n*c*h*w < 2^32");
+			rows_params q = {};
+			int access = 0;
+			// (a strip reads one row and a warp a column that another one writes: not with z over x or over the residual)
+			const bool in_place = fused && (p.z == p.x || p.z == p.res);
+			if (!in_place && plan_rows(q, access, p.g, p.planes, common_alignment({p.x, p.z, p.res}), fused, false))
+			{
+				q.x = p.x; q.res = p.res; q.z = p.z; q.pooled = p.pooled; q.argmax = p.argmax;
+				q.gamma = p.gamma; q.beta = p.beta; q.mean = p.mean; q.invsigma = p.invsigma; q.slope = p.slope;
+				const bool is_min = p.g.is_min != 0;
+				switch (access * 2 + (fused ? 1 : 0))
+				{
+				case 9: rows_fwd<4, true>(q, p.g.win_w, is_min, s); break;
+				case 8: rows_fwd<4, false>(q, p.g.win_w, is_min, s); break;
+				case 5: rows_fwd<2, true>(q, p.g.win_w, is_min, s); break;
+				case 4: rows_fwd<2, false>(q, p.g.win_w, is_min, s); break;
+				case 3: rows_fwd<1, true>(q, p.g.win_w, is_min, s); break;
+				default: rows_fwd<1, false>(q, p.g.win_w, is_min, s); break;
+				}
+				return check_launch("pool_rows_fwd_kernel");
+			}
 			bool vec_ok = aligned16(p.x) && (!fused || (aligned16(p.z) && (!p.res || aligned16(p.res))));
 			const int grp = choose_group(p.g, p.planes, vec_ok);
 			if (grp == 0)
@@ -735,7 +698,7 @@ namespace nnf
 					return set_error(NNF_ERR_UNSUPPORTED, "fused max subsampling: a %ux%u plane does not fit shared memory", p.g.w, p.g.h);
 				const int64_t blocks = div_up(p.planes * p.g.ohw, kThreads);
 				const int grid = (int)(blocks < int64_t(sm_count()) * 8 ? blocks : int64_t(sm_count()) * 8);
-				pool_fwd_direct_kernel<<<grid, kThreads, 0, s>>>(p.pooled, p.argmax, p.x, p.g, p.planes);
+				launch(pool_fwd_direct_kernel, grid, kThreads, 0, s, p.pooled, p.argmax, p.x, p.g, p.planes);
 				return check_launch("pool_fwd_direct_kernel");
 			}
 			p.group = grp;
@@ -753,7 +716,7 @@ namespace nnf
 			{ \
 				e = cudaFuncSetAttribute(pool_fwd_staged_kernel<FUSED, WW, WH, CLIP>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit()); \
 				if (e == cudaSuccess) \
-					pool_fwd_staged_kernel<FUSED, WW, WH, CLIP><<<grid, kThreads, smem, s>>>(p); \
+					launch(pool_fwd_staged_kernel<FUSED, WW, WH, CLIP>, grid, kThreads, smem, s, p); \
 			}
 #define NNF_POOL_FWD_SHAPE(FUSED) \
 			if (!clip && ww == 3 && wh == 3) NNF_POOL_FWD(FUSED, 3, 3, false) \
@@ -785,18 +748,35 @@ namespace nnf
 				return set_error(NNF_ERR_UNSUPPORTED, "max subsampling: more than 2^31 planes");
 			if (p.planes * p.g.hw > int64_t(0xffffffffll))
 				return set_error(NNF_ERR_UNSUPPORTED, "max subsampling: argmax offsets need n*c*h*w < 2^32");
+			rows_params q = {};
+			int access = 0;
+			if (plan_rows(q, access, p.g, p.planes, common_alignment({p.z, p.dx, p.dres}), fused, true))
+			{
+				q.pooled = const_cast<float *>(p.dpooled); q.argmax = const_cast<uint32_t *>(p.argmax); q.z = const_cast<float *>(p.z);
+				q.dx = p.dx; q.dres = p.dres; q.gamma = p.gamma; q.invsigma = p.invsigma; q.slope = p.slope; q.add = p.add;
+				switch (access * 2 + (fused ? 1 : 0))
+				{
+				case 9: rows_bwd<4, true>(q, p.g.win_w, s); break;
+				case 8: rows_bwd<4, false>(q, p.g.win_w, s); break;
+				case 5: rows_bwd<2, true>(q, p.g.win_w, s); break;
+				case 4: rows_bwd<2, false>(q, p.g.win_w, s); break;
+				case 3: rows_bwd<1, true>(q, p.g.win_w, s); break;
+				default: rows_bwd<1, false>(q, p.g.win_w, s); break;
+				}
+				return check_launch("pool_rows_bwd_kernel");
+			}
 			bool vec_ok = (!p.dx || aligned16(p.dx)) && (!fused || (aligned16(p.z) && (!p.dres || aligned16(p.dres))));
 			const int grp = choose_group(p.g, p.planes, vec_ok);
-			const bool ragged_fast = fused && p.g.win_w == 3 && p.g.win_h == 3 && p.g.sw == 2 && p.g.sh == 2 && !((p.g.w & 3) == 0 && vec_ok);
+			const bool ragged_fast = fused && p.g.win_w == 3 && p.g.win_h == 3 && p.g.sw == 2 && p.g.sh == 2;
 			const size_t smem = (((size_t(grp) * p.g.ohw * 2 + 3) & ~size_t(3)) + (ragged_fast ? ((size_t(grp) * p.g.hw + 3) & ~size_t(3)) + size_t(grp) : 0)) * sizeof(float);
 			if (grp == 0 || smem > staging_smem_limit())
 			{
 				const int64_t blocks = div_up(p.planes * p.g.hw, kThreads);
 				const int grid = (int)(blocks < int64_t(sm_count()) * 8 ? blocks : int64_t(sm_count()) * 8);
 				if (fused)
-					pool_bwd_direct_kernel<true><<<grid, kThreads, 0, s>>>(p);
+					launch(pool_bwd_direct_kernel<true>, grid, kThreads, 0, s, p);
 				else
-					pool_bwd_direct_kernel<false><<<grid, kThreads, 0, s>>>(p);
+					launch(pool_bwd_direct_kernel<false>, grid, kThreads, 0, s, p);
 				return check_launch("pool_bwd_direct_kernel");
 			}
 			p.group = grp;
@@ -806,41 +786,25 @@ namespace nnf
 			per_sm = per_sm < 1 ? 1 : (per_sm > 8 ? 8 : per_sm);
 			const int64_t cap = int64_t(sm_count()) * per_sm * pool_waves();
 			const int grid = (int)(ngroups < cap ? ngroups : cap);
-			const int ww = p.g.win_w, wh = p.g.win_h, sw = p.g.sw, sh = p.g.sh;
-			cudaError_t e = cudaSuccess;
+						cudaError_t e = cudaSuccess;
 #define NNF_POOL_BWD(FUSED, WW, WH, SW, SH) \
 			{ \
 				e = cudaFuncSetAttribute(pool_bwd_staged_kernel<FUSED, WW, WH, SW, SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit()); \
 				if (e == cudaSuccess) \
-					pool_bwd_staged_kernel<FUSED, WW, WH, SW, SH><<<grid, kThreads, smem, s>>>(p); \
+					launch(pool_bwd_staged_kernel<FUSED, WW, WH, SW, SH>, grid, kThreads, smem, s, p); \
 			}
-			p.row4_vec = ((p.g.w & 3) == 0 && p.vec_ok) ? 1 : 0;
 			p.d_cpr = fastdiv((p.g.w + 3) / 4);
 			p.d_hcpr = fastdiv(p.g.h * ((p.g.w + 3) / 4));
-#define NNF_POOL_BWD_SHAPE(FUSED) \
-			if (ww == 3 && wh == 3 && sw == 2 && sh == 2) \
-			{ \
-				e = cudaFuncSetAttribute(pool_bwd_staged_kernel<FUSED, 3, 3, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit()); \
-				if (e == cudaSuccess) \
-					pool_bwd_staged_kernel<FUSED, 3, 3, 2, 2, true><<<grid, kThreads, smem, s>>>(p); \
-			} \
-			else if (ww == 2 && wh == 2 && sw == 2 && sh == 2 && (p.row4_vec || !FUSED)) \
-			{ \
-				e = cudaFuncSetAttribute(pool_bwd_staged_kernel<FUSED, 2, 2, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit()); \
-				if (e == cudaSuccess) \
-					pool_bwd_staged_kernel<FUSED, 2, 2, 2, 2, true><<<grid, kThreads, smem, s>>>(p); \
-			} \
-			else if (ww == 2 && wh == 2 && sw == 2 && sh == 2) NNF_POOL_BWD(FUSED, 2, 2, 2, 2) \
-			else NNF_POOL_BWD(FUSED, 0, 0, 0, 0)
-			if (fused)
+			if (ragged_fast)
 			{
-				NNF_POOL_BWD_SHAPE(true)
+				e = cudaFuncSetAttribute(pool_bwd_staged_kernel<true, 3, 3, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit());
+				if (e == cudaSuccess)
+					launch(pool_bwd_staged_kernel<true, 3, 3, 2, 2, true>, grid, kThreads, smem, s, p);
 			}
+			else if (fused)
+				NNF_POOL_BWD(true, 0, 0, 0, 0)
 			else
-			{
-				NNF_POOL_BWD_SHAPE(false)
-			}
-#undef NNF_POOL_BWD_SHAPE
+				NNF_POOL_BWD(false, 0, 0, 0, 0)
 #undef NNF_POOL_BWD
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));

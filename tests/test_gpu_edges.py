@@ -1,0 +1,95 @@
+"""Sizes at the edges of the tiles and of the dispatch rules of single kernels, against the CPU checker: rows of every remainder
+modulo the access width, planes and tensors on either side of a rule's limit, buffers off their usual alignment."""
+import numpy as np
+import pytest
+
+import synth
+from util import assert_bits_equal
+
+pytestmark = pytest.mark.gpu
+
+torch = pytest.importorskip("torch")
+
+
+@pytest.fixture(scope="module")
+def capi():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import nnforge_b200.capi as capi
+    return capi
+
+
+@pytest.fixture
+def tuning(capi):
+    yield capi.set_tuning
+    capi.set_tuning("reset", 0)
+
+
+def dev(a, offset=0):
+    """A CUDA copy of the array, `offset` floats behind an aligned address."""
+    t = torch.empty(a.size + offset, dtype=torch.float32 if a.dtype == np.float32 else torch.int32, device="cuda")
+    t[offset:].copy_(torch.from_numpy(np.ascontiguousarray(a)).reshape(-1))
+    return t[offset:].view(a.shape)
+
+
+def host(t):
+    torch.cuda.synchronize()
+    return t.cpu().numpy()
+
+
+# widths of every remainder modulo 4 up to more columns than a warp serves; heights of one pair of rows up to several, odd and even
+ROW_SHAPES = [(2, 3, 3, 3), (1, 5, 4, 4), (3, 2, 5, 5), (2, 2, 6, 6), (2, 3, 7, 7), (1, 3, 8, 9), (2, 1, 9, 34), (1, 2, 3, 131), (1, 1, 10, 130), (1, 1, 11, 128),
+              (5, 7, 13, 13), (2, 3, 33, 35), (9, 16, 14, 14)]
+
+
+@pytest.mark.parametrize("shape", ROW_SHAPES)
+@pytest.mark.parametrize("win", [2, 3])
+@pytest.mark.parametrize("round_up", [False, True])
+@pytest.mark.parametrize("staged", [0, 1])
+def test_max_subsampling_rows_and_plane_groups(capi, oracle, tuning, shape, win, round_up, staged):
+    """3x3 and 2x2 windows at stride 2 through the row kernels and through the plane-group kernels that large tensors take, with
+    NaNs and infinities among the values, stand-alone and fused, in place, and with buffers that only allow narrower accesses."""
+    tuning("pool_staged", staged)
+    g = synth.rng(3, salt=sum(shape) * 7 + win)
+    n, c = shape[:2]
+    ru = (round_up, round_up)
+    x = synth.with_edges(g, np.maximum(synth.normal(g, shape), 0))
+    x.reshape(-1)[g.choice(x.size, max(1, x.size // 40), replace=False)] = np.nan
+    for offset in (0, 2, 1):
+        for is_min in (False, True):
+            p = capi.pool((win, win), (2, 2), ru, is_min)
+            want, want_idx = oracle.maxpool_fwd(x, (win, win), (2, 2), ru, is_min)
+            y, idx = torch.empty(want.shape, device="cuda"), torch.zeros(want.shape, dtype=torch.int32, device="cuda")
+            capi.maxpool_fwd(y, idx, dev(x, offset), p)
+            assert_bits_equal(host(idx).view(np.uint32), want_idx, "argmax")
+            assert_bits_equal(host(y), want, "values")
+        dy, dx0 = synth.normal(g, want.shape), synth.normal(g, shape)
+        dx = dev(dx0, offset)
+        capi.maxpool_bwd(dx, dev(dy), idx, p)
+        assert_bits_equal(host(dx), oracle.maxpool_bwd(dy, want_idx, shape), "gradient")
+        dx = dev(dx0, offset)
+        capi.maxpool_bwd(dx, dev(dy), idx, p, add_to_destination=True)
+        assert_bits_equal(host(dx), oracle.maxpool_bwd(dy, want_idx, shape, dx=dx0), "gradient accumulated")
+
+    x, r = synth.normal(g, shape), synth.normal(g, shape)
+    bn = synth.bn_params(g, c)
+    p = capi.pool((win, win), (2, 2), ru)
+    bnd = [dev(a) for a in bn]
+    s = oracle.add_fwd([oracle.bn_infer(x, *bn), r], 1.0)
+    z_want = oracle.relu_fwd(s, 0.0)
+    want, want_idx = oracle.maxpool_fwd(z_want, (win, win), (2, 2), ru)
+    dyp = synth.normal(g, want.shape)
+    ds = oracle.relu_bwd(oracle.maxpool_bwd(dyp, want_idx, shape), s, 0.0)
+    dx_want = (ds * (bn[0] * bn[3]).astype(np.float32)[None, :, None, None]).astype(np.float32)
+    for offset, over in ((0, None), (2, None), (1, None), (0, "x"), (1, "residual")):
+        xd, rd = dev(x, offset), dev(r, offset)
+        z = {"x": xd, "residual": rd}.get(over, torch.empty(x.size + offset, device="cuda")[offset:].view(shape))
+        y, idx = torch.empty(want.shape, device="cuda"), torch.zeros(want.shape, dtype=torch.int32, device="cuda")
+        capi.bn_add_relu_maxpool_fwd(z, y, idx, xd, rd, bnd, 0.0, p)
+        assert_bits_equal(host(z), z_want, "z")
+        assert_bits_equal(host(y), want, "pooled")
+        assert_bits_equal(host(idx).view(np.uint32), want_idx, "fused argmax")
+        dx, dr = dev(np.zeros(shape, np.float32), offset), dev(np.zeros(shape, np.float32), offset)
+        capi.bn_add_relu_maxpool_bwd(dx, dr, dev(dyp), idx, z, bnd[0], bnd[3], 0.0, p)
+        assert_bits_equal(host(dr), ds, "dresidual")
+        assert_bits_equal(host(dx), dx_want, "dx")
