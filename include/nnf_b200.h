@@ -484,7 +484,7 @@ NNF_API int nnf_bn_train_bwd_sharded(nnf_stream_t stream, float * dx, float * bs
  *   ADAM      m1 = beta1*prev + (1-beta1)*g; m2 = beta2*prev2 + (1-beta2)*g*g;  (momentum = beta1, momentum2 = beta2)
  *             upd = lr*(m1/(1-beta1^t)) / (sqrt(m2/(1-beta2^t)) + 1e-8), t = iteration_id >= 1;   prev_upd = m1, prev_upd2 = m2
  *   w += upd; gradient = 0; *update_accum += sum |upd| (double; skipped when update_accum is NULL).
- * `parts` is a HOST array; the chunk table travels in the kernel parameters (48 chunks per launch), so a batch-norm
+ * `parts` is a HOST array; the chunk table travels in the kernel parameters (up to 500 chunks per launch), so a batch-norm
  * layer's four chunks, or all per-channel chunks of a network, cost one launch. weight_decay is the value that applies
  * to the chunk (0 for chunks outside layer::get_weight_decay_part_id_set()). Results are bit-identical to the plain
  * backend's expressions compiled without FMA contraction; a chunk of up to 1024 weights sums |upd| in a fixed order. */

@@ -467,7 +467,7 @@ def bn_train_bwd_apply_peer(dx, dy, x, gamma, beta, saved, my_buf, world, kmax, 
 
 def apply_gradient(parts, momentum_type=MOMENTUM_NONE, momentum=0.9, momentum2=0.999, normalizer=1.0, iteration_id=1, stream=None):
     """parts: list of dicts {data, gradient, [prev_upd], [prev_upd2], [update_accum (float64 tensor of 1)], learning_rate,
-    [weight_decay]}; every chunk of the list is updated by one launch (48 chunks per launch)."""
+    [weight_decay]}; every chunk of the list is updated by one launch (500 chunks per launch)."""
     _native.apply_gradient(parts, momentum_type, momentum, momentum2, normalizer, iteration_id, stream)
 
 

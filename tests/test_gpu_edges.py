@@ -93,3 +93,32 @@ def test_max_subsampling_rows_and_plane_groups(capi, oracle, tuning, shape, win,
         capi.bn_add_relu_maxpool_bwd(dx, dr, dev(dyp), idx, z, bnd[0], bnd[3], 0.0, p)
         assert_bits_equal(host(dr), ds, "dresidual")
         assert_bits_equal(host(dx), dx_want, "dx")
+
+
+@pytest.mark.parametrize("kind", ["none", "vanilla", "nesterov", "adam"])
+@pytest.mark.parametrize("chunks", [1, 48, 49, 160, 161, 500, 501])
+def test_optimiser_step_chunk_counts_and_alignment(capi, oracle, kind, chunks):
+    """Chunk counts on either side of the parameter blocks' capacities; chunks of every remainder modulo a thread's four weights and a
+    CTA's 1024, each with its buffers aligned and one float off."""
+    g = synth.rng(1, salt=8100 + chunks)
+    mtype = {"none": capi.MOMENTUM_NONE, "vanilla": capi.MOMENTUM_VANILLA, "nesterov": capi.MOMENTUM_NESTEROV, "adam": capi.MOMENTUM_ADAM}[kind]
+    sizes = [1023, 1024, 1025, 1, 2, 3, 4, 5, 2047, 2050]
+    names = ["data", "gradient"] + (["prev_upd"] if kind != "none" else []) + (["prev_upd2"] if kind == "adam" else [])
+    hostp, devp = [], []
+    for k in range(chunks):
+        n = sizes[k % len(sizes)]
+        hp = {"data": synth.normal(g, (n,)), "gradient": synth.normal(g, (n,)), "prev_upd": synth.normal(g, (n,), 0.0, 0.01),
+              "prev_upd2": np.abs(synth.normal(g, (n,), 0.0, 0.1))}
+        dp = {name: dev(hp[name], (k // len(sizes)) % 2 if name != "gradient" else 0) for name in names}
+        dp.update(learning_rate=0.01, weight_decay=0.0005 if k % 2 else 0.0, update_accum=torch.zeros(1, dtype=torch.float64, device="cuda"))
+        hostp.append(hp)
+        devp.append(dp)
+    capi.apply_gradient(devp, mtype, 0.9, 0.999, 1.0 / 32, 2)
+    for k, (hp, dp) in enumerate(zip(hostp, devp)):
+        accum = oracle.apply_gradient(hp["data"], hp["gradient"], hp["prev_upd"], hp["prev_upd2"], kind, 0.01, 1.0 / 32, dp["weight_decay"], 0.9, 0.999, 2)
+        assert not host(dp["gradient"]).any()
+        for name in names:
+            if name != "gradient":
+                assert_bits_equal(host(dp[name]), hp[name], "%s, chunk %d" % (name, k))
+        # two orders of a double sum of at most 2050 terms of one sign: 2050 * 2^-53 < 3e-13 relative
+        assert abs(float(host(dp["update_accum"])[0]) - accum) <= 1e-12 * accum
