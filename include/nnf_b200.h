@@ -95,7 +95,7 @@ NNF_API int nnf_get_running_configuration(nnf_running_configuration * out);
 /* Knobs of the launch plans (process-wide; nothing in the library reads the environment). No counterpart in
  * the reference. name: "elementwise_waves", "elementwise_group_waves", "pool_waves", "pool_group_floats", "pool_staged",
  * "channel_waves", "group_waves", "chain_s_kb", "chain_a_kb", "chain_dist" (-1: built-in), "chain_chunk_mb",
- * "chain_lag" (lag + 1), "no_grouped", "apply_flat", "peer_wait_ns" (how long a batch-sharded launch waits for
+ * "chain_lag" (lag + 1), "chain_cluster" (99: not that form), "no_grouped", "apply_flat", "peer_wait_ns" (how long a batch-sharded launch waits for
  * another rank's statistics before it gives up; default 10 s), or "reset" (all back to the built-in choices).
  * A value <= 0 selects the built-in choice. Meant for tests that walk the geometries and for tuning. */
 NNF_API int nnf_set_tuning(const char * name, long long value);
@@ -262,10 +262,11 @@ NNF_API int nnf_bn_train_apply_act(nnf_stream_t stream, float * y, float * saved
 
 /* Single-GPU forward in one call and, for 16-byte aligned tensors whose planes are whole float4s or fill
  * channel groups, one launch: statistics items and apply items share it and the second read of x comes
- * from L2 (8 bytes/element through HBM). Other shapes run nnf_bn_train_stats + nnf_bn_train_apply_act,
- * for which `sums` (2C floats) is required. The workspace (nnf_bn_train_workspace_bytes, 16-byte aligned)
- * is always required: NNF_ERR_WORKSPACE without it. saved receives {mean, invstd}; sums (may be NULL for
- * single-launch shapes) receives {sum x, sum x^2}. Replaces
+ * from L2 (8 bytes/element through HBM). Aligned tensors whose channels fit the shared memory of a cluster
+ * of CTAs take one launch that holds them there instead. Other shapes run nnf_bn_train_stats +
+ * nnf_bn_train_apply_act. `sums` (2C floats, receives {sum x, sum x^2}) may be NULL where planes are whole
+ * float4s or fill channel groups. The workspace (nnf_bn_train_workspace_bytes, 16-byte aligned) is always
+ * required: NNF_ERR_WORKSPACE without it. saved receives {mean, invstd}. Replaces
  * batch_norm_layer_updater_cuda::enqueue_forward_propagation
  * (nnforge/cuda/batch_norm_layer_updater_cuda.cu:60-107) plus the activation layers behind it. */
 NNF_API int nnf_bn_train_fwd(nnf_stream_t stream, float * y, float * saved, float * sums, const float * x,

@@ -3,7 +3,7 @@
     python -m nnforge_b200.build
 
 -fmad=false for every file whose kernels are held to nnForge's plain (CPU) backend bit for bit: there products
-and sums must be rounded separately. The single-launch training batch norm (nnf_bn_chain.cu) is a tolerance
+and sums must be rounded separately. The single-launch training batch norm (nnf_bn_chain.cu, nnf_bn_cluster.cu) is a tolerance
 row - the reference's arithmetic there is cuDNN's - and is built with contraction: its launches are bound by
 how instruction issue and memory overlap, and every fused multiply-add is an instruction less.
 """
@@ -19,10 +19,10 @@ LIB = os.path.join(HERE, "libnnf_b200.so")
 HOST_LIB = os.path.join(HERE, "libnnf_b200_host.so")
 HOST_SRC = os.path.join(CSRC, "host", "nnf_layers.cpp")
 HOST_SOURCES = [HOST_SRC, os.path.join(CSRC, "host", "nnf_fusion.cpp"), os.path.join(CSRC, "host", "nnf_fused_layers.cpp")]
-SOURCES = ["nnf_api.cu", "nnf_elementwise.cu", "nnf_softmax.cu", "nnf_loss.cu", "nnf_maxpool.cu", "nnf_avgpool.cu", "nnf_optimizer.cu", "nnf_bn_train.cu", "nnf_bn_chain.cu", "nnf_peer.cu"]
+SOURCES = ["nnf_api.cu", "nnf_elementwise.cu", "nnf_softmax.cu", "nnf_loss.cu", "nnf_maxpool.cu", "nnf_avgpool.cu", "nnf_optimizer.cu", "nnf_bn_train.cu", "nnf_bn_chain.cu", "nnf_bn_cluster.cu", "nnf_peer.cu"]
 NVCC_FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
               "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
-CONTRACTING = {"nnf_bn_chain.cu"}   # sources built with FMA contraction; all others get -fmad=false
+CONTRACTING = {"nnf_bn_chain.cu", "nnf_bn_cluster.cu"}   # sources built with FMA contraction; all others get -fmad=false
 
 
 def _nvcc():

@@ -64,7 +64,7 @@ namespace nnf
 
 	tuning& tune()
 	{
-		static tuning t = {0, 0, 0, 0, 0, 0, 0, 0, 0, -1, 0, 0, 0, 0, 0};
+		static tuning t = {0, 0, 0, 0, 0, 0, 0, 0, 0, -1, 0, 0, 0, 0, 0, 0};
 		return t;
 	}
 }
@@ -97,7 +97,7 @@ extern "C" int nnf_set_tuning(const char * name, long long value)
 		{"pool_waves", &t.pool_waves}, {"pool_group_floats", &t.pool_group_floats}, {"pool_staged", &t.pool_staged},
 		{"channel_waves", &t.channel_waves}, {"group_waves", &t.group_waves},
 		{"chain_s_kb", &t.chain_s_kb}, {"chain_a_kb", &t.chain_a_kb}, {"chain_dist", &t.chain_dist},
-		{"chain_chunk_mb", &t.chain_chunk_mb}, {"chain_lag", &t.chain_lag},
+		{"chain_chunk_mb", &t.chain_chunk_mb}, {"chain_lag", &t.chain_lag}, {"chain_cluster", &t.chain_cluster},
 		{"no_grouped", &t.no_grouped}, {"apply_flat", &t.apply_flat},
 	};
 	if (strcmp(name, "peer_wait_ns") == 0)
@@ -107,7 +107,7 @@ extern "C" int nnf_set_tuning(const char * name, long long value)
 	}
 	if (strcmp(name, "reset") == 0)
 	{
-		t = nnf::tuning{0, 0, 0, 0, 0, 0, 0, 0, 0, -1, 0, 0, 0, 0, 0};
+		t = nnf::tuning{0, 0, 0, 0, 0, 0, 0, 0, 0, -1, 0, 0, 0, 0, 0, 0};
 		return NNF_OK;
 	}
 	for (const entry& e : table)

@@ -37,6 +37,7 @@
 //
 // Planes that are not whole float4s (7x7, 13x13) take the channel-group kernel further down, whose
 // items follow an older scheme (counters, chunks of channel groups, apply items that fold the sums).
+// On one GPU channels that fit the shared memory of a cluster are left to nnf_bn_cluster.cu.
 #include "nnf_common.cuh"
 
 #include <atomic>
@@ -299,26 +300,6 @@ namespace nnf
 		__device__ __forceinline__ size_t mail_index(const stream_params& p, uint32_t source_rank, uint32_t ch)
 		{
 			return ((size_t(p.seq & 1u) * kMaxRanks + source_rank) * p.c + ch) * 2;
-		}
-
-		// Backward through the chain from u = bn output: returns du, `term` = the PReLU slope gradient's term. PReLU
-		// followed by ELU, the chain the kernel is measured on, has a shorter form: the ELU's derivative for a
-		// negative input, (e^t - 1) + 1 in the layer-by-layer arithmetic, is taken as e^t itself (they differ by
-		// one rounding of a number near 1, far inside the tolerance of this row).
-		template <int A0, int A1>
-		__device__ __forceinline__ float stream_backward(const act_chain& ch, float u, float dy, float slope, float& term)
-		{
-			if constexpr (A0 == NNF_ACT_PRELU && A1 == NNF_ACT_ELU)
-			{
-				const float k = u >= 0.0F ? 1.0F : slope;
-				const float t1 = u * k;
-				const float e = fast_exp(t1);
-				const float g = dy * (t1 >= 0.0F ? 1.0F : e);
-				term = g * fminf(u, 0.0F);
-				return g * k;
-			}
-			else
-				return chain_backward<A0, A1>(ch, u, dy, slope, term);
 		}
 
 		template <int A0, int A1, bool BWD, bool PEER>
@@ -645,7 +626,7 @@ namespace nnf
 								const float xc = xs[j] - mean;
 								const float uu = fmaf(xc, mult, beta);
 								float term;
-								const float du = stream_backward<A0, A1>(p.chain, uu, ds[j], slope, term);
+								const float du = chain_backward_short<A0, A1>(p.chain, uu, ds[j], slope, term);
 								acc[0] += du;
 								acc[1] = fmaf(du, xc, acc[1]);
 								acc[K - 1] += term;
@@ -782,7 +763,7 @@ namespace nnf
 							const float xc = xs[j] - f0.w;
 							const float uu = fmaf(xc, f0.x, f1.x);
 							float term;
-							const float du = stream_backward<A0, A1>(p.chain, uu, ds[j], slope, term);
+							const float du = chain_backward_short<A0, A1>(p.chain, uu, ds[j], slope, term);
 							r_[j] = fmaf(du, f0.x, fmaf(xc, f0.y, f0.z));
 						}
 						o = make_float4(r_[0], r_[1], r_[2], r_[3]);
@@ -1569,6 +1550,12 @@ namespace nnf
 			return workspace && (reinterpret_cast<uintptr_t>(workspace) & 15) == 0 && have >= need;
 		}
 
+		// what the statistics kernels of the two-kernel form ask of a workspace: a call that they would refuse is refused in every form
+		bool two_kernel_workspace_ok(const void * workspace, size_t bytes, int64_t n, int64_t c, int64_t hw)
+		{
+			return workspace && bytes >= nnf_bn_train_workspace_bytes(n, c, hw) && (reinterpret_cast<uintptr_t>(workspace) & 7) == 0;
+		}
+
 		template <bool PEER>
 		int chain_forward_impl(cudaStream_t stream, float * y, float * saved, float * sums, const float * x, const float * gamma, const float * beta,
 			float eps, const act_chain& chain, int64_t n, int64_t c, int64_t hw, void * workspace, size_t workspace_bytes, const chain_peer * peer)
@@ -1580,6 +1567,12 @@ namespace nnf
 			{
 				if (!workspace_ok(workspace, workspace_bytes, chain_workspace_needed(gp)))
 					return 2;
+				if constexpr (!PEER)
+				{
+					const int st = cluster_train_fwd(stream, y, saved, sums, x, gamma, beta, eps, chain, n, c, hw, workspace, kClusterSliceGroups);
+					if (st != -1)
+						return st;
+				}
 				gp.x = x; gp.out = y; gp.gamma = gamma; gp.beta = beta; gp.saved = saved; gp.sums = sums;
 				gp.chain = chain;
 				gp.eps = eps;
@@ -1600,6 +1593,12 @@ namespace nnf
 				return 1;
 			if (!workspace_ok(workspace, workspace_bytes, stream_workspace_needed(p)))
 				return 2;
+			if constexpr (!PEER)
+			{
+				const int st = cluster_train_fwd(stream, y, saved, sums, x, gamma, beta, eps, chain, n, c, hw, workspace, kClusterSliceForward);
+				if (st != -1)
+					return st;
+			}
 			p.x = x; p.out = y; p.gamma = gamma; p.beta = beta; p.saved = saved; p.sums = sums;
 			p.chain = chain;
 			p.eps = eps;
@@ -1630,6 +1629,13 @@ namespace nnf
 			{
 				if (!workspace_ok(workspace, workspace_bytes, chain_workspace_needed(gp)))
 					return 2;
+				if constexpr (!PEER)
+				{
+					const int st = cluster_train_bwd(stream, dx, bsums, dy, x, gamma, beta, saved, chain, grad_gamma, grad_beta, grad_mean, grad_invsigma, grad_slope,
+						mean, invsigma, entry_count, n, c, hw, workspace, kClusterSliceGroups);
+					if (st != -1)
+						return st;
+				}
 				gp.x = x; gp.dy = dy; gp.out = dx; gp.gamma = gamma; gp.beta = beta; gp.saved = const_cast<float *>(saved); gp.sums = bsums;
 				gp.grad_gamma = grad_gamma; gp.grad_beta = grad_beta; gp.grad_mean = grad_mean; gp.grad_invsigma = grad_invsigma; gp.grad_slope = grad_slope;
 				gp.mean = mean; gp.invsigma = invsigma; gp.entry_count = entry_count;
@@ -1651,6 +1657,13 @@ namespace nnf
 				return 1;
 			if (!workspace_ok(workspace, workspace_bytes, stream_workspace_needed(p)))
 				return 2;
+			if constexpr (!PEER)
+			{
+				const int st = cluster_train_bwd(stream, dx, bsums, dy, x, gamma, beta, saved, chain, grad_gamma, grad_beta, grad_mean, grad_invsigma, grad_slope,
+					mean, invsigma, entry_count, n, c, hw, workspace, kClusterSliceBackward);
+				if (st != -1)
+					return st;
+			}
 			p.x = x; p.dy = dy; p.out = dx; p.gamma = gamma; p.beta = beta; p.saved = const_cast<float *>(saved); p.sums = bsums;
 			p.grad_gamma = grad_gamma; p.grad_beta = grad_beta; p.grad_mean = grad_mean; p.grad_invsigma = grad_invsigma; p.grad_slope = grad_slope;
 			p.mean = mean; p.invsigma = invsigma; p.entry_count = entry_count;
@@ -1846,6 +1859,12 @@ extern "C" int nnf_bn_train_fwd(nnf_stream_t stream, float * y, float * saved, f
 	// channel groups, extents beyond its index range): statistics kernel, then apply kernel
 	if (!sums)
 		return set_error(NNF_ERR_INVALID_ARGUMENT, "nnf_bn_train_fwd: this shape needs the two-kernel form, which requires the sums buffer");
+	if (aligned16(x) && aligned16(y) && two_kernel_workspace_ok(workspace, workspace_bytes, n, c, hw))
+	{
+		st = cluster_train_fwd((cudaStream_t)stream, y, saved, sums, x, gamma, beta, eps, chain, n, c, hw, nullptr, kClusterSliceAny);
+		if (st != -1)
+			return st;
+	}
 	st = nnf_bn_train_stats(stream, sums, x, n, c, hw, workspace, workspace_bytes);
 	if (st != NNF_OK)
 		return st;
@@ -1885,6 +1904,13 @@ extern "C" int nnf_bn_train_bwd(nnf_stream_t stream, float * dx, float * bsums, 
 				nnf_bn_train_workspace_bytes(n, c, hw), workspace_bytes);
 		if (st != 1)
 			return st;
+		if (aligned16(x) && aligned16(dy) && aligned16(dx) && two_kernel_workspace_ok(workspace, workspace_bytes, n, c, hw))
+		{
+			st = cluster_train_bwd((cudaStream_t)stream, dx, bsums, dy, x, gamma, beta, saved, chain, grad_gamma, grad_beta, grad_mean, grad_invsigma,
+				grad_slope, mean, invsigma, entry_count, n, c, hw, nullptr, kClusterSliceAny);
+			if (st != -1)
+				return st;
+		}
 	}
 	// dx accumulated into its destination, or a shape the single launch does not take: two kernels
 	st = nnf_bn_train_bwd_stats(stream, bsums, nullptr, dy, x, gamma, beta, saved, acts, n_acts, n, c, hw, workspace, workspace_bytes);

@@ -87,6 +87,7 @@ namespace nnf
 		int chain_s_kb, chain_a_kb;   // single-launch training kernel: KB of one tensor per statistics / apply item
 		int chain_dist;               // channels between an apply item and the statistics items it shares a step with
 		int chain_chunk_mb, chain_lag;// channel-group form of that kernel: chunk size and lag in chunks
+		int chain_cluster;            // CTAs per channel of the cluster form (1, 2, 4, 8); 99: never that form
 		int no_grouped;               // 1: planes that are not whole float4s take the per-channel kernels
 		int apply_flat;               // 1: training apply through the flat streaming kernel
 		long long peer_wait_ns;       // how long a launch waits for another rank's statistics before it gives up
@@ -324,6 +325,26 @@ namespace nnf
 		return g;
 	}
 
+	// Backward through the chain from u = bn output: returns du, `term` = the PReLU slope gradient's term. PReLU
+	// followed by ELU, the chain the kernel is measured on, has a shorter form (for the kernels built with contraction): the ELU's derivative for a
+	// negative input, (e^t - 1) + 1 in the layer-by-layer arithmetic, is taken as e^t itself (they differ by
+	// one rounding of a number near 1, far inside the tolerance of this row).
+	template <int A0, int A1>
+	__device__ __forceinline__ float chain_backward_short(const act_chain& ch, float u, float dy, float slope, float& term)
+	{
+		if constexpr (A0 == NNF_ACT_PRELU && A1 == NNF_ACT_ELU)
+		{
+			const float k = u >= 0.0F ? 1.0F : slope;
+			const float t1 = u * k;
+			const float e = fast_exp(t1);
+			const float g = dy * (t1 >= 0.0F ? 1.0F : e);
+			term = g * fminf(u, 0.0F);
+			return g * k;
+		}
+		else
+			return chain_backward<A0, A1>(ch, u, dy, slope, term);
+	}
+
 	__device__ __forceinline__ float chain_slope(const act_chain& ch, uint32_t channel)
 	{
 		float a = 0.0F;
@@ -465,6 +486,21 @@ namespace nnf
 
 	int make_peer_dst(peer_dst& d, void * const * peer_bufs, int rank, int world, int k, int kmax, uint32_t seq, const char * who);
 	int * device_error_word();
+
+	// Training batch norm of channels that fit a cluster's shared memory (nnf_bn_cluster.cu): -1 where this shape's do not.
+	// `report`: the 64 words at the head of the workspace that say the launch went well, or null. All tensors 16-byte aligned.
+	// `slice_limit`: most shared memory per CTA for which this form is taken, by what takes the shape otherwise. Measured on one
+	// B200, us: against the statistics and apply items of planes of whole float4s, whose second read comes from L2, slices of up to
+	// 56 KB win forward (x[128,512,28,28] 85 against 92; 98 KB: x[256,256,28,28] 98 against 80) and of up to 104 KB backward
+	// (x[512,128,14,14] 45.8 against 51.6; 196 KB: x[64,64,56,56] 54 against 47); against those of channel groups up to 104 KB
+	// (x[256,512,13,13] 45 / 71 against 57 / 88); against two kernels whatever fits (x[64,96,55,55] 40 / 75 against 60 / 151).
+	constexpr size_t kClusterSliceForward = 56 * 1024, kClusterSliceBackward = 104 * 1024, kClusterSliceGroups = 104 * 1024;
+	constexpr size_t kClusterSliceAny = ~size_t(0);
+	int cluster_train_fwd(cudaStream_t s, float * y, float * saved, float * sums, const float * x, const float * gamma, const float * beta, float eps,
+		const act_chain& chain, int64_t n, int64_t c, int64_t hw, void * report, size_t slice_limit);
+	int cluster_train_bwd(cudaStream_t s, float * dx, float * bsums, const float * dy, const float * x, const float * gamma, const float * beta, const float * saved,
+		const act_chain& chain, float * grad_gamma, float * grad_beta, float * grad_mean, float * grad_invsigma, float * grad_slope,
+		const float * mean, const float * invsigma, float entry_count, int64_t n, int64_t c, int64_t hw, void * report, size_t slice_limit);
 
 	// workspace of the single-launch training batch norm (nnf_bn_chain.cu)
 	size_t chain_workspace_bytes(int64_t n, int64_t c, int64_t hw);

@@ -122,3 +122,66 @@ def test_optimiser_step_chunk_counts_and_alignment(capi, oracle, kind, chunks):
                 assert_bits_equal(host(dp[name]), hp[name], "%s, chunk %d" % (name, k))
         # two orders of a double sum of at most 2050 terms of one sign: 2050 * 2^-53 < 3e-13 relative
         assert abs(float(host(dp["update_accum"])[0]) - accum) <= 1e-12 * accum
+
+
+# planes of whole float4s, planes of every remainder modulo 4, entries that do not divide by the CTAs, a tensor that ends inside a float4
+TRAIN_SHAPES = [(8, 3, 8, 8), (9, 4, 9, 9), (5, 5, 9, 11), (16, 3, 13, 10), (33, 7, 27, 27), (4, 2, 56, 56), (17, 6, 19, 21), (64, 1, 8, 8), (12, 3, 55, 57),
+                (7, 8, 7, 7), (5, 9, 4, 4)]
+
+
+@pytest.mark.parametrize("shape", TRAIN_SHAPES)
+@pytest.mark.parametrize("acts", ["none", "relu", "prelu_elu", "tanh"])
+@pytest.mark.parametrize("ctas", [0, 1, 2, 4, 8])
+def test_training_batch_norm_in_a_cluster(capi, tuning, shape, acts, ctas):
+    """The cluster form at every count of CTAs per channel, out of place and in place, against float64 arithmetic. y and dx carry
+    some ten roundings of 2^-24 and an exponential good to 2^-22: 1e-6 and 3e-6 of the 2-norm. A channel's gradient is a sum of m
+    terms of either sign around 1, each good to some 2^-22: 4e-6 * sqrt(m)."""
+    tuning("chain_cluster", ctas)
+    g = torch.Generator(device="cuda")
+    g.manual_seed(sum(shape) * 3 + ctas)
+    n, c, h, w = shape
+    x = torch.empty(shape, device="cuda").normal_(0.5, 2.0, generator=g)
+    dy = torch.empty(shape, device="cuda").normal_(generator=g)
+    gamma = torch.empty(c, device="cuda").uniform_(0.5, 1.5, generator=g)
+    beta, mean, slope = (torch.empty(c, device="cuda").normal_(0.0, 0.1, generator=g) for _ in range(3))
+    slope.abs_()
+    invsigma = torch.empty(c, device="cuda").uniform_(0.5, 1.5, generator=g)
+    per = lambda t: t.view(1, -1, 1, 1)
+
+    def norm(xd, ga, be):
+        var, mu = torch.var_mean(xd, dim=(0, 2, 3), correction=0)
+        inv = (var + 1e-5).rsqrt()
+        return (xd - per(mu)) * per(inv) * per(ga) + per(be), mu, inv
+
+    # off the rectifiers' kink, where two correct evaluations may be on different sides
+    x.add_((norm(x.double(), gamma.double(), beta.double())[0].abs() < 1e-4).float() * 0.01)
+    xd, sl, ga, be = (t.double().requires_grad_(True) for t in (x, slope, gamma, beta))
+    u, mu, inv = norm(xd, ga, be)
+    want = {"none": lambda: u, "relu": lambda: torch.relu(u), "tanh": lambda: torch.tanh(u),
+            "prelu_elu": lambda: torch.nn.functional.elu(torch.where(u >= 0, u, u * per(sl)))}[acts]()
+    want.backward(dy.double())
+    chain = {"none": [], "relu": [capi.relu()], "prelu_elu": [capi.prelu(slope), capi.elu()], "tanh": [capi.tanh(1.0, 1.0)]}[acts]
+    ws = torch.empty(capi.bn_train_workspace_bytes(n, c, h * w), dtype=torch.uint8, device="cuda")
+    close = lambda a, b, tol: float((a.double() - b.detach()).norm()) <= tol * float(b.detach().norm()) + 1e-12
+    room = 4e-6 * (n * h * w) ** 0.5
+    for in_place in (False, True):
+        y = x.clone() if in_place else torch.full_like(x, float("nan"))
+        saved, sums, bsums = (torch.full((k * c,), float("nan"), device="cuda") for k in (2, 2, 3))
+        capi.bn_train_fwd(y, saved, sums, y if in_place else x, gamma, beta, 1e-5, chain, workspace=ws)
+        assert close(y, want, 1e-6)
+        assert close(saved[:c], mu, 1e-6) and close(saved[c:], inv, 1e-6)
+        assert close(sums[:c], xd.sum((0, 2, 3)), 2e-6) and close(sums[c:], (xd ** 2).sum((0, 2, 3)), 2e-6)
+        grads = [torch.full((c,), 0.25, device="cuda") for _ in range(5)]
+        dx = dy.clone() if in_place else torch.full_like(x, float("nan"))
+        capi.bn_train_bwd(dx, bsums, dx if in_place else dy, x, gamma, beta, saved, chain, grad_gamma=grads[0], grad_beta=grads[1], grad_mean=grads[2],
+                          grad_invsigma=grads[3], grad_slope=grads[4] if acts == "prelu_elu" else None, mean=mean, invsigma=invsigma, entry_count=float(n),
+                          workspace=ws)
+        assert close(dx, xd.grad, 3e-6)
+        for got, gradient in ((grads[0], ga), (grads[1], be)) + (((grads[4], sl),) if acts == "prelu_elu" else ()):
+            assert float((got.double() - 0.25 - gradient.grad).abs().max()) <= room
+        assert close(grads[2] - 0.25, n * (saved[:c] - mean).double(), 1e-5) and close(grads[3] - 0.25, n * (saved[c:] - invsigma).double(), 1e-5)
+        if h * w % 4 == 0:
+            report = torch.zeros(capi.REPORT_WORDS, dtype=torch.int64).pin_memory()
+            capi.read_report(report, ws)
+            torch.cuda.synchronize()
+            assert capi.parse_report(report)["status"] == 0
