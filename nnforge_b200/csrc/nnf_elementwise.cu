@@ -125,6 +125,57 @@ namespace nnf
 			return chain_forward<A0, A1>(p.chain, t, q.slope);
 		}
 
+		// Four elements of one channel: what an element takes is decided once per vector. TanH alone looks at the four exponents
+		// together: only if one of them is beyond 2^126, where act_fwd must look at the quotient, does the vector go through act_fwd (the
+		// same bits either way). On tensors of gigabytes TanH is bound by instructions, the more so once the power limit lowers the
+		// clocks: x[1024,128,64,64] 743 -> 719 us with this, ReLU 630.
+		template <int A0, int A1>
+		__device__ __forceinline__ float4 ew_vector(const ew_params& p, bool has_bn, bool has_res, const elem_params& q, float4 x, float4 r)
+		{
+			float t[4] = {x.x, x.y, x.z, x.w};
+			if (p.bias)
+			{
+				#pragma unroll
+				for (int i = 0; i < 4; ++i)
+					t[i] = __fadd_rn(t[i], q.bias);
+			}
+			if (has_bn)
+			{
+				#pragma unroll
+				for (int i = 0; i < 4; ++i)
+					t[i] = __fadd_rn(__fmul_rn(t[i], q.mult), q.add);
+			}
+			if (has_res)
+			{
+				const float rs[4] = {r.x, r.y, r.z, r.w};
+				#pragma unroll
+				for (int i = 0; i < 4; ++i)
+					t[i] = __fmul_rn(__fadd_rn(__fadd_rn(0.0F, t[i]), rs[i]), p.add_alpha);
+			}
+			if constexpr (A0 == NNF_ACT_TANH && A1 == 0)
+			{
+				const float p0 = p.chain.a[0].p0, p1 = p.chain.a[0].p1;
+				float s[4];
+				#pragma unroll
+				for (int i = 0; i < 4; ++i)
+					s[i] = __fmul_rn(t[i], p1);
+				if (fmaxf(fmaxf(s[0], s[1]), fmaxf(s[2], s[3])) < 87.0F)   // e^87 < 2^126; a NaN passes through the quotient
+				{
+					#pragma unroll
+					for (int i = 0; i < 4; ++i)
+					{
+						const float e = fast_exp(s[i]);
+						t[i] = __fmul_rn(__fmul_rn(__fsub_rn(e, 1.0F), fast_rcp(__fadd_rn(e, 1.0F))), p0);
+					}
+					return make_float4(t[0], t[1], t[2], t[3]);
+				}
+			}
+			#pragma unroll
+			for (int i = 0; i < 4; ++i)
+				t[i] = chain_forward<A0, A1>(p.chain, t[i], q.slope);
+			return make_float4(t[0], t[1], t[2], t[3]);
+		}
+
 		// MODE 0: 128-bit accesses, one channel per vector (hw % 4 == 0, or no per-channel parameters)
 		// MODE 1: 128-bit accesses, channel derived per element (planes not multiples of 4 elements)
 		// MODE 2: scalar accesses (a buffer is not 16-byte aligned)
@@ -249,10 +300,7 @@ namespace nnf
 						if (MODE == 0)
 						{
 							const elem_params q = fetch_params(p, s_mult, s_add, e);
-							o.x = ew_element<A0, A1>(p, has_bn, has_res, q, xv[j].x, rv[j].x);
-							o.y = ew_element<A0, A1>(p, has_bn, has_res, q, xv[j].y, rv[j].y);
-							o.z = ew_element<A0, A1>(p, has_bn, has_res, q, xv[j].z, rv[j].z);
-							o.w = ew_element<A0, A1>(p, has_bn, has_res, q, xv[j].w, rv[j].w);
+							o = ew_vector<A0, A1>(p, has_bn, has_res, q, xv[j], rv[j]);
 						}
 						else if (p.hw.d >= 4)
 						{

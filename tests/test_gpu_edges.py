@@ -185,3 +185,21 @@ def test_training_batch_norm_in_a_cluster(capi, tuning, shape, acts, ctas):
             capi.read_report(report, ws)
             torch.cuda.synchronize()
             assert capi.parse_report(report)["status"] == 0
+
+
+def test_tanh_vectors_with_large_exponents(capi, oracle):
+    """Vectors of which no, one or every element's exponent is beyond 2^126, up to overflow, infinities and NaN."""
+    g = synth.rng(1, salt=77)
+    x = synth.normal(g, (3, 4, 8, 8), 0.0, 20.0)
+    x.reshape(-1)[::7] *= 40.0
+    x[0, 0, 0] = [43.4, 43.6, 44.3, 44.4, 87.0, -87.0, 1e30, -1e30]
+    x[0, 0, 1, :5] = [np.inf, -np.inf, np.nan, 0.0, -0.0]
+    one, zero = np.ones(4, np.float32), np.zeros(4, np.float32)
+    y = torch.empty(x.shape, device="cuda")
+    capi.bn_infer_act(y, dev(x), bn=[dev(a) for a in (one, zero, zero, one)], acts=[capi.tanh(1.0, 1.0)])
+    want = oracle.tanh_fwd(x, 1.0, 1.0)
+    got = host(y)
+    assert (np.isnan(got) == np.isnan(want)).all()
+    ok = ~np.isnan(want)
+    # the exponential is good to 2^-22 + 6e-8 |2 x| relative, which a quotient near 1 hardly sees
+    assert np.abs(got[ok] - want[ok]).max() <= 1e-6
