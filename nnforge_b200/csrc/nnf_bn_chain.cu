@@ -11,7 +11,12 @@
 //   F(channel)         one warp: waits (bounded) until every deposit of the channel carries the tag, adds
 //                      them in a fixed order in double, derives the channel's constants (and writes the
 //                      per-channel outputs), releases the channel's apply items
-//   A(channel, slice)  apply: issues its first copies, then waits (bounded) for F(channel), normalises
+//   A(channel, slice)  apply: issues its first copies, then waits (bounded) for F(channel)'s two constants, normalises
+// The constants travel like the deposits, as words that carry the launch's tag, and F writes them before the per-channel
+// results: an A item whose channel is finished needs one round trip for them. With a flag in front of five constants (release,
+// acquire, two round trips, F's gradient updates before the flag) x[256,256,28,28] took 82.4 / 151.6 us forward / backward, now
+// 80.6 / 125.3. Thread 0 asks and the CTA's barrier hands the answer on: every warp asking for itself, with no barrier, let the
+// warps of a CTA drift apart and cost the forward launch 15 %.
 // Ticket step k holds S(k), F(k - dist/2) and A(k - dist), interleaved, so that the apply items of a
 // channel run while later channels' statistics are being read: the lines of x that the S items pulled in
 // a few microseconds earlier are still in the 126 MB L2 (they are loaded with an evict-last hint, the
@@ -248,9 +253,8 @@ namespace nnf
 			double count, count_total;         // elements per channel on this rank / over all ranks
 			float eps;
 			uint32_t tag;                      // this launch's tag in the deposit words
+			unsigned long long * constants;    // [c][2] tagged words: what the A items cannot know without the channel's sums
 			unsigned long long * deposit;      // [c][ss][4] tagged words
-			float4 * fin;                      // [c][2] per-channel constants for the A items
-			uint32_t * ready;                  // [c]
 			launch_report * report;
 			int * error_word;                  // the library's process-wide word: raised too, never consulted
 			// batch-sharded runs: mail[r] = mailbox of rank r (peer memory), mail[rank] this GPU's own;
@@ -271,6 +275,12 @@ namespace nnf
 			unsigned long long v;
 			asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
 			return v;
+		}
+
+		__device__ __forceinline__ void ld_relaxed_u64x2(const unsigned long long * p, unsigned long long& a, unsigned long long& b)
+		{
+			// two words that validate themselves: nothing is asked of the pair as a whole
+			asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "l"(p) : "memory");
 		}
 
 		__device__ __forceinline__ void st_release_u32(uint32_t * p, uint32_t v)
@@ -312,8 +322,8 @@ namespace nnf
 			constexpr int STAGES = BWD ? kStagesBwd : kStagesFwd;
 			extern __shared__ float4 ring[];   // [STAGES][T][L][kChainThreads]: a thread reads back only what it copied itself
 			__shared__ uint32_t s_item[4];
-			__shared__ float4 s_fin[2];
 			__shared__ float s_sum[kStreamWarps][3];
+			__shared__ float s_constants[2];
 
 			if (threadIdx.x == 0)
 			{
@@ -478,34 +488,38 @@ namespace nnf
 					const unsigned long long waited = chain_timer_ns() - t0;
 					atomicAdd(&p.report->wait_ns_total, waited);
 					atomicMax(&p.report->wait_ns_max, waited);
-					float4 f0v, f1v = make_float4(0.0F, 0.0F, 0.0F, 0.0F);
+					// the constants first: the channel's apply items may be waiting for them
+					float fmean = 0.0F, finv = 0.0F, k0, k1;
 					if (!BWD)
 					{
 						var_d = var_d < 0.0 ? 0.0 : var_d;
-						const float fmean = float(mean_d);
-						const float finv = float(1.0 / sqrt(var_d + double(p.eps)));
-						const float mult = __ldg(p.gamma + ch) * finv;
-						f0v = make_float4(mult, fmaf(-mult, fmean, __ldg(p.beta + ch)), 0.0F, 0.0F);
-						p.saved[ch] = fmean;
-						p.saved[p.c + ch] = finv;
-						if (p.sums)
-						{
-							p.sums[ch] = m0;
-							p.sums[p.c + ch] = m1;
-						}
+						fmean = float(mean_d);
+						finv = float(1.0 / sqrt(var_d + double(p.eps)));
+						k0 = __ldg(p.gamma + ch) * finv;
+						k1 = fmaf(-k0, fmean, __ldg(p.beta + ch));
 					}
 					else
 					{
-						const float mult = __ldg(p.gamma + ch) * saved_invstd;
 						// dx = mult * ((du - c2) - xhat * c3) with xhat = (x - mean) * invstd, as two fused multiply-adds
-						f0v = make_float4(mult, -(mult * c3 * saved_invstd), -(mult * c2), saved_mean);
-						f1v = make_float4(__ldg(p.beta + ch), 0.0F, 0.0F, 0.0F);
-						if (p.sums)
-						{
-							p.sums[ch] = m0;
-							p.sums[p.c + ch] = m1;
-							p.sums[2 * p.c + ch] = m2;
-						}
+						const float mult = __ldg(p.gamma + ch) * saved_invstd;
+						k0 = -(mult * c3 * saved_invstd);
+						k1 = -(mult * c2);
+					}
+					st_relaxed_u64(p.constants + 2 * ch, (static_cast<unsigned long long>(p.tag) << 32) | __float_as_uint(k0));
+					st_relaxed_u64(p.constants + 2 * ch + 1, (static_cast<unsigned long long>(p.tag) << 32) | __float_as_uint(k1));
+					if (!BWD)
+					{
+						p.saved[ch] = fmean;
+						p.saved[p.c + ch] = finv;
+					}
+					if (p.sums)
+					{
+						p.sums[ch] = m0;
+						p.sums[p.c + ch] = m1;
+						if (BWD) p.sums[2 * p.c + ch] = m2;
+					}
+					if (BWD)
+					{
 						// per-channel gradients accumulate this rank's sums (batch_norm_layer_updater_cuda.cu:138-139, 167-182)
 						if (p.grad_beta) p.grad_beta[ch] += m0;
 						if (p.grad_gamma) p.grad_gamma[ch] += m1;
@@ -513,9 +527,6 @@ namespace nnf
 						if (p.grad_mean) p.grad_mean[ch] += p.entry_count * (saved_mean - p.mean[ch]);
 						if (p.grad_invsigma) p.grad_invsigma[ch] += p.entry_count * (saved_invstd - p.invsigma[ch]);
 					}
-					p.fin[2 * ch] = f0v;
-					p.fin[2 * ch + 1] = f1v;
-					st_release_u32(p.ready + ch, 1u);
 				}
 				return;
 			}
@@ -697,17 +708,19 @@ namespace nnf
 			#pragma unroll
 			for (int g = 0; g < STAGES; ++g)
 				issue(g);
+			const float mean = BWD ? __ldg(p.saved + ch) : 0.0F;
+			const float mult = BWD ? __ldg(p.gamma + ch) * __ldg(p.saved + p.c + ch) : 0.0F;
+			const float beta = BWD ? __ldg(p.beta + ch) : 0.0F;
 			if (threadIdx.x == 0)
 			{
 				bool ok = false;
-				unsigned long long t0 = 0;
+				unsigned long long t0 = 0, w0 = 0, w1 = 0;
 				for (uint32_t round = 0; round < kChainPollLimit; ++round)
 				{
-					if (ld_acquire(p.ready + ch) != 0)
-					{
-						ok = true;
+					ld_relaxed_u64x2(p.constants + 2 * ch, w0, w1);
+					ok = uint32_t(w0 >> 32) == p.tag && uint32_t(w1 >> 32) == p.tag;
+					if (ok)
 						break;
-					}
 					if (round == 0)
 						t0 = chain_timer_ns();
 					if ((round & 63) == 63 && *reinterpret_cast<volatile int *>(&p.report->status) != 0)
@@ -725,12 +738,11 @@ namespace nnf
 					p.report->status = 4;
 					if (p.error_word) *p.error_word = 4;
 				}
-				s_fin[0] = __ldcg(p.fin + 2 * ch);
-				s_fin[1] = __ldcg(p.fin + 2 * ch + 1);
+				s_constants[0] = __uint_as_float(uint32_t(w0));
+				s_constants[1] = __uint_as_float(uint32_t(w1));
 			}
 			__syncthreads();
-			const float4 f0 = s_fin[0];
-			const float4 f1 = s_fin[1];
+			const float k0 = s_constants[0], k1 = s_constants[1];
 			uint32_t crs = 0, cct = 0, coff = 0;
 			int g = 0;
 			while (row_sweeps)
@@ -746,10 +758,10 @@ namespace nnf
 					float4 o;
 					if (!BWD)
 					{
-						o.x = chain_forward<A0, A1>(p.chain, fmaf(a.x, f0.x, f0.y), slope);
-						o.y = chain_forward<A0, A1>(p.chain, fmaf(a.y, f0.x, f0.y), slope);
-						o.z = chain_forward<A0, A1>(p.chain, fmaf(a.z, f0.x, f0.y), slope);
-						o.w = chain_forward<A0, A1>(p.chain, fmaf(a.w, f0.x, f0.y), slope);
+						o.x = chain_forward<A0, A1>(p.chain, fmaf(a.x, k0, k1), slope);
+						o.y = chain_forward<A0, A1>(p.chain, fmaf(a.y, k0, k1), slope);
+						o.z = chain_forward<A0, A1>(p.chain, fmaf(a.z, k0, k1), slope);
+						o.w = chain_forward<A0, A1>(p.chain, fmaf(a.w, k0, k1), slope);
 					}
 					else
 					{
@@ -760,11 +772,11 @@ namespace nnf
 						#pragma unroll
 						for (int j = 0; j < 4; ++j)
 						{
-							const float xc = xs[j] - f0.w;
-							const float uu = fmaf(xc, f0.x, f1.x);
+							const float xc = xs[j] - mean;
+							const float uu = fmaf(xc, mult, beta);
 							float term;
 							const float du = chain_backward_short<A0, A1>(p.chain, uu, ds[j], slope, term);
-							r_[j] = fmaf(du, f0.x, fmaf(xc, f0.y, f0.z));
+							r_[j] = fmaf(du, mult, fmaf(xc, k0, k1));
 						}
 						o = make_float4(r_[0], r_[1], r_[2], r_[3]);
 					}
@@ -1325,8 +1337,8 @@ namespace nnf
 
 		// Geometry of the kernel for planes of whole float4s. Defaults measured on B200 with x[256,256,28,28],
 		// PReLU+ELU (forward / backward): items of 48 KB (statistics) and 64 KB (apply) of one tensor, apply items 32 /
-		// 24 channels behind the statistics items: 86 / 150 us. Shorter distances make every apply item wait for its
-		// channel (16 channels: 94 / 164 us), longer ones push the first read out of L2 before the second.
+		// 24 channels behind the statistics items: 81 / 125 us. Shorter distances make every apply item wait for its
+		// channel (16 channels: 85 / 128 us), longer ones push the first read out of L2 before the second.
 		// Knobs: chain_s_kb, chain_a_kb, chain_dist (nnf_set_tuning).
 		bool plan_stream(stream_params& p, int64_t n, int64_t c, int64_t hw, bool backward, bool sharded = false)
 		{
@@ -1479,10 +1491,8 @@ namespace nnf
 		{
 			launch_report * report = static_cast<launch_report *>(workspace);
 			p.report = report;
-			p.ready = reinterpret_cast<uint32_t *>(report + 1);
-			char * after = reinterpret_cast<char *>(p.ready) + (size_t(p.c) * sizeof(uint32_t) + 15) / 16 * 16;
-			p.fin = reinterpret_cast<float4 *>(after);
-			p.deposit = reinterpret_cast<unsigned long long *>(p.fin + size_t(p.c) * 2);
+			p.constants = reinterpret_cast<unsigned long long *>(report + 1);
+			p.deposit = p.constants + size_t(p.c) * 2;
 			p.error_word = device_error_word();
 			p.wait_limit_ns = peer_wait_limit();
 			uint32_t tag = ++g_launch_tag;
@@ -1493,7 +1503,8 @@ namespace nnf
 			cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "%s: cudaFuncSetAttribute: %s", what, cudaGetErrorString(e));
-			e = cudaMemsetAsync(workspace, 0, sizeof(launch_report) + size_t(p.c) * sizeof(uint32_t), s);
+			// the words too: a launch that is replayed from a graph carries the tag it was captured with
+			e = cudaMemsetAsync(workspace, 0, sizeof(launch_report) + size_t(p.c) * (2 + size_t(p.ss) * 4) * sizeof(unsigned long long), s);
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "%s: cudaMemsetAsync: %s", what, cudaGetErrorString(e));
 			launch(kernel, p.total, kChainThreads, smem, s, p);

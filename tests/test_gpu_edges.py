@@ -203,3 +203,34 @@ def test_tanh_vectors_with_large_exponents(capi, oracle):
     ok = ~np.isnan(want)
     # the exponential is good to 2^-22 + 6e-8 |2 x| relative, which a quotient near 1 hardly sees
     assert np.abs(got[ok] - want[ok]).max() <= 1e-6
+
+
+def test_training_batch_norm_replayed_from_a_graph(capi, tuning):
+    """The launch of statistics, finishing and apply items, captured once and replayed with other inputs in the same buffers: nothing
+    that an earlier replay left in the workspace may pass for this one's."""
+    tuning("chain_cluster", 99)
+    shape = (64, 24, 28, 28)
+    c = shape[1]
+    x, dy, y, dx = (torch.zeros(shape, device="cuda") for _ in range(4))
+    gamma, beta = torch.full((c,), 1.25, device="cuda"), torch.full((c,), 0.1, device="cuda")
+    saved, sums, bsums = (torch.zeros(k * c, device="cuda") for k in (2, 2, 3))
+    ws = torch.zeros(capi.bn_train_workspace_bytes(shape[0], c, 784), dtype=torch.uint8, device="cuda")
+
+    def step():
+        capi.bn_train_fwd(y, saved, sums, x, gamma, beta, 1e-5, [capi.relu()], workspace=ws)
+        capi.bn_train_bwd(dx, bsums, dy, x, gamma, beta, saved, [capi.relu()], workspace=ws)
+
+    step()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph, stream=side):
+        step()
+    for k in range(4):
+        x.normal_(float(k), 1.0 + k)
+        dy.normal_()
+        graph.replay()
+        got = [host(t).copy() for t in (y, saved, dx, bsums)]
+        step()
+        for a, t in zip(got, (y, saved, dx, bsums)):
+            assert_bits_equal(a, host(t), "replay %d" % k)
