@@ -45,6 +45,7 @@
 // On one GPU channels that fit the shared memory of a cluster are left to nnf_bn_cluster.cu.
 #include "nnf_common.cuh"
 
+#include <algorithm>
 #include <atomic>
 #include <mutex>
 
@@ -1373,7 +1374,11 @@ namespace nnf
 			// batch-sharded launches: a channel's constants also wait for the other ranks' sums (an NVLink round trip and whatever
 			// the ranks are apart), so the forward launch keeps a longer distance (two GPUs, before the staging ring: 119 us at
 			// 48 against 127-130 at 32; with it 88 us at either)
-			int64_t dist = t.chain_dist >= 0 ? t.chain_dist : (backward ? 24 : (sharded ? 48 : 32));
+			// On one GPU the distance in bytes decides, 26 MB of x forward and 19 MB each of x and dy backward: with 32 / 24 channels of
+			// 3.2 MB the second read came from HBM (x[64,64,112,112] 91 / 148 us, at 8 / 6 channels 76 / 114; x[128,32,112,112], 6.4 MB,
+			// 94 / 154 us, at 4 channels 77 / 118; x[512,128,28,28], 1.6 MB, 86 / 146 us, at 16 / 12 channels 78 / 118).
+			const int64_t most = backward ? 24 : 32, bytes = backward ? 19300000 : 25700000, channel = n * plane_bytes;
+			int64_t dist = t.chain_dist >= 0 ? t.chain_dist : sharded ? (backward ? 24 : 48) : std::max(int64_t(2), std::min(most, (bytes + channel / 2) / channel));
 			if (dist > c) dist = c;
 			p.dist = (uint32_t)dist;
 			p.dist_f = (uint32_t)(dist / 2);
