@@ -490,7 +490,7 @@ namespace nnf
 	// Training batch norm of channels that fit a cluster's shared memory (nnf_bn_cluster.cu): -1 where this shape's do not.
 	// `report`: the 64 words at the head of the workspace that say the launch went well, or null. All tensors 16-byte aligned.
 	// `slice_limit`: most shared memory per CTA for which this form is taken, by what takes the shape otherwise. Measured on one
-	// B200, us: against the statistics and apply items of planes of whole float4s, whose second read comes from L2, slices of up to
+	// B200 before the items' constants carried their own tag, us: against the statistics and apply items of planes of whole float4s, whose second read comes from L2, slices of up to
 	// 56 KB win forward (x[128,512,28,28] 85 against 92; 98 KB: x[256,256,28,28] 98 against 80) and of up to 104 KB backward
 	// (x[512,128,14,14] 45.8 against 51.6; 196 KB: x[64,64,56,56] 54 against 47); against those of channel groups up to 104 KB
 	// (x[256,512,13,13] 45 / 71 against 57 / 88); against two kernels whatever fits (x[64,96,55,55] 40 / 75 against 60 / 151).
