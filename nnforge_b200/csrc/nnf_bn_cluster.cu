@@ -147,8 +147,9 @@ namespace nnf
 				for (uint32_t i = g * p.per_stage + threadIdx.x; i < end; i += threads)
 				{
 					const piece<WHOLE> f(p, start, i);
-					// a frame may be a piece shorter than the pitch, and the tensor may end inside the last one
-					const uint32_t bytes = WHOLE ? 16 : f.hi > 0 ? min(16u, (p.total - f.at) * 4) : 0;
+					// a frame may be a piece shorter than the pitch, and the tensor may end inside the last one (the elements that are
+					// left are compared before they become bytes, which 32 bits do not hold from 2^30 elements on)
+					const uint32_t bytes = WHOLE ? 16 : f.hi > 0 ? min(4u, p.total - f.at) * 4 : 0;
 					const uint32_t at = WHOLE || bytes > 0 ? f.at : 0;
 					copy16(tile + i, p.x + at, bytes);
 					if (BWD)

@@ -187,6 +187,35 @@ def test_training_batch_norm_in_a_cluster(capi, tuning, shape, acts, ctas):
             assert capi.parse_report(report)["status"] == 0
 
 
+def test_training_batch_norm_in_a_cluster_beyond_2_to_30_elements(capi):
+    """Ragged planes of a tensor whose bytes do not fit 32 bits: the channel whose first elements are 2^30 elements from the tensor's end,
+    those next to it and those at both ends, against float64 arithmetic (tolerances as above)."""
+    n, c, h, w = 4, 368228, 27, 27
+    total = n * c * h * w
+    assert 2 ** 30 < total < 2 ** 31
+    if torch.cuda.mem_get_info()[0] < 24 * 2 ** 30:
+        pytest.skip("needs 24 GiB of device memory")
+    g = torch.Generator(device="cuda")
+    g.manual_seed(30)
+    x, dy = (torch.empty((n, c, h, w), device="cuda").normal_(mu, 1.5, generator=g) for mu in (1.0, 0.0))
+    gamma = torch.empty(c, device="cuda").uniform_(0.5, 1.5, generator=g)
+    beta = torch.empty(c, device="cuda").normal_(0.0, 0.1, generator=g)
+    y, dx = (torch.full_like(x, float("nan")) for _ in range(2))
+    saved, sums, bsums = (torch.empty(k * c, device="cuda") for k in (2, 2, 3))
+    ws = torch.empty(capi.bn_train_workspace_bytes(n, c, h * w), dtype=torch.uint8, device="cuda")
+    capi.bn_train_fwd(y, saved, sums, x, gamma, beta, 1e-5, [], workspace=ws)
+    capi.bn_train_bwd(dx, bsums, dy, x, gamma, beta, saved, [], workspace=ws)
+    at = (total - 2 ** 30) // (h * w)
+    pick = torch.tensor([0, 1, at - 1, at, at + 1, c - 2, c - 1], device="cuda")
+    xd, ga, be = (t[:, pick].double().requires_grad_(True) if t is x else t[pick].double().requires_grad_(True) for t in (x, gamma, beta))
+    want = torch.nn.functional.batch_norm(xd, None, None, ga, be, training=True, eps=1e-5)
+    want.backward(dy[:, pick].double())
+    norm = lambda t: (t * t).sum((0, 2, 3)).sqrt()
+    assert bool((norm(y[:, pick].double() - want) <= 1e-6 * norm(want)).all())
+    assert bool((norm(dx[:, pick].double() - xd.grad) <= 3e-6 * norm(xd.grad)).all())
+    assert not bool(torch.isnan(y.view(-1)).any()) and not bool(torch.isnan(dx.view(-1)).any())
+
+
 def test_tanh_vectors_with_large_exponents(capi, oracle):
     """Vectors of which no, one or every element's exponent is beyond 2^126, up to overflow, infinities and NaN."""
     g = synth.rng(1, salt=77)
