@@ -358,6 +358,14 @@ namespace nnf
 			}
 		}
 
+		// Most shared memory that a CTA may ask for: what all CTAs of an SM can share, and no more than a CTA may have beside the
+		// kernel's static arrays (less than 1 KB).
+		int cluster_smem_limit()
+		{
+			const int optin = running_config().max_shared_memory_per_block_optin - 1024, budget = (int)sm_smem_budget();
+			return budget < optin ? budget : optin;
+		}
+
 		struct cluster_plan
 		{
 			int threads;
@@ -389,7 +397,7 @@ namespace nnf
 				while (k < int64_t(kClusterMax) && c * k <= sms && slice(k) > 4 * 1024)
 					k *= 2;
 			}
-			const int64_t bytes = slice(k), room = sm_smem_budget();
+			const int64_t bytes = slice(k), room = cluster_smem_limit();
 			if (k > int64_t(kClusterMax) || bytes > room || size_t(bytes) > slice_limit)
 				return false;
 			p.cluster = (uint32_t)k;
@@ -414,7 +422,9 @@ namespace nnf
 		int launch_cluster(const cluster_params& p, const cluster_plan& plan, cudaStream_t s, const char * what)
 		{
 			auto kernel = bn_train_cluster_kernel<A0, A1, BWD, WHOLE>;
-			const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)plan.smem);
+			// the attribute is the kernel's, not the launch's: the same value whatever the shape, so that host threads with different
+			// shapes do not lower it under each other's launches
+			const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, cluster_smem_limit());
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "%s: cudaFuncSetAttribute: %s", what, cudaGetErrorString(e));
 			cudaLaunchAttribute attr[2];

@@ -216,6 +216,54 @@ def test_training_batch_norm_in_a_cluster_beyond_2_to_30_elements(capi):
     assert not bool(torch.isnan(y.view(-1)).any()) and not bool(torch.isnan(dx.view(-1)).any())
 
 
+def test_host_threads_launch_clusters_of_different_sizes(capi):
+    """Two threads, each on its own stream, with channels that need 50 KB and 512 bytes of shared memory per CTA (twice that backward) in the same
+    instantiation: a launch does not depend on what the other thread's needs. Same results as from one thread."""
+    import threading
+
+    def state(shape, seed):
+        g = torch.Generator(device="cuda")
+        g.manual_seed(seed)
+        c = shape[1]
+        x, dy = (torch.empty(shape, device="cuda").normal_(generator=g) for _ in range(2))
+        gamma, beta = torch.ones(c, device="cuda"), torch.zeros(c, device="cuda")
+        y, dx = torch.empty_like(x), torch.empty_like(x)
+        saved, sums, bsums = (torch.empty(k * c, device="cuda") for k in (2, 2, 3))
+        ws = torch.empty(capi.bn_train_workspace_bytes(shape[0], c, shape[2] * shape[3]), dtype=torch.uint8, device="cuda")
+        return x, dy, gamma, beta, y, dx, saved, sums, bsums, ws, torch.cuda.Stream()
+
+    def step(s):
+        x, dy, gamma, beta, y, dx, saved, sums, bsums, ws, stream = s
+        capi.bn_train_fwd(y, saved, sums, x, gamma, beta, 1e-5, [], workspace=ws, stream=stream)
+        capi.bn_train_bwd(dx, bsums, dy, x, gamma, beta, saved, [], workspace=ws, stream=stream)
+
+    states = [state((16, 160, 28, 28), 1), state((2, 160, 8, 8), 2)]
+    torch.cuda.synchronize()
+    want = []
+    for s in states:
+        step(s)
+        want.append([host(t).copy() for t in (s[4], s[5], s[6], s[8])])
+    failures = []
+
+    def work(s):
+        try:
+            for _ in range(4000):
+                step(s)
+        except Exception as e:
+            failures.append(e)
+
+    threads = [threading.Thread(target=work, args=(s,)) for s in states]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert not failures, failures
+    for s, w in zip(states, want):
+        for t, a in zip((s[4], s[5], s[6], s[8]), w):
+            assert_bits_equal(host(t), a, "threads")
+
+
 def test_tanh_vectors_with_large_exponents(capi, oracle):
     """Vectors of which no, one or every element's exponent is beyond 2^126, up to overflow, infinities and NaN."""
     g = synth.rng(1, salt=77)
