@@ -38,31 +38,33 @@ namespace
 	};
 
 	// Reads the positional arguments of one call in order. The first conversion that fails leaves its exception set, and
-	// the rest of the reads return zeros.
+	// the rest of the reads return zeros without looking at their argument: nothing may call into Python, or clear an exception,
+	// while one is set.
 	class arguments
 	{
 	public:
-		arguments(PyObject * const * a, Py_ssize_t n) : a(a), n(n) {}
+		// `streamed`: the last argument is the stream. It is read before the others, as a caller without a device hears of that
+		// before it hears of anything else.
+		arguments(PyObject * const * a, Py_ssize_t n, bool streamed) : a(a), n(n)
+		{
+			if (streamed && n > 0)
+				read_stream(a[n - 1]);
+		}
 
 		bool ok() const { return good; }
 
 		PyObject * next()
 		{
 			if (i >= n)
-			{
-				if (good)
-					PyErr_SetString(PyExc_TypeError, "missing argument");
-				good = false;
-				return Py_None;
-			}
-			return a[i++];
+				fail(PyExc_TypeError, "missing argument");
+			return good ? a[i++] : Py_None;
 		}
 
 		// a tensor's address (None: null; an int: itself)
 		template <bool CHECKED = true>
 		void * address_of(PyObject * o)
 		{
-			if (o == Py_None)
+			if (!good || o == Py_None)
 				return nullptr;
 			if (THPVariable_Check(o))
 			{
@@ -88,7 +90,7 @@ namespace
 		const at::Tensor * tensor()
 		{
 			PyObject * o = next();
-			if (!THPVariable_Check(o))
+			if (!good || !THPVariable_Check(o))
 			{
 				fail(PyExc_TypeError, "a tensor is expected");
 				return nullptr;
@@ -138,7 +140,13 @@ namespace
 
 		double number()
 		{
-			PyObject * o = next();
+			return number(next());
+		}
+
+		double number(PyObject * o)
+		{
+			if (!good)
+				return 0.0;
 			const double v = PyFloat_CheckExact(o) ? PyFloat_AS_DOUBLE(o) : PyFloat_AsDouble(o);
 			if (v == -1.0 && PyErr_Occurred())
 				good = false;
@@ -147,7 +155,8 @@ namespace
 
 		long long integer()
 		{
-			const long long v = PyLong_AsLongLong(next());
+			PyObject * o = next();
+			const long long v = good ? PyLong_AsLongLong(o) : 0;
 			if (v == -1 && PyErr_Occurred())
 				good = false;
 			return v;
@@ -155,7 +164,8 @@ namespace
 
 		int flag()
 		{
-			const int v = PyObject_IsTrue(next());
+			PyObject * o = next();
+			const int v = good ? PyObject_IsTrue(o) : 0;
 			if (v < 0)
 				good = false;
 			return v;
@@ -172,23 +182,10 @@ namespace
 			return p;
 		}
 
-		// torch's current stream unless one is given (an object with a cuda_stream, or the stream's address)
 		nnf_stream_t stream()
 		{
-			PyObject * o = next();
-			if (o == Py_None)
-				return (nnf_stream_t)c10::cuda::getCurrentCUDAStream().stream();
-			PyObject * v = PyObject_GetAttrString(o, "cuda_stream");
-			if (!v)
-			{
-				PyErr_Clear();
-				v = PyNumber_Long(o);
-			}
-			void * s = v ? PyLong_AsVoidPtr(v) : nullptr;
-			Py_XDECREF(v);
-			if (PyErr_Occurred())
-				good = false;
-			return (nnf_stream_t)s;
+			next();
+			return given_stream;
 		}
 
 		// the fields of one ctypes structure
@@ -251,9 +248,29 @@ namespace
 		}
 
 	private:
+		// torch's current stream unless one is given (an object with a cuda_stream, or the stream's address)
+		void read_stream(PyObject * o)
+		{
+			if (o == Py_None)
+			{
+				given_stream = (nnf_stream_t)c10::cuda::getCurrentCUDAStream().stream();
+				return;
+			}
+			PyObject * v = PyObject_GetAttrString(o, "cuda_stream");
+			if (!v && PyErr_ExceptionMatches(PyExc_AttributeError))
+			{
+				PyErr_Clear();
+				v = PyNumber_Long(o);
+			}
+			given_stream = v ? (nnf_stream_t)PyLong_AsVoidPtr(v) : nullptr;
+			Py_XDECREF(v);
+			good = !PyErr_Occurred();
+		}
+
 		PyObject * const * a;
 		Py_ssize_t n, i = 0;
 		bool good = true;
+		nnf_stream_t given_stream = nullptr;
 		std::vector<nnf_act> chain;
 	};
 
@@ -292,7 +309,8 @@ namespace
 	}
 
 	#define NNF_NATIVE(name) PyObject * name(PyObject *, PyObject * const * args, Py_ssize_t nargs)
-	#define NNF_READ arguments a(args, nargs)
+	#define NNF_READ arguments a(args, nargs, true)
+	#define NNF_READ_OBJECT arguments a(args, nargs, false)   // the layer objects run on torch's current stream
 
 	// (gamma, beta, mean, invsigma) or None
 	struct bn_arrays
@@ -684,10 +702,8 @@ namespace
 		NNF_READ;
 		std::vector<nnf_opt_part> parts;
 		PyObject * list = a.next();
-		const Py_ssize_t hint = PySequence_Check(list) ? PySequence_Size(list) : 0;
-		if (hint > 0)
-			parts.reserve((size_t)hint);
-		PyErr_Clear();
+		if (PyList_Check(list))
+			parts.reserve((size_t)PyList_GET_SIZE(list));
 		a.sequence(list, [&](PyObject * d)
 		{
 			if (!PyDict_Check(d))
@@ -714,13 +730,6 @@ namespace
 					a.fail(nullptr, nullptr);
 					return;
 				}
-			auto number = [&](PyObject * o)
-			{
-				const double x = PyFloat_CheckExact(o) ? PyFloat_AS_DOUBLE(o) : PyFloat_AsDouble(o);
-				if (x == -1.0 && PyErr_Occurred())
-					a.fail(nullptr, nullptr);
-				return (float)x;
-			};
 			auto address = [&](int k) { return v[k] ? a.address_of(v[k]) : nullptr; };
 			nnf_opt_part p = {};
 			p.data = static_cast<float *>(address(kData));
@@ -728,8 +737,8 @@ namespace
 			p.prev_upd = static_cast<float *>(address(kPrevUpd));
 			p.prev_upd2 = static_cast<float *>(address(kPrevUpd2));
 			p.update_accum = static_cast<double *>(address(kUpdateAccum));
-			p.learning_rate = number(v[kLearningRate]);
-			p.weight_decay = v[kWeightDecay] ? number(v[kWeightDecay]) : 0.0F;
+			p.learning_rate = (float)a.number(v[kLearningRate]);
+			p.weight_decay = v[kWeightDecay] ? (float)a.number(v[kWeightDecay]) : 0.0F;
 			if (!THPVariable_Check(v[kData]))
 				a.fail(PyExc_TypeError, "a chunk's data is a tensor");
 			if (!a.ok())
@@ -749,7 +758,7 @@ namespace
 
 	NNF_NATIVE(tester_forward)   // handle, output, data, inputs, entry_count
 	{
-		NNF_READ;
+		NNF_READ_OBJECT;
 		std::vector<void *> data, in;
 		void * h = a.handle(), * out = a.loose();
 		a.addresses<false>(data);
@@ -760,7 +769,7 @@ namespace
 
 	NNF_NATIVE(updater_forward)   // handle, output, data, inputs, working, fixed, per_entry, entry_count
 	{
-		NNF_READ;
+		NNF_READ_OBJECT;
 		std::vector<void *> data, in;
 		void * h = a.handle(), * out = a.loose();
 		a.addresses<false>(data);
@@ -773,7 +782,7 @@ namespace
 
 	NNF_NATIVE(object_forward)   // handle, outputs, data, inputs, working, fixed, per_entry, entry_count
 	{
-		NNF_READ;
+		NNF_READ_OBJECT;
 		std::vector<void *> out, data, in;
 		void * h = a.handle();
 		a.addresses<false>(out);
@@ -787,7 +796,7 @@ namespace
 
 	NNF_NATIVE(object_backward_data)   // handle, input_index, input_errors, output_errors, data, input_neurons, output_neurons, fixed, per_entry, add, entry_count
 	{
-		NNF_READ;
+		NNF_READ_OBJECT;
 		std::vector<void *> data, in;
 		void * h = a.handle();
 		const unsigned int index = (unsigned int)a.integer();
@@ -802,7 +811,7 @@ namespace
 
 	NNF_NATIVE(object_backward_weights)   // handle, gradient, input_neurons, output_errors, working, entry_count
 	{
-		NNF_READ;
+		NNF_READ_OBJECT;
 		std::vector<void *> gradient, in;
 		void * h = a.handle();
 		a.addresses<false>(gradient);
@@ -816,7 +825,7 @@ namespace
 
 	NNF_NATIVE(object_backward_data_and_weights)   // handle, input_errors, output_errors, gradient, data, input_neurons, output_neurons, working, fixed, add, entry_count
 	{
-		NNF_READ;
+		NNF_READ_OBJECT;
 		std::vector<void *> ie, gradient, data, in;
 		void * h = a.handle();
 		a.addresses<false>(ie);
