@@ -6,7 +6,9 @@
 // stream from c10 costs a few tens of nanoseconds.
 //
 // The interpreter's lock is released around every call into the library, as ctypes does: a launch can block while the
-// stream's queue is full, and other threads keep enqueueing on theirs.
+// stream's queue is full, and other threads keep enqueueing on theirs. torch's functions throw (no usable device, a tensor without
+// storage), and so may an allocation: every function of the module runs inside guarded(), which makes a Python error of it.
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -35,6 +37,13 @@ namespace
 	struct extents
 	{
 		int64_t n = 0, c = 0, h = 1, w = 1, hw = 1;
+	};
+
+	// a reference that is given back however the scope is left
+	struct owned
+	{
+		PyObject * object;
+		~owned() { Py_XDECREF(object); }
 	};
 
 	// Reads the positional arguments of one call in order. The first conversion that fails leaves its exception set, and
@@ -228,16 +237,14 @@ namespace
 		template <class F>
 		void sequence(PyObject * o, F f)
 		{
-			PyObject * s = good ? PySequence_Fast(o, "a sequence is expected") : nullptr;
-			if (!s)
+			const owned s{good ? PySequence_Fast(o, "a sequence is expected") : nullptr};
+			if (!s.object)
 			{
 				good = false;
 				return;
 			}
-			const Py_ssize_t count = PySequence_Fast_GET_SIZE(s);
-			for (Py_ssize_t k = 0; k < count && good; ++k)
-				f(PySequence_Fast_GET_ITEM(s, k));
-			Py_DECREF(s);
+			for (Py_ssize_t k = 0; k < PySequence_Fast_GET_SIZE(s.object) && good; ++k)
+				f(PySequence_Fast_GET_ITEM(s.object, k));
 		}
 
 		void fail(PyObject * type, const char * text)
@@ -274,16 +281,48 @@ namespace
 		std::vector<nnf_act> chain;
 	};
 
+	// runs f without the interpreter's lock, which is taken again if f throws, too
+	template <class F>
+	int without_lock(F f)
+	{
+		int status;
+		PyThreadState * const state = PyEval_SaveThread();
+		try
+		{
+			status = f();
+		}
+		catch (const std::exception&)
+		{
+			PyEval_RestoreThread(state);
+			throw;
+		}
+		PyEval_RestoreThread(state);
+		return status;
+	}
+
+	// (what is no std::exception is none of torch's or the library's: the unwinding of a thread that is being ended passes through)
+	template <PyObject * (*F)(PyObject *, PyObject * const *, Py_ssize_t)>
+	PyObject * guarded(PyObject * self, PyObject * const * args, Py_ssize_t nargs)
+	{
+		try
+		{
+			return F(self, args, nargs);
+		}
+		catch (const std::exception&)
+		{
+			PyErr_Clear();   // an exception is translated with none set
+			torch::translate_exception_to_python(std::current_exception());
+		}
+		return nullptr;
+	}
+
 	// calls the library without the interpreter's lock; a status raises NnfError with the library's text
 	template <class F>
 	PyObject * call(const arguments& a, F f)
 	{
 		if (!a.ok())
 			return nullptr;
-		int status;
-		Py_BEGIN_ALLOW_THREADS
-		status = f();
-		Py_END_ALLOW_THREADS
+		const int status = without_lock(f);
 		if (status == 0)
 			Py_RETURN_NONE;
 		PyObject * e = PyObject_CallFunction(g_error_type ? g_error_type : PyExc_RuntimeError, "is", status, nnf_last_error_string());
@@ -301,10 +340,8 @@ namespace
 	{
 		if (!a.ok())
 			return nullptr;
-		int status;
-		Py_BEGIN_ALLOW_THREADS
-		status = f();
-		Py_END_ALLOW_THREADS
+		const nnf_stream_t stream = (nnf_stream_t)c10::cuda::getCurrentCUDAStream().stream();
+		const int status = without_lock([&] { return f(stream); });
 		return PyLong_FromLong(status);
 	}
 
@@ -754,8 +791,6 @@ namespace
 	}
 
 	// ---- layer objects (host.py) ---------------------------------------------------------------------
-	nnf_stream_t current_stream() { return (nnf_stream_t)c10::cuda::getCurrentCUDAStream().stream(); }
-
 	NNF_NATIVE(tester_forward)   // handle, output, data, inputs, entry_count
 	{
 		NNF_READ_OBJECT;
@@ -764,7 +799,7 @@ namespace
 		a.addresses<false>(data);
 		a.addresses<false>(in);
 		const unsigned int n = (unsigned int)a.integer();
-		return call_object(a, [&] { return nnfh_tester_forward(h, current_stream(), out, data.data(), (int)data.size(), in.data(), (int)in.size(), n); });
+		return call_object(a, [&](nnf_stream_t s) { return nnfh_tester_forward(h, s, out, data.data(), (int)data.size(), in.data(), (int)in.size(), n); });
 	}
 
 	NNF_NATIVE(updater_forward)   // handle, output, data, inputs, working, fixed, per_entry, entry_count
@@ -777,7 +812,7 @@ namespace
 		size_t bytes;
 		void * ws = a.buffer<false>(bytes), * fixed = a.loose(), * per_entry = a.loose();
 		const unsigned int n = (unsigned int)a.integer();
-		return call_object(a, [&] { return nnfh_updater_forward(h, current_stream(), out, data.data(), (int)data.size(), in.data(), (int)in.size(), ws, bytes, fixed, per_entry, n); });
+		return call_object(a, [&](nnf_stream_t s) { return nnfh_updater_forward(h, s, out, data.data(), (int)data.size(), in.data(), (int)in.size(), ws, bytes, fixed, per_entry, n); });
 	}
 
 	NNF_NATIVE(object_forward)   // handle, outputs, data, inputs, working, fixed, per_entry, entry_count
@@ -791,7 +826,7 @@ namespace
 		size_t bytes;
 		void * ws = a.buffer<false>(bytes), * fixed = a.loose(), * per_entry = a.loose();
 		const unsigned int n = (unsigned int)a.integer();
-		return call_object(a, [&] { return nnfh_forward(h, current_stream(), out.data(), (int)out.size(), data.data(), (int)data.size(), in.data(), (int)in.size(), ws, bytes, fixed, per_entry, n); });
+		return call_object(a, [&](nnf_stream_t s) { return nnfh_forward(h, s, out.data(), (int)out.size(), data.data(), (int)data.size(), in.data(), (int)in.size(), ws, bytes, fixed, per_entry, n); });
 	}
 
 	NNF_NATIVE(object_backward_data)   // handle, input_index, input_errors, output_errors, data, input_neurons, output_neurons, fixed, per_entry, add, entry_count
@@ -806,7 +841,7 @@ namespace
 		void * on = a.loose(), * fixed = a.loose(), * per_entry = a.loose();
 		const int add = a.flag();
 		const unsigned int n = (unsigned int)a.integer();
-		return call_object(a, [&] { return nnfh_backward_data(h, current_stream(), index, ie, oe, data.data(), (int)data.size(), in.data(), (int)in.size(), on, fixed, per_entry, add, n); });
+		return call_object(a, [&](nnf_stream_t s) { return nnfh_backward_data(h, s, index, ie, oe, data.data(), (int)data.size(), in.data(), (int)in.size(), on, fixed, per_entry, add, n); });
 	}
 
 	NNF_NATIVE(object_backward_weights)   // handle, gradient, input_neurons, output_errors, working, entry_count
@@ -820,7 +855,7 @@ namespace
 		size_t bytes;
 		void * ws = a.buffer<false>(bytes);
 		const unsigned int n = (unsigned int)a.integer();
-		return call_object(a, [&] { return nnfh_backward_weights(h, current_stream(), gradient.data(), (int)gradient.size(), in.data(), (int)in.size(), oe, ws, bytes, n); });
+		return call_object(a, [&](nnf_stream_t s) { return nnfh_backward_weights(h, s, gradient.data(), (int)gradient.size(), in.data(), (int)in.size(), oe, ws, bytes, n); });
 	}
 
 	NNF_NATIVE(object_backward_data_and_weights)   // handle, input_errors, output_errors, gradient, data, input_neurons, output_neurons, working, fixed, add, entry_count
@@ -838,7 +873,7 @@ namespace
 		void * ws = a.buffer<false>(bytes), * fixed = a.loose();
 		const int add = a.flag();
 		const unsigned int n = (unsigned int)a.integer();
-		return call_object(a, [&] { return nnfh_backward_data_and_weights(h, current_stream(), ie.data(), (int)ie.size(), oe, gradient.data(), (int)gradient.size(),
+		return call_object(a, [&](nnf_stream_t s) { return nnfh_backward_data_and_weights(h, s, ie.data(), (int)ie.size(), oe, gradient.data(), (int)gradient.size(),
 			data.data(), (int)data.size(), in.data(), (int)in.size(), on, ws, bytes, fixed, add, n); });
 	}
 
@@ -849,8 +884,8 @@ namespace
 		Py_RETURN_NONE;
 	}
 
-	#define NNF_ENTRY(name) {#name, (PyCFunction)(void (*)(void))name, METH_FASTCALL, nullptr}
-	#define NNF_ENTRY_AS(name, ...) {name, (PyCFunction)(void (*)(void))__VA_ARGS__, METH_FASTCALL, nullptr}
+	#define NNF_ENTRY(name) {#name, (PyCFunction)(void (*)(void))guarded<name>, METH_FASTCALL, nullptr}
+	#define NNF_ENTRY_AS(name, ...) {name, (PyCFunction)(void (*)(void))guarded<__VA_ARGS__>, METH_FASTCALL, nullptr}
 	PyMethodDef g_methods[] = {
 		NNF_ENTRY(bn_infer_act), NNF_ENTRY(act_fwd), NNF_ENTRY(act_bwd), NNF_ENTRY(prelu_bwd_weights), NNF_ENTRY(add_fwd), NNF_ENTRY(add_bwd),
 		NNF_ENTRY(softmax_fwd), NNF_ENTRY(softmax_bwd), NNF_ENTRY(maxpool_fwd), NNF_ENTRY(maxpool_bwd), NNF_ENTRY(bn_add_relu_maxpool_fwd),

@@ -1,6 +1,13 @@
 """What the native call path does with arguments that it refuses and with the errors of what it calls: a Python error each, the one
-that names the cause, and no other. Nothing is launched, so no GPU is needed."""
+that names the cause, and no other. Nothing is launched, so no GPU is needed; where no device must be found, the calls are made in a
+process that sees none."""
+import os
+import subprocess
+import sys
+
 import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 torch = pytest.importorskip("torch")
 
@@ -52,3 +59,28 @@ def test_errors_of_the_stream_are_its_own(capi):
 def test_an_empty_step_is_no_error(capi):
     capi.apply_gradient([], stream=0)
     capi.apply_gradient((), stream=StreamAddress())
+
+
+def test_errors_of_torch_are_python_errors():
+    """No device, a tensor without storage: errors that a program can catch, from the functions and from the layer objects."""
+    code = """
+import torch
+import nnforge_b200.capi as capi, nnforge_b200.host as host
+x = torch.zeros(2, 4)
+sparse = x.to_sparse()
+tester, updater = host.Tester("TanH", 4, 1, 1), host.Updater("TanH", 4, 1, 1)
+for f in (lambda: capi.softmax_fwd(x, x),
+          lambda: capi.apply_gradient([]),
+          lambda: tester.enqueue_forward_propagation(x, [], [x], 2),
+          lambda: updater.enqueue_forward_propagation(x, [], [x], 2),
+          lambda: tester.enqueue_forward_propagation(sparse, [], [x], 2),
+          lambda: tester.enqueue_forward_propagation(x, [], [sparse], 2)):
+    try:
+        f()
+        print("none")
+    except RuntimeError:
+        print("caught")
+"""
+    p = subprocess.run([sys.executable, "-c", code], cwd=ROOT, env=dict(os.environ, CUDA_VISIBLE_DEVICES=""), capture_output=True, text=True, timeout=300)
+    assert p.returncode == 0, "exit status %d\n%s" % (p.returncode, p.stderr[-2000:])
+    assert p.stdout.split() == ["caught"] * 6
