@@ -720,7 +720,8 @@ namespace
 
 	// The fields of one chunk's dict. A step hands over hundreds of chunks, so the dict is walked once and its keys, which are interned
 	// strings in nearly every program, are told apart by address; other strings are compared. (Seven look-ups per chunk took
-	// 110 ns, three times the GPU's time for a network of small layers; the walk takes 60.)
+	// 110 ns, three times the GPU's time for a network of small layers; the walk takes 60.) Any other mapping, a subclass of dict among
+	// them, is asked through its own item and get.
 	enum part_field { kData, kGradient, kLearningRate, kUpdateAccum, kPrevUpd, kPrevUpd2, kWeightDecay, kPartFields };
 	struct part_keys
 	{
@@ -743,14 +744,22 @@ namespace
 			parts.reserve((size_t)PyList_GET_SIZE(list));
 		a.sequence(list, [&](PyObject * d)
 		{
-			if (!PyDict_Check(d))
-			{
-				a.fail(PyExc_TypeError, "a chunk is a dict");
-				return;
-			}
 			PyObject * v[kPartFields] = {};
+			owned asked[kPartFields] = {};
+			if (!PyDict_CheckExact(d))
+				for (int k = 0; k < kPartFields; ++k)
+				{
+					const bool required = k <= kLearningRate;
+					asked[k].object = required ? PyObject_GetItem(d, keys.key[k]) : PyObject_CallMethod(d, "get", "O", keys.key[k]);
+					if (!asked[k].object)
+					{
+						a.fail(nullptr, nullptr);
+						return;
+					}
+					v[k] = required || asked[k].object != Py_None ? asked[k].object : nullptr;
+				}
 			PyObject * key, * value;
-			for (Py_ssize_t pos = 0; PyDict_Next(d, &pos, &key, &value);)
+			for (Py_ssize_t pos = 0; PyDict_CheckExact(d) && PyDict_Next(d, &pos, &key, &value);)
 			{
 				int k = 0;
 				while (k < kPartFields && key != keys.key[k])

@@ -1,9 +1,11 @@
 """What the native call path does with arguments that it refuses and with the errors of what it calls: a Python error each, the one
 that names the cause, and no other. Nothing is launched, so no GPU is needed; where no device must be found, the calls are made in a
 process that sees none."""
+import collections
 import os
 import subprocess
 import sys
+import types
 
 import pytest
 
@@ -59,6 +61,21 @@ def test_errors_of_the_stream_are_its_own(capi):
 def test_an_empty_step_is_no_error(capi):
     capi.apply_gradient([], stream=0)
     capi.apply_gradient((), stream=StreamAddress())
+
+
+def test_a_chunk_is_any_mapping(capi):
+    """A chunk that is not a plain dict is asked through its own item and get: it gets as far as the check of its tensors."""
+    x = torch.zeros(4)                                # not on a device
+    full = {"data": x, "gradient": x, "learning_rate": 0.1, "weight_decay": 0.0}
+    for chunk in (types.MappingProxyType(full), collections.UserDict(full), collections.OrderedDict(full),
+                  collections.defaultdict(lambda: 0.1, data=x, gradient=x)):
+        with pytest.raises(AssertionError, match="contiguous CUDA tensors"):
+            capi.apply_gradient([chunk], stream=0)
+    for chunk in ({"data": x, "gradient": x}, types.MappingProxyType({"data": x, "gradient": x})):
+        with pytest.raises(KeyError, match="learning_rate"):
+            capi.apply_gradient([chunk], stream=0)
+    with pytest.raises(TypeError):
+        capi.apply_gradient([x.numpy], stream=0)
 
 
 def test_errors_of_torch_are_python_errors():

@@ -1,5 +1,8 @@
 """Sizes at the edges of the tiles and of the dispatch rules of single kernels, against the CPU checker: rows of every remainder
 modulo the access width, planes and tensors on either side of a rule's limit, buffers off their usual alignment."""
+import collections
+import types
+
 import numpy as np
 import pytest
 
@@ -122,6 +125,25 @@ def test_optimiser_step_chunk_counts_and_alignment(capi, oracle, kind, chunks):
                 assert_bits_equal(host(dp[name]), hp[name], "%s, chunk %d" % (name, k))
         # two orders of a double sum of at most 2050 terms of one sign: 2050 * 2^-53 < 3e-13 relative
         assert abs(float(host(dp["update_accum"])[0]) - accum) <= 1e-12 * accum
+
+
+def test_optimiser_step_chunks_of_any_mapping(capi):
+    """The same step from plain dicts and from other mappings, optional fields there, absent and None."""
+    def chunks(kind):
+        g = torch.Generator(device="cuda")
+        g.manual_seed(12)
+        make = lambda: torch.empty(70, device="cuda").normal_(generator=g)
+        return [kind(data=make(), gradient=make(), prev_upd=make(), prev_upd2=None, update_accum=torch.zeros(1, dtype=torch.float64, device="cuda"),
+                     learning_rate=0.1, weight_decay=0.01), kind(data=make(), gradient=make(), prev_upd=make(), learning_rate=0.1)]
+
+    results = []
+    for kind in (dict, collections.OrderedDict, collections.UserDict, lambda **kw: types.MappingProxyType(kw)):
+        parts = chunks(kind)
+        capi.apply_gradient(parts, capi.MOMENTUM_VANILLA, 0.9)
+        results.append([host(p[f]).copy() for p in parts for f in ("data", "gradient", "prev_upd")] + [host(parts[0]["update_accum"]).copy()])
+    for got in results[1:]:
+        for a, b in zip(results[0], got):
+            assert a.tobytes() == b.tobytes()
 
 
 # planes of whole float4s, planes of every remainder modulo 4, entries that do not divide by the CTAs, a tensor that ends inside a float4
