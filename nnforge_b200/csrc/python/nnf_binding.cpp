@@ -83,28 +83,23 @@ namespace
 				return good ? t.data_ptr() : nullptr;
 			}
 			if (CHECKED && PyLong_Check(o))
-			{
-				void * p = PyLong_AsVoidPtr(o);
-				if (p == nullptr && PyErr_Occurred())
-					good = false;
-				return p;
-			}
-			fail(PyExc_TypeError, "a tensor, an address or None is expected");
-			return nullptr;
+				return address_in(o);
+			// an object that answers as a tensor does (storage, a wrapper)
+			if (CHECKED && !(truth(member(o, "is_cuda")) && truth(result(o, "is_contiguous"))))
+				fail(PyExc_AssertionError, "tensors must be contiguous CUDA tensors");
+			const owned p{good ? result(o, "data_ptr") : nullptr};
+			return p.object && p.object != Py_None ? address_in(p.object) : nullptr;
 		}
 		float * ptr() { return static_cast<float *>(address_of(next())); }
 		void * raw() { return address_of(next()); }
 		void * loose() { return address_of<false>(next()); }
 
-		const at::Tensor * tensor()
+		// the number of elements of a tensor
+		int64_t numel(PyObject * o)
 		{
-			PyObject * o = next();
-			if (!good || !THPVariable_Check(o))
-			{
-				fail(PyExc_TypeError, "a tensor is expected");
-				return nullptr;
-			}
-			return &THPVariable_Unpack(o);
+			if (!good || THPVariable_Check(o))
+				return good ? THPVariable_Unpack(o).numel() : 0;
+			return count(result(o, "numel"));
 		}
 
 		// a tensor's address and its extents [n][c][h...][w]
@@ -112,27 +107,38 @@ namespace
 		{
 			PyObject * o = next();
 			float * p = static_cast<float *>(address_of(o));
-			if (!good || !THPVariable_Check(o))
-			{
-				fail(PyExc_TypeError, "a tensor is expected");
+			if (!good)
 				return nullptr;
-			}
-			const auto s = THPVariable_Unpack(o).sizes();
-			if (s.size() < 2 || (planes && s.size() != 4))
+			if (THPVariable_Check(o))
 			{
-				fail(PyExc_ValueError, planes ? "a tensor [n][c][h][w] is expected" : "a tensor [n][c][...] is expected");
-				return nullptr;
+				const auto s = THPVariable_Unpack(o).sizes();
+				set_extents(e, s.data(), s.size(), planes);
+				return p;
 			}
+			std::vector<int64_t> s;
+			const owned shape{member(o, "shape")};
+			sequence(shape.object, [&](PyObject * d) { s.push_back(PyLong_AsLongLong(d)); good = !PyErr_Occurred(); });
+			set_extents(e, s.data(), s.size(), planes);
+			return p;
+		}
+
+		void set_extents(extents& e, const int64_t * s, size_t dims, bool planes)
+		{
+			if (planes && dims != 4)
+				fail(PyExc_ValueError, "a tensor [n][c][h][w] is expected");
+			else if (dims < 2)
+				fail(PyExc_IndexError, "a tensor [n][c][...] is expected");
+			if (!good)
+				return;
 			e.n = s[0];
 			e.c = s[1];
-			for (size_t d = 2; d < s.size(); ++d)
+			for (size_t d = 2; d < dims; ++d)
 				e.hw *= s[d];
 			if (planes)
 			{
 				e.h = s[2];
 				e.w = s[3];
 			}
-			return p;
 		}
 
 		// a working buffer and its size in bytes (None: none of 0 bytes)
@@ -142,8 +148,12 @@ namespace
 			PyObject * o = next();
 			bytes = 0;
 			void * p = address_of<CHECKED>(o);
-			if (good && THPVariable_Check(o))
+			if (!good || o == Py_None)
+				return p;
+			if (THPVariable_Check(o))
 				bytes = THPVariable_Unpack(o).nbytes();
+			else if (!PyLong_Check(o))
+				bytes = size_t(count(result(o, "numel")) * count(result(o, "element_size")));
 			return p;
 		}
 
@@ -255,6 +265,45 @@ namespace
 		}
 
 	private:
+		void * address_in(PyObject * number)
+		{
+			void * p = PyLong_AsVoidPtr(number);
+			if (p == nullptr && PyErr_Occurred())
+				good = false;
+			return p;
+		}
+
+		PyObject * member(PyObject * o, const char * name)
+		{
+			PyObject * v = good ? PyObject_GetAttrString(o, name) : nullptr;
+			good = v != nullptr;
+			return v;
+		}
+
+		PyObject * result(PyObject * o, const char * name)
+		{
+			PyObject * v = good ? PyObject_CallMethod(o, name, nullptr) : nullptr;
+			good = v != nullptr;
+			return v;
+		}
+
+		// take the reference that they are given
+		bool truth(PyObject * o)
+		{
+			const owned v{o};
+			const int t = v.object ? PyObject_IsTrue(v.object) : 0;
+			good = good && t >= 0;
+			return t > 0;
+		}
+
+		long long count(PyObject * o)
+		{
+			const owned v{o};
+			const long long n = v.object ? PyLong_AsLongLong(v.object) : 0;
+			good = good && !(n == -1 && PyErr_Occurred());
+			return n;
+		}
+
 		// torch's current stream unless one is given (an object with a cuda_stream, or the stream's address)
 		void read_stream(PyObject * o)
 		{
@@ -423,25 +472,27 @@ namespace
 	NNF_NATIVE(add_fwd)   // y, inputs, alpha, stream
 	{
 		NNF_READ;
-		const at::Tensor * t = a.tensor();
-		float * y = a.ok() ? static_cast<float *>(a.address_of(args[0])) : nullptr;
+		PyObject * const t = a.next();
+		float * y = static_cast<float *>(a.address_of(t));
+		const int64_t count = a.numel(t);
 		std::vector<void *> in;
 		a.addresses<true>(in);
 		const float alpha = (float)a.number();
 		const nnf_stream_t s = a.stream();
-		return call(a, [&] { return nnf_add_fwd(s, y, (const float * const *)in.data(), (int)in.size(), alpha, t->numel()); });
+		return call(a, [&] { return nnf_add_fwd(s, y, (const float * const *)in.data(), (int)in.size(), alpha, count); });
 	}
 
 	NNF_NATIVE(add_bwd)   // dx, dy, alpha, add_to_destination, stream
 	{
 		NNF_READ;
 		float * dx = a.ptr();
-		const at::Tensor * t = a.tensor();
-		const float * dy = a.ok() ? static_cast<const float *>(a.address_of(args[1])) : nullptr;
+		PyObject * const t = a.next();
+		const float * dy = static_cast<const float *>(a.address_of(t));
+		const int64_t count = a.numel(t);
 		const float alpha = (float)a.number();
 		const int add = a.flag();
 		const nnf_stream_t s = a.stream();
-		return call(a, [&] { return nnf_add_bwd(s, dx, dy, alpha, t->numel(), add); });
+		return call(a, [&] { return nnf_add_bwd(s, dx, dy, alpha, count, add); });
 	}
 
 	NNF_NATIVE(softmax_fwd)   // y, x, stream
@@ -785,11 +836,9 @@ namespace
 			p.update_accum = static_cast<double *>(address(kUpdateAccum));
 			p.learning_rate = (float)a.number(v[kLearningRate]);
 			p.weight_decay = v[kWeightDecay] ? (float)a.number(v[kWeightDecay]) : 0.0F;
-			if (!THPVariable_Check(v[kData]))
-				a.fail(PyExc_TypeError, "a chunk's data is a tensor");
+			p.elem_count = a.numel(v[kData]);
 			if (!a.ok())
 				return;
-			p.elem_count = THPVariable_Unpack(v[kData]).numel();
 			parts.push_back(p);
 		});
 		const int type = (int)a.integer();

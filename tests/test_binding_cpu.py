@@ -78,6 +78,53 @@ def test_a_chunk_is_any_mapping(capi):
         capi.apply_gradient([x.numpy], stream=0)
 
 
+class Likeness:
+    """Answers what a tensor is asked, without being one."""
+
+    def __init__(self, *shape, cuda=True, address=0):
+        self.shape, self.is_cuda, self.address, self.asked = shape, cuda, address, 0
+
+    def is_contiguous(self):
+        return True
+
+    def data_ptr(self):
+        self.asked += 1
+        return self.address
+
+    def numel(self):
+        return 24
+
+    def element_size(self):
+        return 4
+
+
+def test_what_answers_as_a_tensor_is_taken_as_one(capi):
+    """The library itself refuses these for their null addresses, after every argument has been read."""
+    x, ws = Likeness(2, 3, 2, 2), Likeness(24)
+    for f in (lambda: capi.softmax_fwd(x, x, stream=0),
+              lambda: capi.add_fwd(x, [x, x], stream=0),
+              lambda: capi.add_bwd(x, x, stream=0),
+              lambda: capi.maxpool_fwd(x, x, x, capi.pool((2, 2), (2, 2)), stream=0),
+              lambda: capi.bn_train_fwd(x, x, x, x, x, x, 1e-5, workspace=ws, stream=0),
+              lambda: capi.apply_gradient([{"data": x, "gradient": x, "learning_rate": 0.1}], stream=0)):
+        x.asked = 0
+        with pytest.raises(capi.NnfError, match="null|has no data"):
+            f()
+        assert x.asked >= 2
+    with pytest.raises(AssertionError, match="contiguous CUDA tensors"):
+        capi.softmax_fwd(x, Likeness(2, 3, cuda=False), stream=0)
+    with pytest.raises(AttributeError):
+        capi.softmax_fwd(x, object(), stream=0)
+
+
+def test_extents_that_do_not_suffice(capi):
+    """As indexing and unpacking a shape report them."""
+    with pytest.raises(IndexError):
+        capi.softmax_fwd(0, Likeness(6), stream=0)
+    with pytest.raises(ValueError):
+        capi.maxpool_fwd(0, 0, Likeness(6, 4, 4), capi.pool((2, 2), (2, 2)), stream=0)
+
+
 def test_errors_of_torch_are_python_errors():
     """No device, a tensor without storage: errors that a program can catch, from the functions and from the layer objects."""
     code = """

@@ -146,6 +146,17 @@ def test_optimiser_step_chunks_of_any_mapping(capi):
             assert a.tobytes() == b.tobytes()
 
 
+def test_layer_objects_take_storages():
+    """The layer objects ask a buffer for its address alone."""
+    import nnforge_b200.host as host_layers
+    x = torch.empty(3, 4, 5, 5, device="cuda").normal_()
+    y, z = torch.empty_like(x), torch.empty_like(x)
+    tester = host_layers.Tester("TanH", 4, 5, 5)
+    tester.enqueue_forward_propagation(y, [], [x], 3)
+    tester.enqueue_forward_propagation(z.untyped_storage(), [], [x.untyped_storage()], 3)
+    assert_bits_equal(host(z), host(y), "storages")
+
+
 # planes of whole float4s, planes of every remainder modulo 4, entries that do not divide by the CTAs, a tensor that ends inside a float4
 TRAIN_SHAPES = [(8, 3, 8, 8), (9, 4, 9, 9), (5, 5, 9, 11), (16, 3, 13, 10), (33, 7, 27, 27), (4, 2, 56, 56), (17, 6, 19, 21), (64, 1, 8, 8), (12, 3, 55, 57),
                 (7, 8, 7, 7), (5, 9, 4, 4)]
