@@ -36,9 +36,6 @@ class NnfError(RuntimeError):
         self.status = status
 
 
-_native.set_error_type(NnfError)
-
-
 class Act(ct.Structure):
     _fields_ = [("kind", ct.c_int32), ("p0", ct.c_float), ("p1", ct.c_float), ("slope", ct.c_void_p)]
 
@@ -46,6 +43,9 @@ class Act(ct.Structure):
 class Pool(ct.Structure):
     _fields_ = [("win_w", ct.c_int32), ("win_h", ct.c_int32), ("stride_w", ct.c_int32), ("stride_h", ct.c_int32),
                 ("round_up_w", ct.c_int32), ("round_up_h", ct.c_int32), ("is_min", ct.c_int32)]
+
+
+_native.set_types(NnfError, Act, Pool)
 
 
 _P, _I64, _F, _I, _D, _SZ = ct.c_void_p, ct.c_int64, ct.c_float, ct.c_int, ct.c_double, ct.c_size_t

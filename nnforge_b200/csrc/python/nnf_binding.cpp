@@ -33,6 +33,9 @@ extern "C"
 namespace
 {
 	PyObject * g_error_type = nullptr;   // capi.NnfError
+	PyObject * g_act_type = nullptr, * g_pool_type = nullptr;   // capi.Act, capi.Pool
+	PyObject * ctypes_type(const nnf_act&) { return g_act_type; }
+	PyObject * ctypes_type(const nnf_pool&) { return g_pool_type; }
 
 	struct extents
 	{
@@ -207,12 +210,18 @@ namespace
 			return given_stream;
 		}
 
-		// the fields of one ctypes structure
+		// the fields of one ctypes structure: an object of the type itself, as other bytes of its size may hold any address
 		template <class T>
 		void structure(PyObject * o, T& out)
 		{
+			if (!good)
+				return;
+			PyObject * const type = ctypes_type(out);
+			const int is = type ? PyObject_IsInstance(o, type) : 0;
+			if (is == 0)
+				fail(PyExc_TypeError, "an activation (Act) or a pooling geometry (Pool) is expected");
 			Py_buffer b;
-			if (!good || PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) != 0)
+			if (is <= 0 || PyObject_GetBuffer(o, &b, PyBUF_SIMPLE) != 0)
 			{
 				good = false;
 				return;
@@ -935,10 +944,14 @@ namespace
 			data.data(), (int)data.size(), in.data(), (int)in.size(), on, ws, bytes, fixed, add, n); });
 	}
 
-	PyObject * set_error_type(PyObject *, PyObject * type)
+	PyObject * set_types(PyObject *, PyObject * types)   // (NnfError, Act, Pool)
 	{
-		Py_INCREF(type);
-		Py_XSETREF(g_error_type, type);
+		PyObject * error, * act, * pool;
+		if (!PyArg_ParseTuple(types, "OOO", &error, &act, &pool))
+			return nullptr;
+		Py_XSETREF(g_error_type, Py_NewRef(error));
+		Py_XSETREF(g_act_type, Py_NewRef(act));
+		Py_XSETREF(g_pool_type, Py_NewRef(pool));
 		Py_RETURN_NONE;
 	}
 
@@ -955,7 +968,7 @@ namespace
 		NNF_ENTRY(softmax_nll_fwd), NNF_ENTRY_AS("softmax_nll_bwd", loss_bwd<nnf_softmax_nll_bwd>), NNF_ENTRY(apply_gradient),
 		NNF_ENTRY(tester_forward), NNF_ENTRY(updater_forward), NNF_ENTRY(object_forward), NNF_ENTRY(object_backward_data),
 		NNF_ENTRY(object_backward_weights), NNF_ENTRY(object_backward_data_and_weights),
-		{"set_error_type", set_error_type, METH_O, nullptr},
+		{"set_types", set_types, METH_VARARGS, nullptr},
 		{nullptr, nullptr, 0, nullptr}};
 
 	PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_native", "Call path between Python and the C ABI.", -1, g_methods, nullptr, nullptr, nullptr, nullptr};

@@ -117,6 +117,20 @@ def test_what_answers_as_a_tensor_is_taken_as_one(capi):
         capi.softmax_fwd(x, object(), stream=0)
 
 
+def test_structures_are_of_their_own_type(capi):
+    """24 bytes of anything else are no activation: they would hold an address that nobody gave."""
+    import ctypes
+    x = Likeness(2, 3, 2, 2)
+    for wrong in (bytes(ctypes.sizeof(capi.Act)), capi.pool((2, 2), (2, 2)), "tanh"):
+        with pytest.raises(TypeError):
+            capi.act_fwd(x, x, wrong, stream=0)
+        with pytest.raises(TypeError):
+            capi.bn_infer_act(x, x, acts=[wrong], stream=0)
+    for wrong in (bytes(ctypes.sizeof(capi.Pool)), capi.relu()):
+        with pytest.raises(TypeError):
+            capi.maxpool_fwd(x, x, x, wrong, stream=0)
+
+
 def test_extents_that_do_not_suffice(capi):
     """As indexing and unpacking a shape report them."""
     with pytest.raises(IndexError):
