@@ -302,54 +302,30 @@ namespace nnf
 
 		// Gradient reaching input element (iy, ix) of a plane whose pooled gradients / argmax start at
 		// dyp / idx; abs_off is the element's absolute offset as the argmax stores it. Windows are visited in
-		// ascending output index. WW/WH/SW/SH > 0: compile-time window and stride (divisions become shifts
-		// and the candidate loops unroll to ceil(WH/SH) x ceil(WW/SW) predicated steps).
-		template <int WW, int WH, int SW, int SH>
+		// ascending output index.
 		__device__ __forceinline__ float gather_element(const pool_geom& g, const float * dyp, const uint32_t * idx, uint32_t iy, uint32_t ix, uint32_t abs_off, float seed)
 		{
-			const uint32_t win_w = WW ? WW : g.win_w, win_h = WH ? WH : g.win_h;
-			const uint32_t oy_lo = iy < win_h ? 0u : (SH ? (iy - win_h) / (SH ? SH : 1) : g.d_sh.div(iy - win_h)) + 1u;
-			uint32_t oy_hi = SH ? iy / (SH ? SH : 1) : g.d_sh.div(iy);
+			const uint32_t win_w = g.win_w, win_h = g.win_h;
+			const uint32_t oy_lo = iy < win_h ? 0u : g.d_sh.div(iy - win_h) + 1u;
+			uint32_t oy_hi = g.d_sh.div(iy);
 			if (oy_hi > g.oh - 1)
 				oy_hi = g.oh - 1;
-			const uint32_t ox_lo = ix < win_w ? 0u : (SW ? (ix - win_w) / (SW ? SW : 1) : g.d_sw.div(ix - win_w)) + 1u;
-			uint32_t ox_hi = SW ? ix / (SW ? SW : 1) : g.d_sw.div(ix);
+			const uint32_t ox_lo = ix < win_w ? 0u : g.d_sw.div(ix - win_w) + 1u;
+			uint32_t ox_hi = g.d_sw.div(ix);
 			if (ox_hi > g.ow - 1)
 				ox_hi = g.ow - 1;
 			float sum = seed;
-			if (WW && WH && SW && SH)
-			{
-				constexpr int NY = (WH + (SH ? SH : 1) - 1) / (SH ? SH : 1), NX = (WW + (SW ? SW : 1) - 1) / (SW ? SW : 1);
-				#pragma unroll
-				for (int a = 0; a < NY; ++a)
+			for (uint32_t oy = oy_lo; oy <= oy_hi; ++oy)
+				for (uint32_t ox = ox_lo; ox <= ox_hi; ++ox)
 				{
-					#pragma unroll
-					for (int b = 0; b < NX; ++b)
-					{
-						const uint32_t oy = oy_lo + a, ox = ox_lo + b;
-						if (oy <= oy_hi && ox <= ox_hi)
-						{
-							const uint32_t o = oy * g.ow + ox;
-							if (idx[o] == abs_off)
-								sum = __fadd_rn(sum, dyp[o]);
-						}
-					}
+					const uint32_t o = oy * g.ow + ox;
+					if (idx[o] == abs_off)
+						sum = __fadd_rn(sum, dyp[o]);
 				}
-			}
-			else
-			{
-				for (uint32_t oy = oy_lo; oy <= oy_hi; ++oy)
-					for (uint32_t ox = ox_lo; ox <= ox_hi; ++ox)
-					{
-						const uint32_t o = oy * g.ow + ox;
-						if (idx[o] == abs_off)
-							sum = __fadd_rn(sum, dyp[o]);
-					}
-			}
 			return sum;
 		}
 
-		// 3x3 windows, stride 2, four consecutive elements of one input row (W % 4 == 0). The four elements
+		// 3x3 windows, stride 2, four consecutive elements of one input row. The four elements
 		// share their candidate windows: rows {oy_lo..oy_hi} (at most two) and columns {k-1, k, k+1} with
 		// k = ix0/2, so a vector needs 6 (argmax, gradient) pairs instead of 16. Within a row the columns
 		// are visited in ascending order, rows in ascending order: ascending output index per element.
@@ -392,7 +368,8 @@ namespace nnf
 			}
 		}
 
-		template <bool FUSED, int WW, int WH, int SW, int SH, bool ROW4 = false>
+		// ROW4: 3x3 windows at stride 2 behind the fused layers, rows in chunks of four elements; otherwise any window, element by element
+		template <bool FUSED, bool ROW4>
 		__global__ void __launch_bounds__(kThreads) pool_bwd_staged_kernel(const pool_bwd_params p)
 		{
 			pdl_begin();
@@ -432,7 +409,7 @@ namespace nnf
 					const uint32_t rem = e - lp * g.hw;
 					const uint32_t iy = g.d_w.div(rem);
 					const uint32_t ix = rem - iy * g.w;
-					const float dz = gather_element<WW, WH, SW, SH>(g, s_dy + lp * g.ohw, s_idx + lp * g.ohw, iy, ix, (uint32_t)(base + e), seed);
+					const float dz = gather_element(g, s_dy + lp * g.ohw, s_idx + lp * g.ohw, iy, ix, (uint32_t)(base + e), seed);
 					if (FUSED)
 					{
 						// ReLU gate from the sign bit of z (negative pre-activations were multiplied by a
@@ -579,7 +556,7 @@ namespace nnf
 				const uint32_t iy = g.d_w.div(rem);
 				const uint32_t ix = rem - iy * g.w;
 				const float seed = (!FUSED && p.add) ? p.dx[e] : 0.0F;
-				const float dz = gather_element<0, 0, 0, 0>(g, p.dpooled + plane * g.ohw, p.argmax + plane * g.ohw, iy, ix, (uint32_t)e, seed);
+				const float dz = gather_element(g, p.dpooled + plane * g.ohw, p.argmax + plane * g.ohw, iy, ix, (uint32_t)e, seed);
 				if (FUSED)
 				{
 					const float ds = (__float_as_uint(p.z[e]) >> 31) ? __fmul_rn(dz, p.slope) : dz;
@@ -786,26 +763,12 @@ namespace nnf
 			per_sm = per_sm < 1 ? 1 : (per_sm > 8 ? 8 : per_sm);
 			const int64_t cap = int64_t(sm_count()) * per_sm * pool_waves();
 			const int grid = (int)(ngroups < cap ? ngroups : cap);
-						cudaError_t e = cudaSuccess;
-#define NNF_POOL_BWD(FUSED, WW, WH, SW, SH) \
-			{ \
-				e = cudaFuncSetAttribute(pool_bwd_staged_kernel<FUSED, WW, WH, SW, SH>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit()); \
-				if (e == cudaSuccess) \
-					launch(pool_bwd_staged_kernel<FUSED, WW, WH, SW, SH>, grid, kThreads, smem, s, p); \
-			}
 			p.d_cpr = fastdiv((p.g.w + 3) / 4);
 			p.d_hcpr = fastdiv(p.g.h * ((p.g.w + 3) / 4));
-			if (ragged_fast)
-			{
-				e = cudaFuncSetAttribute(pool_bwd_staged_kernel<true, 3, 3, 2, 2, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit());
-				if (e == cudaSuccess)
-					launch(pool_bwd_staged_kernel<true, 3, 3, 2, 2, true>, grid, kThreads, smem, s, p);
-			}
-			else if (fused)
-				NNF_POOL_BWD(true, 0, 0, 0, 0)
-			else
-				NNF_POOL_BWD(false, 0, 0, 0, 0)
-#undef NNF_POOL_BWD
+			const auto kernel = ragged_fast ? pool_bwd_staged_kernel<true, true> : fused ? pool_bwd_staged_kernel<true, false> : pool_bwd_staged_kernel<false, false>;
+			const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit());
+			if (e == cudaSuccess)
+				launch(kernel, grid, kThreads, smem, s, p);
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "cudaFuncSetAttribute: %s", cudaGetErrorString(e));
 			return check_launch("pool_bwd_staged_kernel");
