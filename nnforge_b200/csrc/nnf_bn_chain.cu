@@ -1393,11 +1393,14 @@ namespace nnf
 			return true;
 		}
 
-		size_t stream_workspace_needed(const stream_params& p)
+		// Workspace of the kernel above, as launch_stream lays it out: the report, two constants per channel, four words per
+		// statistics item and channel.
+		size_t stream_workspace(size_t c, size_t items)
 		{
-			return sizeof(launch_report) + size_t(p.c) * sizeof(uint32_t) + 16 + size_t(p.c) * 2 * sizeof(float4)
-				+ size_t(p.c) * p.ss * 4 * sizeof(unsigned long long);
+			return sizeof(launch_report) + c * (2 + items * 4) * sizeof(unsigned long long);
 		}
+
+		size_t stream_workspace_needed(const stream_params& p) { return stream_workspace(p.c, p.ss); }
 
 		// The grouped kernel's plan: items are channel groups. Returns false where the shape does not suit it (planes
 		// of whole float4s take the kernel above; runs shorter than 16 vectors or longer than 256 the separate kernels).
@@ -1509,7 +1512,7 @@ namespace nnf
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "%s: cudaFuncSetAttribute: %s", what, cudaGetErrorString(e));
 			// the words too: a launch that is replayed from a graph carries the tag it was captured with
-			e = cudaMemsetAsync(workspace, 0, sizeof(launch_report) + size_t(p.c) * (2 + size_t(p.ss) * 4) * sizeof(unsigned long long), s);
+			e = cudaMemsetAsync(workspace, 0, stream_workspace_needed(p), s);
 			if (e != cudaSuccess)
 				return set_error(NNF_ERR_CUDA, "%s: cudaMemsetAsync: %s", what, cudaGetErrorString(e));
 			launch(kernel, p.total, kChainThreads, smem, s, p);
@@ -1524,8 +1527,7 @@ namespace nnf
 		(void)n; (void)hw;
 		const size_t grouped = sizeof(launch_report) + (size_t(c) + 2) / 2 * 2 * sizeof(uint32_t) + size_t(c) * kChainMaxSplit * 3 * sizeof(double)
 			+ 16 + size_t(c) * 8 * sizeof(float);
-		const size_t stream = sizeof(launch_report) + size_t(c) * sizeof(uint32_t) + 16 + size_t(c) * 2 * sizeof(float4)
-			+ size_t(c) * kChainMaxSplit * 4 * sizeof(unsigned long long);
+		const size_t stream = stream_workspace(size_t(c), kChainMaxSplit);
 		return grouped > stream ? grouped : stream;
 	}
 

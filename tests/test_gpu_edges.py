@@ -220,6 +220,29 @@ def test_training_batch_norm_in_a_cluster(capi, tuning, shape, acts, ctas):
             assert capi.parse_report(report)["status"] == 0
 
 
+@pytest.mark.parametrize("shape", [(49200, 4, 4, 4), (3000, 8, 3, 3), (600, 8, 28, 28)])
+def test_training_batch_norm_stays_in_its_workspace(capi, tuning, shape):
+    """As many items per channel as a plan makes (64 at most), with a workspace of exactly the size that is asked for: what follows it
+    stays as it was."""
+    tuning("chain_cluster", 99)
+    tuning("chain_s_kb", 1)
+    n, c, h, w = shape
+    x, dy = (torch.empty(shape, device="cuda").normal_() for _ in range(2))
+    gamma, beta = torch.ones(c, device="cuda"), torch.zeros(c, device="cuda")
+    y, dx = torch.empty_like(x), torch.empty_like(x)
+    saved, sums, bsums = (torch.empty(k * c, device="cuda") for k in (2, 2, 3))
+    need = capi.bn_train_workspace_bytes(n, c, h * w)
+    room = torch.full((need + 65536,), 0xa5, dtype=torch.uint8, device="cuda")
+    ws = room[:need]
+    capi.bn_train_fwd(y, saved, sums, x, gamma, beta, 1e-5, [], workspace=ws)
+    capi.bn_train_bwd(dx, bsums, dy, x, gamma, beta, saved, [], workspace=ws)
+    assert bool((room[need:] == 0xa5).all())
+    xd = x.double().requires_grad_(True)
+    want = torch.nn.functional.batch_norm(xd, None, None, training=True, eps=1e-5)
+    want.backward(dy.double())
+    assert float((y - want.detach()).norm() / want.detach().norm()) <= 1e-6 and float((dx - xd.grad).norm() / xd.grad.norm()) <= 3e-6
+
+
 def test_training_batch_norm_in_a_cluster_beyond_2_to_30_elements(capi):
     """Ragged planes of a tensor whose bytes do not fit 32 bits: the channel whose first elements are 2^30 elements from the tensor's end,
     those next to it and those at both ends, against float64 arithmetic (tolerances as above)."""
