@@ -202,7 +202,9 @@ NNF_API int nnf_maxpool_bwd(nnf_stream_t stream, float * dx, const float * dy, c
 	int64_t n, int64_t c, int64_t h, int64_t w, const nnf_pool * pool, int add_to_destination);
 
 /* ResNet block tail in one pass: z = relu(((0 + bn(x)) + residual) * 1, slope), pooled = maxpool(z).
- * z is written because later layers and the backward pass need it. gamma == NULL skips the batch norm. */
+ * z is written because later layers and the backward pass need it. gamma == NULL skips the batch norm. z may be x or residual
+ * itself. A plane must fit a CTA's shared memory (51200 values) - NNF_ERR_UNSUPPORTED otherwise -, except for 3x3 and 2x2
+ * windows at stride 2 with z in a buffer of its own, which take planes of any size. */
 NNF_API int nnf_bn_add_relu_maxpool_fwd(nnf_stream_t stream, float * z, float * pooled, uint32_t * argmax,
 	const float * x, const float * residual,
 	const float * gamma, const float * beta, const float * mean, const float * invsigma,

@@ -98,6 +98,30 @@ def test_max_subsampling_rows_and_plane_groups(capi, oracle, tuning, shape, win,
         assert_bits_equal(host(dx), dx_want, "dx")
 
 
+@pytest.mark.parametrize("win", [2, 3])
+def test_fused_max_subsampling_of_planes_beyond_shared_memory(capi, oracle, win):
+    """Planes of 231 KB: taken at stride 2 where z is written to a buffer of its own, refused over x, over the residual and at other
+    strides, as the header says."""
+    g = synth.rng(3, salt=win)
+    shape = (1, 2, 241, 246)
+    x, r = synth.normal(g, shape), synth.normal(g, shape)
+    bn = synth.bn_params(g, 2)
+    bnd, xd, rd = [dev(a) for a in bn], dev(x), dev(r)
+    z_want = oracle.relu_fwd(oracle.add_fwd([oracle.bn_infer(x, *bn), r], 1.0), 0.0)
+    want, want_idx = oracle.maxpool_fwd(z_want, (win, win), (2, 2), (False, False))
+    p = capi.pool((win, win), (2, 2))
+    z, y, idx = torch.empty(shape, device="cuda"), torch.empty(want.shape, device="cuda"), torch.zeros(want.shape, dtype=torch.int32, device="cuda")
+    capi.bn_add_relu_maxpool_fwd(z, y, idx, xd, rd, bnd, 0.0, p)
+    assert_bits_equal(host(z), z_want, "z")
+    assert_bits_equal(host(y), want, "pooled")
+    assert_bits_equal(host(idx).view(np.uint32), want_idx, "argmax")
+    for over in (xd, rd):
+        with pytest.raises(capi.NnfError, match="does not fit"):
+            capi.bn_add_relu_maxpool_fwd(over, y, idx, xd, rd, bnd, 0.0, p)
+    with pytest.raises(capi.NnfError, match="does not fit"):
+        capi.bn_add_relu_maxpool_fwd(z, y, idx, xd, rd, bnd, 0.0, capi.pool((win, win), (1, 1)))
+
+
 @pytest.mark.parametrize("kind", ["none", "vanilla", "nesterov", "adam"])
 @pytest.mark.parametrize("chunks", [1, 48, 49, 160, 161, 500, 501])
 def test_optimiser_step_chunk_counts_and_alignment(capi, oracle, kind, chunks):
