@@ -40,6 +40,32 @@ def host(t):
     return t.cpu().numpy()
 
 
+def launches(call):
+    """What the call puts on its stream, from a capture of it: the CTAs per cluster of each kernel (1: no cluster), "memset", or "other".
+    The call itself is not run."""
+    import ctypes as ct
+    cuda = ct.CDLL("libcuda.so.1")
+
+    def ok(status):
+        assert status == 0, "status %d" % status
+
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    handle, count = ct.c_void_p(graph.raw_cuda_graph()), ct.c_size_t(0)
+    ok(cuda.cuGraphGetNodes(handle, None, ct.byref(count)))
+    nodes = (ct.c_void_p * count.value)()
+    ok(cuda.cuGraphGetNodes(handle, nodes, ct.byref(count)))
+    out = []
+    for node in nodes:
+        kind, value = ct.c_int(), (ct.c_uint32 * 16)()
+        ok(cuda.cuGraphNodeGetType(ct.c_void_p(node), ct.byref(kind)))
+        if kind.value == 0:         # CU_GRAPH_NODE_TYPE_KERNEL, CU_LAUNCH_ATTRIBUTE_CLUSTER_DIMENSION
+            ok(cuda.cuGraphKernelNodeGetAttribute(ct.c_void_p(node), 4, value))
+        out.append({0: max(1, value[0]), 2: "memset"}.get(kind.value, "other"))
+    return out
+
+
 # widths of every remainder modulo 4 up to more columns than a warp serves; heights of one pair of rows up to several, odd and even
 ROW_SHAPES = [(2, 3, 3, 3), (1, 5, 4, 4), (3, 2, 5, 5), (2, 2, 6, 6), (2, 3, 7, 7), (1, 3, 8, 9), (2, 1, 9, 34), (1, 2, 3, 131), (1, 1, 10, 130), (1, 1, 11, 128),
               (5, 7, 13, 13), (2, 3, 33, 35), (9, 16, 14, 14)]
@@ -221,18 +247,31 @@ def test_training_batch_norm_in_a_cluster(capi, tuning, shape, acts, ctas):
     ws = torch.empty(capi.bn_train_workspace_bytes(n, c, h * w), dtype=torch.uint8, device="cuda")
     close = lambda a, b, tol: float((a.double() - b.detach()).norm()) <= tol * float(b.detach().norm()) + 1e-12
     room = 4e-6 * (n * h * w) ** 0.5
+
+    def in_cluster(backward, got):
+        # 220 KB of a channel's entries are the most that a CTA takes; where they do not fit, any other form is right
+        row = (h * w // 4 if h * w % 4 == 0 else (h * w + 6) // 4) * 16 * (2 if backward else 1)
+        if -(-n // (ctas or 8)) * row <= 220 * 1024:
+            assert len(got) == 1 and got[0] in ([ctas] if ctas else [1, 2, 4, 8]), got
+        else:
+            assert len(got) > 1, got
+
     for in_place in (False, True):
         y = x.clone() if in_place else torch.full_like(x, float("nan"))
         saved, sums, bsums = (torch.full((k * c,), float("nan"), device="cuda") for k in (2, 2, 3))
-        capi.bn_train_fwd(y, saved, sums, y if in_place else x, gamma, beta, 1e-5, chain, workspace=ws)
+        forward = lambda: capi.bn_train_fwd(y, saved, sums, y if in_place else x, gamma, beta, 1e-5, chain, workspace=ws)
+        in_cluster(False, launches(forward))
+        forward()
         assert close(y, want, 1e-6)
         assert close(saved[:c], mu, 1e-6) and close(saved[c:], inv, 1e-6)
         assert close(sums[:c], xd.sum((0, 2, 3)), 2e-6) and close(sums[c:], (xd ** 2).sum((0, 2, 3)), 2e-6)
         grads = [torch.full((c,), 0.25, device="cuda") for _ in range(5)]
         dx = dy.clone() if in_place else torch.full_like(x, float("nan"))
-        capi.bn_train_bwd(dx, bsums, dx if in_place else dy, x, gamma, beta, saved, chain, grad_gamma=grads[0], grad_beta=grads[1], grad_mean=grads[2],
-                          grad_invsigma=grads[3], grad_slope=grads[4] if acts == "prelu_elu" else None, mean=mean, invsigma=invsigma, entry_count=float(n),
-                          workspace=ws)
+        backward = lambda: capi.bn_train_bwd(dx, bsums, dx if in_place else dy, x, gamma, beta, saved, chain, grad_gamma=grads[0], grad_beta=grads[1],
+                                             grad_mean=grads[2], grad_invsigma=grads[3], grad_slope=grads[4] if acts == "prelu_elu" else None, mean=mean,
+                                             invsigma=invsigma, entry_count=float(n), workspace=ws)
+        in_cluster(True, launches(backward))
+        backward()
         assert close(dx, xd.grad, 3e-6)
         for got, gradient in ((grads[0], ga), (grads[1], be)) + (((grads[4], sl),) if acts == "prelu_elu" else ()):
             assert float((got.double() - 0.25 - gradient.grad).abs().max()) <= room
@@ -242,6 +281,50 @@ def test_training_batch_norm_in_a_cluster(capi, tuning, shape, acts, ctas):
             capi.read_report(report, ws)
             torch.cuda.synchronize()
             assert capi.parse_report(report)["status"] == 0
+
+
+@pytest.mark.parametrize("shape", [(8, 5, 13, 13), (8, 8, 12, 12)])
+@pytest.mark.parametrize("mean", [0.0, 500.0])
+@pytest.mark.parametrize("outlier", [0.0, 20.0])
+def test_training_batch_norm_in_a_cluster_far_from_zero(capi, shape, mean, outlier):
+    """Means of 500 standard deviations and a first element, the one the sums are taken around, 20 of them from the mean. A thread adds
+    the squares of at most 4 elements in float, each good to 2^-24 of (1 + outlier)^2, before sums are taken in double: half of that,
+    relative, is the inverse deviation's error. y also carries the rounding of the mean times the scale, mean * 2^-23."""
+    n, c, h, w = shape
+    g = torch.Generator(device="cuda")
+    g.manual_seed(int(mean + outlier))
+    x = torch.empty(shape, device="cuda").normal_(mean, 1.0, generator=g)
+    x[0, :, 0, 0] = mean + outlier
+    gamma, beta = torch.ones(c, device="cuda"), torch.zeros(c, device="cuda")
+    y, saved, sums = torch.empty_like(x), torch.empty(2 * c, device="cuda"), torch.empty(2 * c, device="cuda")
+    ws = torch.empty(capi.bn_train_workspace_bytes(n, c, h * w), dtype=torch.uint8, device="cuda")
+    forward = lambda: capi.bn_train_fwd(y, saved, sums, x, gamma, beta, 1e-5, [], workspace=ws)
+    got = launches(forward)
+    assert len(got) == 1 and got[0] != "memset"
+    forward()
+    xd = x.double()
+    var, mu = torch.var_mean(xd, dim=(0, 2, 3), correction=0)
+    inv = (var + 1e-5).rsqrt()
+    tol = 4 * (1 + outlier) ** 2 * 2.0 ** -25 + 2.0 ** -23
+    assert float((saved[:c] - mu).abs().max()) <= 2.0 ** -23 * mean + (1 + outlier) * 2.0 ** -22
+    assert float(((saved[c:] - inv) / inv).abs().max()) <= tol
+    want = (xd - mu.view(1, -1, 1, 1)) * inv.view(1, -1, 1, 1)
+    assert float((y - want).norm() / want.norm()) <= tol + (1 + mean) * 2.0 ** -23
+
+
+@pytest.mark.parametrize("shape,clusters", [((3, 5, 3, 5), False), ((3, 5, 5, 5), True), ((3, 5, 2, 6), False), ((3, 5, 4, 4), True)])
+def test_smallest_planes_of_the_cluster_form(capi, shape, clusters):
+    """Planes on either side of the smallest that a cluster takes, ragged and of whole float4s."""
+    n, c, h, w = shape
+    x = torch.empty(shape, device="cuda").normal_()
+    gamma, beta = torch.ones(c, device="cuda"), torch.zeros(c, device="cuda")
+    y, saved, sums = torch.empty_like(x), torch.empty(2 * c, device="cuda"), torch.empty(2 * c, device="cuda")
+    ws = torch.empty(capi.bn_train_workspace_bytes(n, c, h * w), dtype=torch.uint8, device="cuda")
+    forward = lambda: capi.bn_train_fwd(y, saved, sums, x, gamma, beta, 1e-5, [], workspace=ws)
+    assert (len(launches(forward)) == 1) == clusters
+    forward()
+    want = torch.nn.functional.batch_norm(x.double(), None, None, training=True, eps=1e-5)
+    assert float((y - want).norm() / want.norm()) <= 1e-6
 
 
 @pytest.mark.parametrize("shape", [(49200, 4, 4, 4), (3000, 8, 3, 3), (600, 8, 28, 28)])
