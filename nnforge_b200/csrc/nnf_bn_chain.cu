@@ -1613,7 +1613,7 @@ namespace nnf
 				return 2;
 			if constexpr (!PEER)
 			{
-				const int st = cluster_train_fwd(stream, y, saved, sums, x, gamma, beta, eps, chain, n, c, hw, workspace, kClusterSliceForward);
+				const int st = cluster_train_fwd(stream, y, saved, sums, x, gamma, beta, eps, chain, n, c, hw, workspace, kClusterSlice);
 				if (st != -1)
 					return st;
 			}
@@ -1678,7 +1678,7 @@ namespace nnf
 			if constexpr (!PEER)
 			{
 				const int st = cluster_train_bwd(stream, dx, bsums, dy, x, gamma, beta, saved, chain, grad_gamma, grad_beta, grad_mean, grad_invsigma, grad_slope,
-					mean, invsigma, entry_count, n, c, hw, workspace, kClusterSliceBackward);
+					mean, invsigma, entry_count, n, c, hw, workspace, kClusterSlice);
 				if (st != -1)
 					return st;
 			}

@@ -490,11 +490,13 @@ namespace nnf
 	// Training batch norm of channels that fit a cluster's shared memory (nnf_bn_cluster.cu): -1 where this shape's do not.
 	// `report`: the 64 words at the head of the workspace that say the launch went well, or null. All tensors 16-byte aligned.
 	// `slice_limit`: most shared memory per CTA for which this form is taken, by what takes the shape otherwise. Measured on one
-	// B200 before the items' constants carried their own tag, us: against the statistics and apply items of planes of whole float4s, whose second read comes from L2, slices of up to
-	// 56 KB win forward (x[128,512,28,28] 85 against 92; 98 KB: x[256,256,28,28] 98 against 80) and of up to 104 KB backward
-	// (x[512,128,14,14] 45.8 against 51.6; 196 KB: x[64,64,56,56] 54 against 47); against those of channel groups up to 104 KB
-	// (x[256,512,13,13] 45 / 71 against 57 / 88); against two kernels whatever fits (x[64,96,55,55] 40 / 75 against 60 / 151).
-	constexpr size_t kClusterSliceForward = 56 * 1024, kClusterSliceBackward = 104 * 1024, kClusterSliceGroups = 104 * 1024;
+	// B200 with ReLU, us: against the statistics and apply items of planes of whole float4s, whose second read comes from L2, slices of
+	// up to 56 KB win in either direction (forward, 49 KB: x[512,128,14,14] 25.8 against 30.9, x[128,512,28,28] 84 against 84; 61 KB:
+	// x[160,256,28,28] 59 against 54; backward, 49 KB: x[256,256,14,14] 41 against 46, x[64,128,28,28] 26.2 against 27.0; 74 KB:
+	// x[96,256,28,28] 68 against 54; 98 KB: x[128,512,28,28] 153 against 122); against those of channel groups up to 104 KB
+	// (x[512,256,13,13], 43 / 86 KB: 50 / 80 against 59 / 88; forward, 114 KB: x[1024,256,15,15] 171 against 121; backward, 129 KB:
+	// x[768,256,13,13] 151 against 121); against two kernels whatever fits (x[64,96,55,55] 40 / 74 against 61 / 155).
+	constexpr size_t kClusterSlice = 56 * 1024, kClusterSliceGroups = 104 * 1024;
 	constexpr size_t kClusterSliceAny = ~size_t(0);
 	int cluster_train_fwd(cudaStream_t s, float * y, float * saved, float * sums, const float * x, const float * gamma, const float * beta, float eps,
 		const act_chain& chain, int64_t n, int64_t c, int64_t hw, void * report, size_t slice_limit);

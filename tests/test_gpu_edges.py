@@ -249,9 +249,10 @@ def test_training_batch_norm_in_a_cluster(capi, tuning, shape, acts, ctas):
     room = 4e-6 * (n * h * w) ** 0.5
 
     def in_cluster(backward, got):
-        # 220 KB of a channel's entries are the most that a CTA takes; where they do not fit, any other form is right
-        row = (h * w // 4 if h * w % 4 == 0 else (h * w + 6) // 4) * 16 * (2 if backward else 1)
-        if -(-n // (ctas or 8)) * row <= 220 * 1024:
+        # a CTA takes at most 220 KB of a channel's entries, 56 KB where planes are whole float4s; beyond that any other form is right
+        whole = h * w % 4 == 0
+        row = (h * w // 4 if whole else (h * w + 6) // 4) * 16 * (2 if backward else 1)
+        if -(-n // (ctas or 8)) * row <= (56 if whole else 220) * 1024:
             assert len(got) == 1 and got[0] in ([ctas] if ctas else [1, 2, 4, 8]), got
         else:
             assert len(got) > 1, got
@@ -325,6 +326,33 @@ def test_smallest_planes_of_the_cluster_form(capi, shape, clusters):
     forward()
     want = torch.nn.functional.batch_norm(x.double(), None, None, training=True, eps=1e-5)
     assert float((y - want).norm() / want.norm()) <= 1e-6
+
+
+@pytest.mark.parametrize("backward", [False, True])
+@pytest.mark.parametrize("plane,kb", [((4, 4), 56), ((7, 7), 104)])
+def test_largest_slices_of_the_cluster_form(capi, tuning, plane, kb, backward):
+    """As many entries as a CTA's slice may hold, and one more: 56 KB of planes of whole float4s, 104 KB of ragged ones that channel groups
+    take otherwise. One CTA per channel."""
+    tuning("chain_cluster", 1)
+    hw = plane[0] * plane[1]
+    row = (hw // 4 if hw % 4 == 0 else (hw + 6) // 4) * 16 * (2 if backward else 1)
+    for n, clusters in ((kb * 1024 // row, True), (kb * 1024 // row + 1, False)):
+        x, dy = (torch.empty((n, 8) + plane, device="cuda").normal_() for _ in range(2))
+        gamma, beta = torch.ones(8, device="cuda"), torch.zeros(8, device="cuda")
+        out, saved, sums = torch.empty_like(x), torch.empty(16, device="cuda"), torch.empty(24, device="cuda")
+        ws = torch.empty(capi.bn_train_workspace_bytes(n, 8, hw), dtype=torch.uint8, device="cuda")
+        xd = x.double().requires_grad_(True)
+        want = torch.nn.functional.batch_norm(xd, None, None, training=True, eps=1e-5)
+        forward = lambda: capi.bn_train_fwd(out, saved, sums, x, gamma, beta, 1e-5, [], workspace=ws)
+        call = forward
+        if backward:
+            forward()
+            want.backward(dy.double())
+            want = xd.grad
+            call = lambda: capi.bn_train_bwd(out, sums, dy, x, gamma, beta, saved, [], workspace=ws)
+        assert (launches(call) == [1]) == clusters
+        call()
+        assert float((out - want.detach()).norm() / want.detach().norm()) <= (3e-6 if backward else 1e-6)
 
 
 @pytest.mark.parametrize("shape", [(49200, 4, 4, 4), (3000, 8, 3, 3), (600, 8, 28, 28)])
