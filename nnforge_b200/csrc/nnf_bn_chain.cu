@@ -1587,7 +1587,11 @@ namespace nnf
 					return 2;
 				if constexpr (!PEER)
 				{
-					const int st = cluster_train_fwd(stream, y, saved, sums, x, gamma, beta, eps, chain, n, c, hw, workspace, kClusterSliceGroups);
+					// Planes of up to 49 elements are copied as frames that are mostly edges, which shows where HBM is all that is waited for:
+					// forward, tensors beyond 100 MB stay here (us, cluster / here: x[1024,1024,7,7] 114 / 103, x[2048,512,7,7] 116 / 107,
+					// x[1901,1024,5,5] 128 / 111; x[1024,512,7,7], 103 MB, 58 / 57; x[512,1024,7,7], 103 MB, 56 / 60; x[256,512,7,7] 17 / 22).
+					const bool edges = hw <= 49 && n * c * hw * 4 > 100000000;
+					const int st = edges ? -1 : cluster_train_fwd(stream, y, saved, sums, x, gamma, beta, eps, chain, n, c, hw, workspace, kClusterSliceGroups);
 					if (st != -1)
 						return st;
 				}

@@ -355,6 +355,22 @@ def test_largest_slices_of_the_cluster_form(capi, tuning, plane, kb, backward):
         assert float((out - want.detach()).norm() / want.detach().norm()) <= (3e-6 if backward else 1e-6)
 
 
+@pytest.mark.parametrize("shape,clusters", [((2048, 248, 7, 7), True), ((2048, 256, 7, 7), False), ((1024, 256, 9, 11), True)])
+def test_small_ragged_planes_of_large_tensors(capi, shape, clusters):
+    """Forward, 100 MB on either side for planes of 49 elements, and more than that for larger planes; backward, clusters throughout."""
+    n, c, h, w = shape
+    x, dy = (torch.empty(shape, device="cuda").normal_() for _ in range(2))
+    gamma, beta = torch.ones(c, device="cuda"), torch.zeros(c, device="cuda")
+    y, dx, saved, sums, bsums = torch.empty_like(x), torch.empty_like(x), *(torch.empty(k * c, device="cuda") for k in (2, 2, 3))
+    ws = torch.empty(capi.bn_train_workspace_bytes(n, c, h * w), dtype=torch.uint8, device="cuda")
+    forward = lambda: capi.bn_train_fwd(y, saved, sums, x, gamma, beta, 1e-5, [], workspace=ws)
+    assert (len(launches(forward)) == 1) == clusters
+    assert len(launches(lambda: capi.bn_train_bwd(dx, bsums, dy, x, gamma, beta, saved, [], workspace=ws))) == 1
+    forward()
+    want = torch.nn.functional.batch_norm(x.double(), None, None, training=True, eps=1e-5)
+    assert float((y - want).norm() / want.norm()) <= 1e-6
+
+
 @pytest.mark.parametrize("shape", [(49200, 4, 4, 4), (3000, 8, 3, 3), (600, 8, 28, 28)])
 def test_training_batch_norm_stays_in_its_workspace(capi, tuning, shape):
     """As many items per channel as a plan makes (64 at most), with a workspace of exactly the size that is asked for: what follows it
