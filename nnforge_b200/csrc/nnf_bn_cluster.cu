@@ -122,7 +122,7 @@ namespace nnf
 			__shared__ double s_warp[kClusterMaxThreads / 32][K];
 			__shared__ double s_part[kClusterMax][K];            // the sums of the cluster's CTAs; each CTA has all of them
 			__shared__ float s_const[4];
-			pdl_begin();
+			pdl_begin_early();
 			cluster_arrive();                                    // waited for before the first store into another CTA
 			if (p.report && blockIdx.x == 0 && threadIdx.x < 64)
 				p.report[threadIdx.x] = 0;

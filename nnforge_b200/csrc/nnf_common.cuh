@@ -14,14 +14,25 @@ namespace nnf
 	int check_launch(const char * what);
 
 	// ---- launches ------------------------------------------------------------------------------
-	// Kernels launched through launch() have programmatic stream serialisation and begin with pdl_begin(): it lets the next
-	// launch of the stream be set up as soon as all of this grid's CTAs have started, then waits until the launch in front of
-	// it has completed and its writes are visible. Nothing is read or written before that wait, so the stream's order holds
-	// as without it; what overlaps is the set-up of a launch with the end of the one before it. A kernel that some other
-	// launch (a copy, another library's kernel) follows or precedes waits as usual. Without it a launch that depends on the one
-	// in front of it costs about 4.1 us from start to start however little it does (B200, back to back in one stream); with it
-	// batch norm + ReLU of one 64x32x32 image takes 2.9 us, softmax of 32x21x128x128 forward and backward 34 us instead of 38.
+	// Kernels launched through launch() have programmatic stream serialisation and begin with pdl_begin(), which waits until the
+	// launch in front has completed and its writes are visible. Nothing is read or written before that wait, so the stream's
+	// order holds as without it; what overlaps is the set-up of a launch with the end of the one before it: the next launch's CTAs
+	// come in once every CTA of this one has exited, before its writes have been flushed. A kernel that some other launch (a copy,
+	// another library's kernel) follows or precedes waits as usual. Without it a launch that depends on the one in front of it
+	// costs about 4.1 us from start to start however little it does (B200, back to back in one stream); with it batch norm + ReLU
+	// of one 64x32x32 image takes 2.6 us, softmax of 32x21x128x128 forward and backward 34 us instead of 38.
 	__device__ __forceinline__ void pdl_begin()
+	{
+		asm volatile("griddepcontrol.wait;" ::: "memory");
+	}
+
+	// The same for kernels of many CTAs with one short piece of work each: the next launch's CTAs come in as soon as all of this
+	// one's have started. They take the slots that are free then, so where the CTAs are few and long, or stage tiles, a launch is
+	// spread unevenly over the SMs: us with this / pdl_begin() / no overlap at all, statistics of x[14563,515] 59 / 39 / 39,
+	// PReLU slope gradient of the same 118 / 70 / 70, batch norm -> add -> ReLU -> average of [152,64,16,16] 24 / 20 / 21, max
+	// subsampling of staged planes [4,64,130,130] 24 / 19 / 20. The other way round: add layer [19,64,7,7] 1.4 / 1.9 / 4.1, row
+	// kernel of max subsampling [124,64,56,56] 25.2 / 28.8 / 25.6, training batch norm in a cluster [2,515,7,7] 3.7 / 4.4.
+	__device__ __forceinline__ void pdl_begin_early()
 	{
 		asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 		asm volatile("griddepcontrol.wait;" ::: "memory");

@@ -782,7 +782,7 @@ namespace nnf
 		template <int MODE>
 		__global__ void __launch_bounds__(kThreads) add_kernel(const add_params p)
 		{
-			pdl_begin();
+			pdl_begin_early();
 			if (MODE == 2)
 			{
 				const uint32_t stride = gridDim.x * kThreads;
@@ -828,7 +828,7 @@ namespace nnf
 		template <int MODE>
 		__global__ void __launch_bounds__(kThreads) scale_kernel(float * dx, const float * dy, float alpha, uint32_t count, int add)
 		{
-			pdl_begin();
+			pdl_begin_early();
 			if (MODE == 2)
 			{
 				const uint32_t stride = gridDim.x * kThreads;

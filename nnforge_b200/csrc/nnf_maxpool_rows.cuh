@@ -147,7 +147,7 @@ namespace nnf
 			uint32_t * argmax = p.argmax ? p.argmax + obase : nullptr;
 			const uint32_t abs0 = uint32_t(pbase);
 			const float none = __int_as_float(MIN ? 0x7f800000 : 0xff800000);
-			pdl_begin();
+			pdl_begin_early();
 
 			float v[ROWS][V], rv[ROWS][V];
 			#pragma unroll
@@ -286,7 +286,7 @@ namespace nnf
 			const float * z = FUSED ? p.z + pbase : nullptr;
 			float * dx = p.dx ? p.dx + pbase : nullptr;
 			float * dres = FUSED && p.dres ? p.dres + pbase : nullptr;
-			pdl_begin();
+			pdl_begin_early();
 
 			float v[2 * PAIRS][V];       // z, or what dx holds already
 			uint32_t id[WROWS][NW];

@@ -86,7 +86,7 @@ namespace nnf
 			const bool vec = part.vec && base + (threadIdx.x + 1) * kOptPerThread <= part.count;
 			const uint32_t i0 = part.vec ? base + threadIdx.x * kOptPerThread : base + threadIdx.x;
 			const uint32_t step = part.vec ? 1 : kOptThreads;
-			pdl_begin();
+			pdl_begin_early();
 			float w[kOptPerThread], gr[kOptPerThread], p1[kOptPerThread], p2[kOptPerThread];
 			auto load = [&](float (&v)[kOptPerThread], const float * from)
 			{
