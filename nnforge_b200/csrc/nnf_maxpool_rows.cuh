@@ -374,18 +374,44 @@ namespace nnf
 			}
 		}
 
+		// From how many values on the plane-group kernels of nnf_maxpool.cu are the faster ones for small planes whose rows are not whole
+		// float4s: their groups of planes start and end on float4s, which counts once the tensors leave L2. us, row / plane-group kernels:
+		// Fused, four tensors per value (two-thirds of the instructions). Forward the two meet at 1.5 M values where rows are odd (27x27,
+		// 34 M values: 97 against 81) and at 6 M where they are even (18x18: 82 against 76), backward at 12 M where rows are odd (21x21,
+		// 34 M values: 97 against 92).
+		// Stand-alone forward, the row kernels waste the more of a thread's columns and of a halo row the smaller the plane is; 3x3 windows,
+		// odd rows: 9x9 10.4 / 9.0 at 5 M values and 44 / 25 at 25 M, 13x13 14.2 / 11.9 at 8 M, 21x21 26 / 23 at 18 M, 23x23 24.4 / 25.7; even
+		// rows: 6x6 8.3 / 7.7 at 5 M, 10x10 23 / 21 at 18 M, 14x14 29.6 / 27.3 at 25 M; 2x2 windows: 9x9 11.7 / 10.0 at 8 M, 21x21 20.9 / 19.5
+		// at 18 M, 6x6 53 / 50 at 50 M, 10x10 level.
+		int64_t plane_groups_from(const pool_geom& g, int access, bool aligned, bool fused, bool backward)
+		{
+			constexpr int64_t million = 1000000, never = int64_t(1) << 62;
+			const bool odd = access == 1, three = g.win_w == 3;
+			if (access == 4)
+				return never;
+			if (fused)
+			{
+				if (g.hw > 1024)
+					return never;
+				return backward ? (odd && three ? 12 * million : never) : odd ? 3 * million / 2 : 6 * million;
+			}
+			if (backward || !aligned)
+				return never;
+			if (odd && g.hw < 36)
+				return 2 * million;
+			if (three)
+				return odd ? (g.hw < 100 ? 5 * million / 2 : g.hw <= 169 ? 5 * million : g.hw <= 441 ? 15 * million : never)
+					: (g.hw <= 64 ? 4 * million : g.hw <= 100 ? 12 * million : g.hw <= 256 ? 20 * million : never);
+			return odd ? (g.hw <= 169 ? 6 * million : g.hw <= 441 ? 16 * million : never) : g.hw <= 49 ? 35 * million : never;
+		}
+
 		// Whether the row kernels take this layer, and the access width. `align`: the common alignment of the full-size buffers in bytes.
 		bool plan_rows(rows_params& q, int& access, const pool_geom& g, int64_t planes, size_t align, bool fused, bool backward)
 		{
 			if (!(g.win_w == g.win_h && (g.win_w == 3 || g.win_w == 2) && g.sw == 2 && g.sh == 2) || tune().pool_staged == 1)
 				return false;
 			access = (g.w % 4 == 0 && align % 16 == 0) ? 4 : ((g.w % 2 == 0 && align % 8 == 0) ? 2 : 1);
-			// Fused, with four tensors' scalar (float2) accesses per value, on large tensors: the plane-group kernels, whose four planes
-			// of up to 16 KB start and end on float4s (two-thirds of the instructions). Forward the two meet at 1.5 M values where
-			// rows are odd (27x27, 34 M values: 97 against 81 us) and at 6 M where they are even (18x18: 82 against 76), backward
-			// at 12 M where rows are odd (21x21, 34 M values: 97 against 92).
-			const int64_t values = planes * g.hw;
-			if (fused && access < 4 && g.hw <= 1024 && (backward ? access == 1 && g.win_w == 3 && values >= 12000000 : values >= (access == 1 ? 1500000 : 6000000)))
+			if (planes * g.hw >= plane_groups_from(g, access, align % 16 == 0, fused, backward))
 				return false;
 			q.c = g.c; q.h = g.h; q.w = g.w; q.hw = g.hw; q.oh = g.oh; q.ow = g.ow; q.ohw = g.ohw;
 			q.cols = (uint32_t)div_up(g.w, access == 4 ? 4 : 2);

@@ -124,6 +124,30 @@ def test_max_subsampling_rows_and_plane_groups(capi, oracle, tuning, shape, win,
         assert_bits_equal(host(dx), dx_want, "dx")
 
 
+# values on either side of the limits beyond which plane groups take small planes
+@pytest.mark.parametrize("plane,win,million", [((9, 9), 3, 2.5), ((13, 13), 3, 5), ((21, 21), 3, 15), ((6, 6), 3, 4), ((10, 10), 3, 12), ((14, 14), 3, 20), ((9, 9), 2, 6), ((5, 5), 2, 2),
+                                               ((21, 21), 2, 16), ((6, 6), 2, 35)])
+@pytest.mark.parametrize("offset", [0, 1])
+def test_max_subsampling_of_many_small_planes(capi, tuning, plane, win, million, offset):
+    """Whichever kernels take the layer, the values and the places are those of the plane-group kernels."""
+    hw = plane[0] * plane[1]
+    p = capi.pool((win, win), (2, 2))
+    for planes in (int(million * 1e6 / hw) - 1, int(million * 1e6 / hw) + 3):
+        shape = (planes, 1) + plane
+        x = torch.empty(planes * hw + offset, device="cuda").normal_()[offset:].view(shape)
+        out = (planes, 1) + capi.pool_out_shape(plane[0], plane[1], p)
+        got = []
+        for staged in (0, 1):
+            tuning("pool_staged", staged)
+            y, idx = torch.full(out, float("nan"), device="cuda"), torch.zeros(out, dtype=torch.int32, device="cuda")
+            dx = torch.full_like(x, float("nan"))
+            capi.maxpool_fwd(y, idx, x, p)
+            capi.maxpool_bwd(dx, y, idx, p)
+            got.append((y, idx, dx))
+        for a, b in zip(*got):
+            assert torch.equal(a, b)
+
+
 @pytest.mark.parametrize("win", [2, 3])
 def test_fused_max_subsampling_of_planes_beyond_shared_memory(capi, oracle, win):
     """Planes of 231 KB: taken at stride 2 where z is written to a buffer of its own, refused over x, over the residual and at other
