@@ -368,8 +368,33 @@ namespace nnf
 			}
 		}
 
-		// ROW4: 3x3 windows at stride 2 behind the fused layers, rows in chunks of four elements; otherwise any window, element by element
-		template <bool FUSED, bool ROW4>
+		// 2x2 windows, stride 2, four consecutive elements of one input row: windows do not overlap, the four elements
+		// belong to the two windows {k, k + 1} of output row iy / 2, k = ix0 / 2 - two (argmax, gradient) pairs per vector
+		__device__ __forceinline__ void gather_row4_2x2s2(const pool_geom& g, const float * dyp, const uint32_t * idp, uint32_t iy, uint32_t ix0,
+			uint32_t abs0, float (&acc)[4])
+		{
+			const uint32_t oy = iy >> 1;
+			if (oy > g.oh - 1)
+				return;
+			const uint32_t k = ix0 >> 1;
+			const uint32_t row = oy * g.ow + k;
+			#pragma unroll
+			for (uint32_t a = 0; a < 2; ++a)
+				if (k + a <= g.ow - 1)
+				{
+					const uint32_t i = idp[row + a];
+					const float d = dyp[row + a];
+					if (i == abs0 + 2 * a) acc[2 * a] = __fadd_rn(acc[2 * a], d);
+					if (i == abs0 + 2 * a + 1) acc[2 * a + 1] = __fadd_rn(acc[2 * a + 1], d);
+				}
+		}
+
+		// How the elements of a plane group are walked.
+		constexpr int kPoolElements = 0;   // one by one, any window
+		constexpr int kPoolChunks = 1;     // rows in chunks of four elements, the last one cut short; windows of WIN x WIN at stride 2
+		constexpr int kPoolVectors = 2;    // the same where every row is whole float4s
+
+		template <bool FUSED, int WIN, int ROWS>
 		__global__ void __launch_bounds__(kThreads) pool_bwd_staged_kernel(const pool_bwd_params p)
 		{
 			pdl_begin();
@@ -392,7 +417,7 @@ namespace nnf
 					s_idx[o] = __ldcs(p.argmax + obase + o);
 				}
 				const uint32_t ch0 = (uint32_t)(plane0 - int64_t(g.d_c.div((uint32_t)plane0)) * g.c);
-				if (ROW4)
+				if (FUSED && ROWS == kPoolChunks)
 					for (uint32_t lp = threadIdx.x; lp < np; lp += kThreads)
 					{
 						uint32_t channel = ch0 + lp;
@@ -430,10 +455,15 @@ namespace nnf
 						out_dx = dz;
 				};
 
-				if (ROW4)
+				auto gather_row4 = [&](uint32_t lp, uint32_t iy, uint32_t ix0, uint32_t abs0, float (&acc)[4])
 				{
-					// rows that are not a multiple of four elements (14x14, 7x7): the same four-element row
-					// chunks, with scalar accesses and the last chunk of a row cut short
+					if (WIN == 2)
+						gather_row4_2x2s2(g, s_dy + lp * g.ohw, s_idx + lp * g.ohw, iy, ix0, abs0, acc);
+					else
+						gather_row4_3x3s2(g, s_dy + lp * g.ohw, s_idx + lp * g.ohw, iy, ix0, abs0, acc);
+				};
+				if (ROWS == kPoolChunks)
+				{
 					const uint32_t cpr = (g.w + 3) >> 2;           // chunks per row
 					const uint32_t nchunks = np * g.h * cpr;
 					for (uint32_t q = threadIdx.x; q < nchunks; q += kThreads)
@@ -445,13 +475,26 @@ namespace nnf
 						const uint32_t e0 = lp * g.hw + iy * g.w + ix0;
 						const uint32_t nvalid = min(4u, g.w - ix0);
 						float acc[4] = {0.0F, 0.0F, 0.0F, 0.0F};
-						gather_row4_3x3s2(g, s_dy + lp * g.ohw, s_idx + lp * g.ohw, iy, ix0, (uint32_t)(base + e0), acc);
+						if (!FUSED && p.add)
+						{
+							#pragma unroll
+							for (int k = 0; k < 4; ++k)
+								if ((uint32_t)k < nvalid)
+									acc[k] = p.dx[base + e0 + k];
+						}
+						gather_row4(lp, iy, ix0, (uint32_t)(base + e0), acc);
 						#pragma unroll
 						for (int k = 0; k < 4; ++k)
 							if ((uint32_t)k < nvalid)
-								s_dz[e0 + k] = acc[k]; // gathered gradient of the group, consumed with coalesced accesses below
+							{
+								if (FUSED)
+									s_dz[e0 + k] = acc[k]; // gathered gradient of the group, consumed with coalesced accesses below
+								else
+									p.dx[base + e0 + k] = acc[k];
+							}
 					}
-					__syncthreads();
+					if (FUSED)
+						__syncthreads();
 					// the batch-norm factor of a plane comes from shared memory; a vector of four elements lies in
 					// one plane unless it straddles a plane boundary (H*W not a multiple of 4)
 					auto finish = [&](float mult, float zval, float dz, float& odx, float& ores)
@@ -460,7 +503,7 @@ namespace nnf
 						ores = ds;
 						odx = p.gamma ? __fmul_rn(ds, mult) : ds;
 					};
-					const uint32_t nvec = p.vec_ok ? (count >> 2) : 0;
+					const uint32_t nvec = FUSED && p.vec_ok ? (count >> 2) : 0;
 					for (uint32_t v = threadIdx.x; v < nvec; v += kThreads)
 					{
 						const float4 z4 = ld_stream(reinterpret_cast<const float4 *>(p.z + base) + v);
@@ -479,7 +522,7 @@ namespace nnf
 						if (p.dres)
 							st_stream(reinterpret_cast<float4 *>(p.dres + base) + v, orr);
 					}
-					for (uint32_t e = (nvec << 2) + threadIdx.x; e < count; e += kThreads)
+					for (uint32_t e = (nvec << 2) + threadIdx.x; FUSED && e < count; e += kThreads)
 					{
 						float odx, ores;
 						finish(s_mult[g.d_hw.div(e)], p.z[base + e], s_dz[e], odx, ores);
@@ -507,9 +550,33 @@ namespace nnf
 							seed[0] = d4.x; seed[1] = d4.y; seed[2] = d4.z; seed[3] = d4.w;
 						}
 						float odx[4], ores[4];
-						#pragma unroll
-						for (int k = 0; k < 4; ++k)
-							element((v << 2) + k, zv[k], seed[k], odx[k], ores[k]);
+						if (ROWS == kPoolVectors)
+						{
+							const uint32_t e0 = v << 2;
+							const uint32_t lp = g.d_hw.div(e0);
+							const uint32_t rem = e0 - lp * g.hw;
+							const uint32_t iy = g.d_w.div(rem);
+							gather_row4(lp, iy, rem - iy * g.w, (uint32_t)(base + e0), seed);
+							float mult = 1.0F;
+							if (FUSED && p.gamma)
+							{
+								uint32_t channel = ch0 + lp;
+								channel -= g.d_c.div(channel) * g.c;
+								mult = __fmul_rn(__ldg(p.gamma + channel), __ldg(p.invsigma + channel));
+							}
+							#pragma unroll
+							for (int k = 0; k < 4; ++k)
+							{
+								ores[k] = FUSED && (__float_as_uint(zv[k]) >> 31) ? __fmul_rn(seed[k], p.slope) : seed[k];
+								odx[k] = FUSED && p.gamma ? __fmul_rn(ores[k], mult) : ores[k];
+							}
+						}
+						else
+						{
+							#pragma unroll
+							for (int k = 0; k < 4; ++k)
+								element((v << 2) + k, zv[k], seed[k], odx[k], ores[k]);
+						}
 						if (p.dx)
 							st_stream(reinterpret_cast<float4 *>(p.dx + base) + v, make_float4(odx[0], odx[1], odx[2], odx[3]));
 						if (FUSED && p.dres)
@@ -744,8 +811,9 @@ namespace nnf
 			}
 			bool vec_ok = (!p.dx || aligned16(p.dx)) && (!fused || (aligned16(p.z) && (!p.dres || aligned16(p.dres))));
 			const int grp = choose_group(p.g, p.planes, vec_ok);
-			const bool ragged_fast = fused && p.g.win_w == 3 && p.g.win_h == 3 && p.g.sw == 2 && p.g.sh == 2;
-			const size_t smem = (((size_t(grp) * p.g.ohw * 2 + 3) & ~size_t(3)) + (ragged_fast ? ((size_t(grp) * p.g.hw + 3) & ~size_t(3)) + size_t(grp) : 0)) * sizeof(float);
+			const int win = p.g.win_w == p.g.win_h && p.g.sw == 2 && p.g.sh == 2 && (p.g.win_w == 2 || p.g.win_w == 3) ? p.g.win_w : 0;
+			const bool vectors = win != 0 && (p.g.w & 3) == 0 && vec_ok, chunks = !vectors && win == (fused ? 3 : 2);
+			const size_t smem = (((size_t(grp) * p.g.ohw * 2 + 3) & ~size_t(3)) + (fused && chunks ? ((size_t(grp) * p.g.hw + 3) & ~size_t(3)) + size_t(grp) : 0)) * sizeof(float);
 			if (grp == 0 || smem > staging_smem_limit())
 			{
 				const int64_t blocks = div_up(p.planes * p.g.hw, kThreads);
@@ -765,7 +833,11 @@ namespace nnf
 			const int grid = (int)(ngroups < cap ? ngroups : cap);
 			p.d_cpr = fastdiv((p.g.w + 3) / 4);
 			p.d_hcpr = fastdiv(p.g.h * ((p.g.w + 3) / 4));
-			const auto kernel = ragged_fast ? pool_bwd_staged_kernel<true, true> : fused ? pool_bwd_staged_kernel<true, false> : pool_bwd_staged_kernel<false, false>;
+			const auto kernel =
+				vectors && fused ? (win == 3 ? pool_bwd_staged_kernel<true, 3, kPoolVectors> : pool_bwd_staged_kernel<true, 2, kPoolVectors>)
+				: vectors ? (win == 3 ? pool_bwd_staged_kernel<false, 3, kPoolVectors> : pool_bwd_staged_kernel<false, 2, kPoolVectors>)
+				: chunks ? (fused ? pool_bwd_staged_kernel<true, 3, kPoolChunks> : pool_bwd_staged_kernel<false, 2, kPoolChunks>)
+				: fused ? pool_bwd_staged_kernel<true, 0, kPoolElements> : pool_bwd_staged_kernel<false, 0, kPoolElements>;
 			const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)staging_smem_limit());
 			if (e == cudaSuccess)
 				launch(kernel, grid, kThreads, smem, s, p);

@@ -383,19 +383,25 @@ namespace nnf
 		// odd rows: 9x9 10.4 / 9.0 at 5 M values and 44 / 25 at 25 M, 13x13 14.2 / 11.9 at 8 M, 21x21 26 / 23 at 18 M, 23x23 24.4 / 25.7; even
 		// rows: 6x6 8.3 / 7.7 at 5 M, 10x10 23 / 21 at 18 M, 14x14 29.6 / 27.3 at 25 M; 2x2 windows: 9x9 11.7 / 10.0 at 8 M, 21x21 20.9 / 19.5
 		// at 18 M, 6x6 53 / 50 at 50 M, 10x10 level.
+		// Backward, rows of 4: a warp's accesses to its two rows cover every second 16 bytes (fused, 8 M values: 4x4 23.5 / 19.9, 28x4
+		// 23.2 / 20.7; stand-alone only the lowest planes, 4x4 55 / 48 at 50 M). Stand-alone 2x2 with odd rows, which the plane groups walk in
+		// chunks of four: 7x7 28 / 24 at 18 M, 300x7 30 / 24, 11x11 38 / 33 at 25 M, 300x11 40 / 33; a fourth chunk element that is mostly
+		// missing (9x9, 5x5) puts the point where they meet three times as high, and from 13 columns on rows are the faster ones.
 		int64_t plane_groups_from(const pool_geom& g, int access, bool aligned, bool fused, bool backward)
 		{
 			constexpr int64_t million = 1000000, never = int64_t(1) << 62;
 			const bool odd = access == 1, three = g.win_w == 3;
 			if (access == 4)
-				return never;
+				return !backward || g.w > 4 ? never : fused ? 9 * million / 2 : g.h <= 8 ? 18 * million : never;
 			if (fused)
 			{
 				if (g.hw > 1024)
 					return never;
 				return backward ? (odd && three ? 12 * million : never) : odd ? 3 * million / 2 : 6 * million;
 			}
-			if (backward || !aligned)
+			if (backward)
+				return !odd || three || g.w > 11 ? never : g.w % 4 == 3 ? 15 * million / 2 : 24 * million;
+			if (!aligned)
 				return never;
 			if (odd && g.hw < 36)
 				return 2 * million;

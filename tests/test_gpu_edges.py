@@ -126,10 +126,10 @@ def test_max_subsampling_rows_and_plane_groups(capi, oracle, tuning, shape, win,
 
 # values on either side of the limits beyond which plane groups take small planes
 @pytest.mark.parametrize("plane,win,million", [((9, 9), 3, 2.5), ((13, 13), 3, 5), ((21, 21), 3, 15), ((6, 6), 3, 4), ((10, 10), 3, 12), ((14, 14), 3, 20), ((9, 9), 2, 6), ((5, 5), 2, 2),
-                                               ((21, 21), 2, 16), ((6, 6), 2, 35)])
+                                               ((21, 21), 2, 16), ((6, 6), 2, 35), ((4, 4), 3, 18), ((4, 4), 2, 18), ((7, 7), 2, 7.5), ((11, 11), 2, 7.5), ((20, 4), 3, 4.5), ((20, 4), 2, 4.5)])
 @pytest.mark.parametrize("offset", [0, 1])
 def test_max_subsampling_of_many_small_planes(capi, tuning, plane, win, million, offset):
-    """Whichever kernels take the layer, the values and the places are those of the plane-group kernels."""
+    """Whichever kernels take the layer, and behind the fused layers where rows are 4 wide, the results are those of the plane-group kernels."""
     hw = plane[0] * plane[1]
     p = capi.pool((win, win), (2, 2))
     for planes in (int(million * 1e6 / hw) - 1, int(million * 1e6 / hw) + 3):
@@ -143,7 +143,13 @@ def test_max_subsampling_of_many_small_planes(capi, tuning, plane, win, million,
             dx = torch.full_like(x, float("nan"))
             capi.maxpool_fwd(y, idx, x, p)
             capi.maxpool_bwd(dx, y, idx, p)
-            got.append((y, idx, dx))
+            got.append([y, idx, dx])
+            if plane[1] == 4:
+                one, zero = torch.ones(1, device="cuda"), torch.zeros(1, device="cuda")
+                z, dr = torch.empty_like(x), torch.full_like(x, float("nan"))
+                capi.bn_add_relu_maxpool_fwd(z, y, idx, x, x, (one * 1.5, one, zero, one), 0.0, p)
+                capi.bn_add_relu_maxpool_bwd(dx, dr, y, idx, z, one * 1.5, one, 0.0, p)
+                got[-1] += [z, dr, dx]
         for a, b in zip(*got):
             assert torch.equal(a, b)
 
