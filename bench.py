@@ -361,8 +361,7 @@ def collect_sweep(args, quick):
                timeit(lambda i: capi.bn_add_relu_avgpool_bwd(dx, dr, dpo, z, bn[0], bn[3], 0.0, (hw, hw), mult), 1), 12 * e)
         del x, r, z, pooled, dpo, dx, dr
     # the stand-alone subsampling layers (no batch norm in front): max 3x3/2 and 2x2/2, average 2x2
-    for c, hw, win in ([] if quick else [(64, 56, 3), (128, 28, 3), (128, 28, 2), (256, 14, 2)]):
-        n = 1024
+    for n, c, hw, win in ([] if quick else [(1024, 64, 56, 3), (1024, 128, 28, 3), (1024, 128, 28, 2), (1024, 256, 14, 2), (256, 96, 55, 3)]):
         shape = (n, c, hw, hw)
         e = n * c * hw * hw
         p = capi.pool((win, win), (2, 2))
@@ -378,8 +377,9 @@ def collect_sweep(args, quick):
             report(3, "avgpool 2x2 fwd N=%d C=%d %dx%d" % (n, c, hw, hw), timeit(lambda i: capi.avgpool_fwd(pooled, x, (2, 2), 0.25), 1), 5 * e)
             report(3, "avgpool 2x2 bwd N=%d C=%d %dx%d" % (n, c, hw, hw), timeit(lambda i: capi.avgpool_bwd(dx, dpo, (2, 2), 0.25), 1), 5 * e)
         del x, pooled, idx, dpo, dx
-    # training batch norm + ReLU on the last stage's 7x7 planes (not whole float4s: the channel-group kernels)
-    for n, c, hw in ([] if quick else [(1024, 512, 7), (256, 2048, 7)]):
+    # training batch norm + ReLU, one launch each: channels that fit a cluster's shared memory (14x14, 27x27, 7x7 backward) and
+    # channel groups (7x7 forward beyond 100 MB)
+    for n, c, hw in ([] if quick else [(256, 512, 14), (128, 96, 27), (1024, 512, 7), (256, 2048, 7)]):
         shape = (n, c, hw, hw)
         e = n * c * hw * hw
         x, dy = torch.randn(shape, device="cuda"), torch.randn(shape, device="cuda")
@@ -388,9 +388,9 @@ def collect_sweep(args, quick):
         saved, sums, bsums = torch.empty(2 * c, device="cuda"), torch.empty(2 * c, device="cuda"), torch.empty(3 * c, device="cuda")
         ws = torch.empty(capi.bn_train_workspace_bytes(n, c, hw * hw), dtype=torch.uint8, device="cuda")
         acts = [capi.relu(0.0)]
-        report(3, "bn_train+relu fwd N=%d C=%d %dx%d, one launch (channel-group items)" % (n, c, hw, hw),
+        report(3, "bn_train+relu fwd N=%d C=%d %dx%d, one launch" % (n, c, hw, hw),
                timeit(lambda i: capi.bn_train_fwd(y, saved, sums, x, gamma, beta, 1e-5, acts, workspace=ws), 1), 8 * e)
-        report(3, "bn_train+relu bwd N=%d C=%d %dx%d, one launch (channel-group items)" % (n, c, hw, hw),
+        report(3, "bn_train+relu bwd N=%d C=%d %dx%d, one launch" % (n, c, hw, hw),
                timeit(lambda i: capi.bn_train_bwd(dx, bsums, dy, x, gamma, beta, saved, acts, workspace=ws), 1), 12 * e)
         del x, dy, y, dx
     # beyond the five configurations: inference BN + ReLU on planes that are not whole float4s (the channel-group kernel)

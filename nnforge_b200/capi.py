@@ -1,4 +1,5 @@
-"""ctypes binding of include/nnf_b200.h (the C ABI of libnnf_b200.so).
+"""Python binding of include/nnf_b200.h (the C ABI of libnnf_b200.so): the calls that a step makes go through the extension module
+_native, set-up calls and the multi-GPU exchange through ctypes.
 
 Tensors are passed as torch CUDA tensors (or ``None``); the binding hands their ``data_ptr()`` to the
 library and enqueues on torch's current stream unless ``stream=`` is given. A non-zero status raises

@@ -1376,7 +1376,9 @@ namespace nnf
 			// 48 against 127-130 at 32; with it 88 us at either)
 			// On one GPU the distance in bytes decides, 26 MB of x forward and 19 MB each of x and dy backward: with 32 / 24 channels of
 			// 3.2 MB the second read came from HBM (x[64,64,112,112] 91 / 148 us, at 8 / 6 channels 76 / 114; x[128,32,112,112], 6.4 MB,
-			// 94 / 154 us, at 4 channels 77 / 118; x[512,128,28,28], 1.6 MB, 86 / 146 us, at 16 / 12 channels 78 / 118).
+			// 94 / 154 us, at 4 channels 77 / 118; x[512,128,28,28], 1.6 MB, 86 / 146 us, at 16 / 12 channels 78 / 118; these distances
+			// were set by hand, and those of the rule are the same or one channel off). It does not go below two channels: where one
+			// alone is 12.8 MB, the second read comes from HBM in part (x[1024,16,56,56] 95 / 142 us, x[256,16,112,112] 98 / 141).
 			const int64_t most = backward ? 24 : 32, bytes = backward ? 19300000 : 25700000, channel = n * plane_bytes;
 			int64_t dist = t.chain_dist >= 0 ? t.chain_dist : sharded ? (backward ? 24 : 48) : std::max(int64_t(2), std::min(most, (bytes + channel / 2) / channel));
 			if (dist > c) dist = c;

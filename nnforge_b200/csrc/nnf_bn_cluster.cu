@@ -15,7 +15,9 @@
 //   x[256,512,7,7]    17.3 / 26.6   (channel groups 22.1 / 30.1;                    7.9 / 11.8)
 //   x[256,512,14,14]  45.2 / 75.2   (statistics and apply items 63.0 / 91.2;       31.4 / 47.1)
 // A CTA's life is copies, about 4 us of latencies (sums, barrier, constants, first store) and stores, and the shared memory it
-// holds meanwhile is what limits the bytes in flight. Persistent clusters with a ring of two to four channels, the next ones'
+// holds meanwhile is what limits the bytes in flight. Backward, the first CTA of a channel's cluster is held longest: one thread updates
+// up to five per-channel gradients, each a round trip to memory behind the one before it, in front of the barrier that the result
+// waits for. Persistent clusters with a ring of two to four channels, the next ones'
 // copies and sums overlapping a channel's exchange, were slower at every shape (x[256,512,14,14] forward 52.8): about 2 us of
 // barriers per channel in series, and clusters of 8 resident on 120 of the SMs only.
 #include "nnf_common.cuh"
@@ -372,7 +374,7 @@ namespace nnf
 			size_t smem;
 		};
 
-		// CTAs per channel: as few as bring a CTA's slice down to 56 KB (four CTAs on an SM), more while the channels do not fill the
+		// CTAs per channel: as few as bring a CTA's slice down to 56 KB (three CTAs on an SM), more while the channels do not fill the
 		// SMs. Threads: as many as the CTAs that an SM will hold leave registers for (x[32,256,14,14] forward, two CTAs per SM: 5.6 us
 		// with 512 threads, 9.4 with 128; x[256,512,14,14], eight: 44 with 128, 85 with 512).
 		bool plan_cluster(cluster_plan& plan, cluster_params& p, int64_t n, int64_t c, int64_t hw, bool backward, size_t slice_limit)

@@ -1,8 +1,9 @@
 // 2-D max subsampling forward/backward, stand-alone and fused behind batch norm -> residual add ->
 // ReLU (the tail of a ResNet block). HBM-bound.
 //
-// Windows of 3x3 or 2x2 at stride 2 go through the row kernels of nnf_maxpool_rows.cuh, the rest (and large fused tensors with odd rows)
-// through the plane-group kernels of this file.
+// Windows of 3x3 or 2x2 at stride 2 go through the row kernels of nnf_maxpool_rows.cuh, except where its rule finds the plane-group
+// kernels of this file the faster ones (large tensors of small planes whose rows are not whole float4s, rows of 4 backward) and where
+// the fused forward writes z over one of its inputs. Every other window goes through the plane-group kernels.
 //
 // Data movement: a CTA owns a group of whole consecutive (n, c) planes, which are contiguous in the
 // planar layout. Forward: the group is read once with coalesced 128-bit loads, the fused

@@ -3,7 +3,7 @@
 // (or two) of rows of one plane. Included by
 // nnf_maxpool.cu only.
 //
-// What bounds these layers is HBM. The plane-group kernels of nnf_maxpool.cu, which take every other window, stage whole planes
+// What bounds these layers is HBM. The plane-group kernels of nnf_maxpool.cu, which take every other window and some of these, stage whole planes
 // in shared memory between a load phase and a window phase, and spend nine shared-memory reads and their index arithmetic
 // on every window; here every element is read into a register once, a row's horizontal maximum is shared by the two windows
 // that overlap in that row, the columns a window needs from its right-hand neighbour come by shuffle, and there is no barrier.

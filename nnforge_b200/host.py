@@ -1,4 +1,5 @@
-"""ctypes driver for the C++ host-side layer objects (csrc/host/nnf_layers.{h,cpp}).
+"""Driver for the C++ host-side layer objects (csrc/host/nnf_layers.{h,cpp}): set-up calls through ctypes, those of a step through the
+extension module _native.
 
 `Tester` / `Updater` create an nnForge-shaped layer object by the reference's type name through the
 C++ factory and forward each call to the object's member of the same name. Used by the tests; an
