@@ -802,24 +802,48 @@ namespace
 		PyObject * list = a.next();
 		if (PyList_Check(list))
 			parts.reserve((size_t)PyList_GET_SIZE(list));
-		a.sequence(list, [&](PyObject * d)
+		auto add = [&](PyObject * const (&v)[kPartFields])
+		{
+			auto address = [&](int k) { return v[k] ? a.address_of(v[k]) : nullptr; };
+			nnf_opt_part p = {};
+			p.data = static_cast<float *>(address(kData));
+			p.gradient = static_cast<float *>(address(kGradient));
+			p.prev_upd = static_cast<float *>(address(kPrevUpd));
+			p.prev_upd2 = static_cast<float *>(address(kPrevUpd2));
+			p.update_accum = static_cast<double *>(address(kUpdateAccum));
+			p.learning_rate = (float)a.number(v[kLearningRate]);
+			p.weight_decay = v[kWeightDecay] ? (float)a.number(v[kWeightDecay]) : 0.0F;
+			p.elem_count = a.numel(v[kData]);
+			if (a.ok())
+				parts.push_back(p);
+		};
+		auto add_mapping = [&](PyObject * d)
 		{
 			PyObject * v[kPartFields] = {};
 			owned asked[kPartFields] = {};
-			if (!PyDict_CheckExact(d))
-				for (int k = 0; k < kPartFields; ++k)
+			for (int k = 0; k < kPartFields; ++k)
+			{
+				const bool required = k <= kLearningRate;
+				asked[k].object = required ? PyObject_GetItem(d, keys.key[k]) : PyObject_CallMethod(d, "get", "O", keys.key[k]);
+				if (!asked[k].object)
 				{
-					const bool required = k <= kLearningRate;
-					asked[k].object = required ? PyObject_GetItem(d, keys.key[k]) : PyObject_CallMethod(d, "get", "O", keys.key[k]);
-					if (!asked[k].object)
-					{
-						a.fail(nullptr, nullptr);
-						return;
-					}
-					v[k] = required || asked[k].object != Py_None ? asked[k].object : nullptr;
+					a.fail(nullptr, nullptr);
+					return;
 				}
+				v[k] = required || asked[k].object != Py_None ? asked[k].object : nullptr;
+			}
+			add(v);
+		};
+		a.sequence(list, [&](PyObject * d)
+		{
+			if (!PyDict_CheckExact(d))
+			{
+				add_mapping(d);
+				return;
+			}
+			PyObject * v[kPartFields] = {};
 			PyObject * key, * value;
-			for (Py_ssize_t pos = 0; PyDict_CheckExact(d) && PyDict_Next(d, &pos, &key, &value);)
+			for (Py_ssize_t pos = 0; PyDict_Next(d, &pos, &key, &value);)
 			{
 				int k = 0;
 				while (k < kPartFields && key != keys.key[k])
@@ -836,19 +860,7 @@ namespace
 					a.fail(nullptr, nullptr);
 					return;
 				}
-			auto address = [&](int k) { return v[k] ? a.address_of(v[k]) : nullptr; };
-			nnf_opt_part p = {};
-			p.data = static_cast<float *>(address(kData));
-			p.gradient = static_cast<float *>(address(kGradient));
-			p.prev_upd = static_cast<float *>(address(kPrevUpd));
-			p.prev_upd2 = static_cast<float *>(address(kPrevUpd2));
-			p.update_accum = static_cast<double *>(address(kUpdateAccum));
-			p.learning_rate = (float)a.number(v[kLearningRate]);
-			p.weight_decay = v[kWeightDecay] ? (float)a.number(v[kWeightDecay]) : 0.0F;
-			p.elem_count = a.numel(v[kData]);
-			if (!a.ok())
-				return;
-			parts.push_back(p);
+			add(v);
 		});
 		const int type = (int)a.integer();
 		const float m1 = (float)a.number(), m2 = (float)a.number(), normalizer = (float)a.number();
