@@ -32,7 +32,7 @@ BYTES_PER_ELEM_BWD = 12
 METRIC = "fused BN+activation fwd/bwd achieved HBM GB/s"
 # dram__bytes_read.sum + dram__bytes_write.sum per launch from the ncu captures summarised under profiles/ (same shape:
 # bn_train_chain_kernel_x256x256x28x28.md, bn_bwd_apply_kernel_cfg2_..., bn_bwd_stats_kernel_cfg2_..., bn_stats_..., bn_apply_channel_...)
-NCU_TRAFFIC_BYTES = {"forward": 364772352, "backward": 625849344, "bwd_apply": 580634624, "bwd_stats": 417700000, "stats": 210000000,
+NCU_TRAFFIC_BYTES = {"forward": 366246656, "backward": 622761216, "bwd_apply": 580634624, "bwd_stats": 417700000, "stats": 210000000,
                      "apply": 363633664}
 WORKLOAD = "bn_train+prelu+elu fwd+bwd, x[256,256,28,28] fp32 per GPU"
 KINK = 1e-5   # |bn output| below which an element is at PReLU's kink for the parity checks of dx
